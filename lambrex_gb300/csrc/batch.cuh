@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "fx64.cuh"
 #include "kernels.cuh"
 
 namespace lbx {
@@ -26,6 +27,7 @@ struct BBox {
   unsigned long long mx, mxy;  // fast-division magics (2^40 / d + 1) of the iteration space
   int dx, dxy;       // divisors: row length and plane size of the iteration space
   double om_s, om_b, rho0;
+  FxRates fx;        // om_s, om_b for the FP64 store's fixed-point collision
 };
 
 struct BTile {

@@ -32,6 +32,8 @@ __global__ void __launch_bounds__(512) k_b_step(const BBox* __restrict__ boxes,
     const T om_s = (T)B.om_s, om_b = (T)B.om_b, rho0 = (T)B.rho0;
     const unsigned long long mx = B.mx, mxy = B.mxy;
     const int dx = B.dx, dxy = B.dxy;
+    DfRates r{};
+    if constexpr (sizeof(T) == 8) r.fx = B.fx;
     for (int i0 = threadIdx.x; i0 < tl.count; i0 += blockDim.x * CPT) {
 #pragma unroll
       for (int u = 0; u < CPT; ++u) {
@@ -39,16 +41,16 @@ __global__ void __launch_bounds__(512) k_b_step(const BBox* __restrict__ boxes,
         if (i >= tl.count) break;
         const unsigned c = (unsigned)(tl.start + i);
         const int z = fdiv(c, mxy);
-        const unsigned r = c - (unsigned)z * (unsigned)dxy;
-        const int y = fdiv(r, mx);
-        const int x = (int)(r - (unsigned)y * (unsigned)dx);
+        const unsigned c2 = c - (unsigned)z * (unsigned)dxy;
+        const int y = fdiv(c2, mx);
+        const int x = (int)(c2 - (unsigned)y * (unsigned)dx);
         // boxes of the batch engine are below 2^23 cells: 32-bit indices
         if constexpr (KIND == kBoxPull)
-          cell_step_pull<T, false, int>(fin, fout, b, x, y, z, om_s, om_b, rho0, DfRates{});
+          cell_step_pull<T, false, int>(fin, fout, b, x, y, z, om_s, om_b, rho0, r);
         else if constexpr (KIND == kBoxPeriodic)
-          cell_step_periodic_pull<T, int>(fin, fout, b, cov, x, y, z, om_s, om_b, rho0);
+          cell_step_periodic_pull<T, int>(fin, fout, b, cov, x, y, z, om_s, om_b, rho0, r);
         else
-          cell_step_patch_pull<T, int>(fin, fout, b, cov, x, y, z, om_s, om_b, rho0);
+          cell_step_patch_pull<T, int>(fin, fout, b, cov, x, y, z, om_s, om_b, rho0, r);
       }
     }
   }
@@ -130,11 +132,11 @@ __global__ void k_b_coalesce(const BBox* __restrict__ boxes, const BCoupling* __
 }
 
 template <typename T>
-__global__ void k_b_to_qform(T* f, Box3 b, IBox cov, T om_s, T om_b, T rho0) {
+__global__ void k_b_to_qform(T* f, Box3 b, IBox cov, T om_s, T om_b, T rho0, DfRates r) {
   const int n = b.n[0] * b.n[1] * b.n[2];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int x = i % b.n[0], y = (i / b.n[0]) % b.n[1], z = i / (b.n[0] * b.n[1]);
-    cell_to_qform<T, int>(f, b, cov, x, y, z, om_s, om_b, rho0);
+    cell_to_qform<T, int>(f, b, cov, x, y, z, om_s, om_b, rho0, r);
   }
 }
 
@@ -157,7 +159,8 @@ int conversion_blocks(const Box3& b) {
 template <typename T>
 cudaError_t launch_b_to_qform(T* f, const Box3& b, const IBox& cov, double om_s, double om_b,
                               double rho0, cudaStream_t st) {
-  k_b_to_qform<T><<<conversion_blocks(b), 256, 0, st>>>(f, b, cov, (T)om_s, (T)om_b, (T)rho0);
+  k_b_to_qform<T><<<conversion_blocks(b), 256, 0, st>>>(f, b, cov, (T)om_s, (T)om_b, (T)rho0,
+                                                       rates_of<T>(om_s, om_b));
   return cudaGetLastError();
 }
 

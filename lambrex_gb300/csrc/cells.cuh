@@ -14,12 +14,16 @@ template <typename T>
 __host__ __device__ __forceinline__ T zero_pop(int q, T rho0) {
   return rho0 == T(0) ? T(0) : T(-W(q)) * rho0;
 }
-// collision of one cell: native in T, or for an FP64 store in paired FP32
-// arithmetic with its twin operations packed (df32.cuh; rho0 is 0 there)
+// collision of one cell: the FP32 store's in FP32; an FP64 store's (rho0 is 0
+// there) in 64-bit fixed point (fx64.cuh; with FP64 instructions where r.fx
+// was not given), or in paired FP32 arithmetic with its twin operations
+// packed (df32.cuh)
 template <typename T, bool PAIRED>
 __host__ __device__ __forceinline__ void collide_cell(T* f, T om_s, T om_b, T rho0, const DfRates& r) {
   if constexpr (PAIRED)
     collide_f64_via_df_w(f, r);
+  else if constexpr (sizeof(T) == 8)
+    collide_f64(f, om_s, om_b, r.fx);
   else
     collide<T>(f, om_s, om_b, rho0);
 }
@@ -279,7 +283,8 @@ __host__ __device__ __forceinline__ void cell_step_periodic_pull(const T* __rest
                                                                 T* __restrict__ fout,
                                                                 const Box3& b, const IBox& cov,
                                                                 int x, int y, int z, T om_s, T om_b,
-                                                                T rho0) {
+                                                                T rho0,
+                                                                const DfRates& r = DfRates{}) {
   if (cov.contains(x, y, z)) {
     if (covered_inside(cov, x, y, z)) return;
     const I c = sidx_i<I>(b, x + b.g, y + b.g, z + b.g), sq = (I)b.sq;
@@ -287,7 +292,7 @@ __host__ __device__ __forceinline__ void cell_step_periodic_pull(const T* __rest
     for (int q = 0; q < NV; ++q) st_pop(fout, (I)q * sq + c, b, zero_pop<T>(q, rho0));
     return;
   }
-  cell_step_pull<T, false, I>(fin, fout, b, x, y, z, om_s, om_b, rho0, DfRates{});
+  cell_step_pull<T, false, I>(fin, fout, b, x, y, z, om_s, om_b, rho0, r);
 }
 
 // AMR patch, storage cell (sx,sy,sz) of the grown box: sources outside the
@@ -296,7 +301,8 @@ template <typename T, typename I = long long>
 __host__ __device__ __forceinline__ void cell_step_patch_pull(const T* __restrict__ fin,
                                                              T* __restrict__ fout, const Box3& b,
                                                              const IBox& cov, int sx, int sy,
-                                                             int sz, T om_s, T om_b, T rho0) {
+                                                             int sz, T om_s, T om_b, T rho0,
+                                                             const DfRates& r = DfRates{}) {
   const int g = b.g;
   const int vx = sx - g, vy = sy - g, vz = sz - g;
   const I c = sidx_i<I>(b, sx, sy, sz), sq = (I)b.sq, rx = (I)b.sx, rxy = (I)b.sxy;
@@ -322,7 +328,7 @@ __host__ __device__ __forceinline__ void cell_step_patch_pull(const T* __restric
                  : zero_pop<T>(q, rho0);
     }
   }
-  if (valid) collide_cell<T, false>(f, om_s, om_b, rho0, DfRates{});
+  if (valid) collide_cell<T, false>(f, om_s, om_b, rho0, r);
 #pragma unroll
   for (int q = 0; q < NV; ++q) st_pop(fout, (I)q * sq + c, b, f[q]);
 }
@@ -333,7 +339,8 @@ __host__ __device__ __forceinline__ void cell_step_patch_pull(const T* __restric
 template <typename T, typename I = long long>
 __host__ __device__ __forceinline__ void cell_to_qform(T* __restrict__ f, const Box3& b,
                                                       const IBox& cov, int x, int y, int z, T om_s,
-                                                      T om_b, T rho0) {
+                                                      T om_b, T rho0,
+                                                      const DfRates& r = DfRates{}) {
   const I c = sidx_i<I>(b, x + b.g, y + b.g, z + b.g), sq = (I)b.sq;
   T p[NV];
   if (cov.contains(x, y, z)) {
@@ -343,7 +350,7 @@ __host__ __device__ __forceinline__ void cell_to_qform(T* __restrict__ f, const 
   } else {
 #pragma unroll
     for (int q = 0; q < NV; ++q) p[q] = ld_pop(f, (I)q * sq + c, b);
-    collide_cell<T, false>(p, om_s, om_b, rho0, DfRates{});
+    collide_cell<T, false>(p, om_s, om_b, rho0, r);
   }
 #pragma unroll
   for (int q = 0; q < NV; ++q) st_pop(f, (I)q * sq + c, b, p[q]);

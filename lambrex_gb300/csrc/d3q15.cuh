@@ -66,7 +66,8 @@ __host__ __device__ __forceinline__ float third_f(float v) {
 #endif
 }
 
-// In-place collision of one cell.  f holds populations (rho0 == 0) or
+// In-place collision of one cell: the FP32 store's, and the FP64 one where
+// the fixed-point form (fx64.cuh) leaves a cell to it.  f holds populations (rho0 == 0) or
 // shifted populations g_q = f_q - w_q rho0 (rho0 > 0); the rest state w rho0
 // is exactly mode 0, so the shift only turns the mode-0 value into
 // delta-rho and adds rho0 back where the density divides.

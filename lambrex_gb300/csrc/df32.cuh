@@ -15,9 +15,10 @@
 #pragma once
 #include <cmath>
 #include <cstdint>
-#include <cstring>
 
+#include "bits.cuh"
 #include "d3q15.cuh"
+#include "fx64.cuh"
 
 namespace lbx {
 
@@ -25,45 +26,6 @@ struct dfl {
   float hi, lo;
 };
 
-__host__ __device__ __forceinline__ float f_bits(uint32_t b) {
-#ifdef __CUDA_ARCH__
-  return __uint_as_float(b);
-#else
-  float f;
-  std::memcpy(&f, &b, 4);
-  return f;
-#endif
-}
-__host__ __device__ __forceinline__ uint32_t bits_f(float f) {
-#ifdef __CUDA_ARCH__
-  return __float_as_uint(f);
-#else
-  uint32_t b;
-  std::memcpy(&b, &f, 4);
-  return b;
-#endif
-}
-__host__ __device__ __forceinline__ void d_words(double x, uint32_t* hi, uint32_t* lo) {
-#ifdef __CUDA_ARCH__
-  *hi = (uint32_t)__double2hiint(x);
-  *lo = (uint32_t)__double2loint(x);
-#else
-  uint64_t b;
-  std::memcpy(&b, &x, 8);
-  *hi = (uint32_t)(b >> 32);
-  *lo = (uint32_t)b;
-#endif
-}
-__host__ __device__ __forceinline__ double d_from_words(uint32_t hi, uint32_t lo) {
-#ifdef __CUDA_ARCH__
-  return __hiloint2double((int)hi, (int)lo);
-#else
-  const uint64_t b = ((uint64_t)hi << 32) | lo;
-  double x;
-  std::memcpy(&x, &b, 8);
-  return x;
-#endif
-}
 __host__ __device__ __forceinline__ float fma_f(float a, float b, float c) {
 #ifdef __CUDA_ARCH__
   return __fmaf_rn(a, b, c);
@@ -92,14 +54,6 @@ __host__ __device__ __forceinline__ float mul_f(float a, float b) {
   return a * b;
 #endif
 }
-__host__ __device__ __forceinline__ float u2f(uint32_t r) {
-#ifdef __CUDA_ARCH__
-  return __uint2float_rn(r);
-#else
-  return (float)r;
-#endif
-}
-
 // High word of a double rebiased from exponent 1023 to 127: the exponent
 // field e (bits 20..30) becomes e - 896, the sign bit stays (no borrow for
 // e >= 896).  Both the range test and the split start from it.
@@ -204,16 +158,6 @@ __host__ __device__ __forceinline__ dfl dconst(double c) {
   const float h = (float)c;
   return dfl{h, (float)(c - (double)h)};
 }
-// approximate FP32 reciprocal (the hardware's; any error below 2^-16 will do)
-__host__ __device__ __forceinline__ float rcp_approx(float x) {
-#ifdef __CUDA_ARCH__
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-#else
-  return 1.0f / x;
-#endif
-}
 // 1 / a from r ~ 1/a.hi: the residual e = 1 - a r comes from two FMAs
 // whose roundings are of the size of e itself (2^-24 |e|), and
 // 1/a = r / (1 - e) = r (1 + e + e^2 + ...); keeping e + e^2 leaves
@@ -306,13 +250,20 @@ __host__ __device__ __forceinline__ void collide_df(dfl* f, dfl om_s, dfl om_b) 
   f[11] = sub_lz(eA, oA);
 }
 
-// Relaxation rates of a launch as FP64 (for the fallback) and as pairs.
+// Relaxation rates of a launch as FP64 (for the fallback), as pairs and as
+// the digits of the fixed-point collision.
 struct DfRates {
   double om_s, om_b;
   dfl ps, pb;
+  FxRates fx;
 };
 inline DfRates df_rates(double om_s, double om_b) {
-  return DfRates{om_s, om_b, dconst(om_s), dconst(om_b)};
+  return DfRates{om_s, om_b, dconst(om_s), dconst(om_b), fx_rates(om_s, om_b)};
+}
+// what a kernel over a store of T needs of them (the FP32 store nothing)
+template <typename T>
+inline DfRates rates_of(double om_s, double om_b) {
+  return sizeof(T) == 8 ? df_rates(om_s, om_b) : DfRates{};
 }
 
 // FP64 populations in, FP64 populations out, arithmetic in float pairs;

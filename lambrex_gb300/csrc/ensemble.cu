@@ -176,6 +176,7 @@ int lbx_ensemble_create(int nbox, const int* dims, const double* tau, int precis
     B.par = 0;
     B.om_s = B.om_b = 1.0 / (tau[b] + 0.5);  // src/AmrSim.cpp:125-126
     B.rho0 = precision == LBX_F64 ? 0.0 : 1.0;
+    B.fx = lbx::fx_rates(B.om_s, B.om_b);
     if (!lbx::set_iteration_space(B)) {
       lbx_ensemble_destroy(e);
       return LBX_ERR_UNSUPPORTED;

@@ -183,7 +183,7 @@ cudaError_t launch_explode(const T* coarse, T* fine, const Coupling& c, double o
       return cudaGetLastError();
     }
   }
-  k_explode<T, false><<<grid, 128, 0, st>>>(coarse, fine, c, (T)om_s, (T)om_b, (T)rho0, DfRates{});
+  k_explode<T, false><<<grid, 128, 0, st>>>(coarse, fine, c, (T)om_s, (T)om_b, (T)rho0, rates_of<T>(om_s, om_b));
   return cudaGetLastError();
 }
 
@@ -207,10 +207,10 @@ cudaError_t launch_step_patch(const T* fin, T* fout, const Box3& b, IBox covered
   }
   if (cov)
     k_step_patch<T, true, false><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, (T)om_s, (T)om_b,
-                                                       (T)rho0, DfRates{});
+                                                       (T)rho0, rates_of<T>(om_s, om_b));
   else
     k_step_patch<T, false, false><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, (T)om_s, (T)om_b,
-                                                        (T)rho0, DfRates{});
+                                                        (T)rho0, rates_of<T>(om_s, om_b));
   return cudaGetLastError();
 }
 
@@ -241,7 +241,7 @@ cudaError_t launch_explode_resc(const T* cprev, const T* cnow, T* fine, const Co
     }
   }
   k_explode_resc<T, false><<<grid, 128, 0, st>>>(cprev, cnow, fine, c, (T)om_s, (T)om_b, (T)rho0,
-                                                 (T)wp, (T)wn, DfRates{});
+                                                 (T)wp, (T)wn, rates_of<T>(om_s, om_b));
   return cudaGetLastError();
 }
 
@@ -257,7 +257,7 @@ cudaError_t launch_restrict_resc(const T* fine, T* coarse, const Coupling& c, do
     }
   }
   k_restrict_resc<T, false><<<blocks_for(n, 128), 128, 0, st>>>(fine, coarse, c, (T)om_s, (T)om_b,
-                                                               (T)rho0, DfRates{});
+                                                               (T)rho0, rates_of<T>(om_s, om_b));
   return cudaGetLastError();
 }
 
@@ -308,7 +308,8 @@ cudaError_t launch_f_collide(double* f, const Box3& b, IBox covered, double om_s
   if (paired)
     k_f_collide<true><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b, df_rates(om_s, om_b));
   else
-    k_f_collide<false><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b, DfRates{});
+    k_f_collide<false><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b,
+                                                     df_rates(om_s, om_b));
   return cudaGetLastError();
 }
 cudaError_t launch_f_stream(const double* src, double* dst, const Box3& b, cudaStream_t st) {

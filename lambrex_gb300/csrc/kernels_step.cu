@@ -431,10 +431,10 @@ cudaError_t launch_step_periodic(const T* fin, T* fout, const Box3& b, IBox cove
   }
   if (cov)
     k_step_periodic<T, true, false><<<grid, rl.block, 0, st>>>(fin, fout, b, covered, (T)om_s,
-                                                            (T)om_b, (T)rho0, DfRates{});
+                                                            (T)om_b, (T)rho0, rates_of<T>(om_s, om_b));
   else
     k_step_periodic<T, false, false><<<grid, rl.block, 0, st>>>(fin, fout, b, covered, (T)om_s,
-                                                             (T)om_b, (T)rho0, DfRates{});
+                                                             (T)om_b, (T)rho0, rates_of<T>(om_s, om_b));
   return cudaGetLastError();
 }
 
@@ -526,7 +526,7 @@ cudaError_t launch_step_pull_i(const T* fin, T* fout, const Box3& b, double om_s
     }
   }
   k_step_pull<T, false, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, (T)om_s, (T)om_b, (T)rho0,
-                                                          DfRates{});
+                                                          rates_of<T>(om_s, om_b));
   return cudaGetLastError();
 }
 
@@ -555,7 +555,7 @@ cudaError_t launch_step_pull_hydro_i(const T* fin, T* fout, const Box3& b, doubl
   }
   const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 256);
   k_step_pull_hydro<T, false, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, (T)om_s, (T)om_b,
-                                                               (T)rho0, DfRates{}, rho0, rho, u);
+                                                               (T)rho0, rates_of<T>(om_s, om_b), rho0, rho, u);
   return cudaGetLastError();
 }
 

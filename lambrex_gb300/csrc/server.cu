@@ -192,6 +192,7 @@ int admit(lbx_server* s, Req& q) {
     lv.box.par = s->F[L];  // "now" is store 0 at admission
     lv.box.om_s = lv.box.om_b = 1.0 / (tau + 0.5);
     lv.box.rho0 = rho0;
+    lv.box.fx = lbx::fx_rates(lv.box.om_s, lv.box.om_b);
     tau *= 2.0;  // conservative scheme: viscosity-preserving tau_{l+1} = 2 tau_l
     lv.box.cov = lbx::empty_ibox();
     if (!lbx::set_iteration_space(lv.box)) return LBX_ERR_UNSUPPORTED;
