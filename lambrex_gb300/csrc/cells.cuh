@@ -12,6 +12,9 @@ namespace lbx {
 // value of an empty population (f = 0) in the storage variable
 template <typename T>
 __host__ __device__ __forceinline__ T zero_pop(int q, T rho0) {
+  // an FP64 store is never shifted; FP64 products of its rho0 = 0 kept the
+  // FP64 pipe of a rescaled patch step 16 % busy
+  if constexpr (sizeof(T) == 8) return T(0);
   return rho0 == T(0) ? T(0) : T(-W(q)) * rho0;
 }
 // collision of one cell: the FP32 store's in FP32; an FP64 store's (rho0 is 0
@@ -134,13 +137,23 @@ __host__ __device__ __forceinline__ void cell_step_pull(const T* __restrict__ fi
 }
 
 // rho and u of one cell's populations p (src/AmrSim.cpp:957-971) into the
-// FP64 fields at cell v of n: moments 0..3 from even/odd pairs, in the
-// storage precision (the shifted FP32 values are fluctuations, so FP32 sums
-// keep ~1e-10 of rho)
+// FP64 fields at cell v of n: moments 0..3 from even/odd pairs, in 64-bit
+// fixed point (FP64 store) or in the storage precision (the shifted FP32
+// values are fluctuations, so FP32 sums keep ~1e-10 of rho)
 template <typename T>
 __host__ __device__ __forceinline__ void store_hydro(const T* p, double rho0, double* __restrict__ rho,
                                                     double* __restrict__ u, long long v,
                                                     long long n) {
+  if constexpr (sizeof(T) == 8) {  // in fixed point where that holds the cell (rho0 is 0 here)
+    double m, v3[3];
+    if (rho0 == 0.0 && hydro_fx(p, &m, v3)) {
+      st_cell(rho, v, n, m);
+      st_cell(u, v, 3 * n, v3[0]);
+      st_cell(u, n + v, 3 * n, v3[1]);
+      st_cell(u, 2 * n + v, 3 * n, v3[2]);
+      return;
+    }
+  }
   const T s1 = p[1] + p[2], s3 = p[3] + p[4], s5 = p[5] + p[6];
   const T d7 = p[7] - p[14], d8 = p[8] - p[13], d9 = p[9] - p[12], dA = p[10] - p[11];
   const T D = (p[7] + p[14]) + (p[8] + p[13]) + ((p[9] + p[12]) + (p[10] + p[11]));

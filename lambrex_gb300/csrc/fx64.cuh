@@ -154,37 +154,72 @@ __host__ __device__ __forceinline__ double fx_to_f64_any(int64_t v, int ex) {
   return v < 0 ? -r : r;
 }
 
+// Populations of one cell in units of 2^-57 of the power of two of exponent
+// field E: population = (2^52 | significand) 2^(e - E + 5) units, e its
+// exponent field.  The largest has its leading bit at 57 (58 where it is one
+// power above E); a sign bit, an infinity or a NaN has to be excluded by the
+// caller.
+__host__ __device__ __forceinline__ int64_t fx_unit(uint32_t h, uint32_t l, uint32_t base) {
+  const uint64_t m = ((uint64_t)((h << 11) | (l >> 21) | 0x80000000u) << 32) | (l << 11);
+  return (int64_t)fx_shr(m, (base - h) >> 20);
+}
+__host__ __device__ __forceinline__ uint32_t fx_base(uint32_t E) { return ((E + 6u) << 20) | 0xfffffu; }
+// largest high word of a cell: a sign bit, an infinity or a NaN makes it large
+__host__ __device__ __forceinline__ uint32_t fx_top(const uint32_t* h) {
+  uint32_t top = h[0];
+#pragma unroll
+  for (int q = 1; q < NV; ++q) top = fx_umax(top, h[q]);
+  return top;
+}
+__host__ __device__ __forceinline__ bool fx_top_ok(uint32_t top) {
+  return top - (73u << 20) < (1950u << 20);
+}
+
+// sums of one cell's populations g (units): pair sums and differences and
+// what the collision and the hydrodynamic fields form from them
+struct FxSums {
+  int64_t s1, s3, s5, D, A, rho, jx, jy, jz, Q1, Q2, Q3, Q4;
+};
+__host__ __device__ __forceinline__ FxSums fx_sums(const int64_t* g) {
+  FxSums m;
+  m.s1 = g[1] + g[2];
+  m.s3 = g[3] + g[4];
+  m.s5 = g[5] + g[6];
+  const int64_t s7 = g[7] + g[14], d7 = g[7] - g[14];
+  const int64_t s8 = g[8] + g[13], d8 = g[8] - g[13];
+  const int64_t s9 = g[9] + g[12], d9 = g[9] - g[12];
+  const int64_t sA = g[10] + g[11], dA = g[10] - g[11];
+  m.Q1 = s7 + s8;
+  m.Q2 = s9 + sA;
+  m.Q3 = s7 - s8;
+  m.Q4 = s9 - sA;
+  m.D = m.Q1 + m.Q2;
+  m.A = m.s1 + m.s3 + m.s5;
+  m.rho = g[0] + m.A + m.D;
+  const int64_t P1 = d7 + d8, P2 = d9 + dA, P3 = d7 - d8, P4 = d9 - dA;
+  m.jx = (g[1] - g[2]) + P1 + P2;
+  m.jy = (g[3] - g[4]) + P1 - P2;
+  m.jz = (g[5] - g[6]) + P3 + P4;
+  return m;
+}
+
 // In-place collision; returns false, f untouched, where the cell is left to
 // collide<double>.
 __host__ __device__ __forceinline__ bool collide_fx(double* f, const FxRates& r) {
   uint32_t h[NV], l[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q) d_words(f[q], &h[q], &l[q]);
-  uint32_t top = h[0];
-#pragma unroll
-  for (int q = 1; q < NV; ++q) top = fx_umax(top, h[q]);
-  // a sign bit, an infinity or a NaN makes `top` large
-  bool ok = (r.ok != 0) & (top - (73u << 20) < (1950u << 20));
+  const uint32_t top = fx_top(h);
+  bool ok = (r.ok != 0) & fx_top_ok(top);
   const int E = (int)(top >> 20);
-  // population = (2^52 | significand) 2^(e - E + 5) units, e its exponent field
-  const uint32_t base = (top | 0xfffffu) + (6u << 20);
+  const uint32_t base = fx_base(top >> 20);
   int64_t g[NV];
 #pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    const uint64_t m = ((uint64_t)((h[q] << 11) | (l[q] >> 21) | 0x80000000u) << 32) | (l[q] << 11);
-    g[q] = (int64_t)fx_shr(m, (base - h[q]) >> 20);
-  }
-  const int64_t s1 = g[1] + g[2], d1 = g[1] - g[2];
-  const int64_t s3 = g[3] + g[4], d3 = g[3] - g[4];
-  const int64_t s5 = g[5] + g[6], d5 = g[5] - g[6];
-  const int64_t s7 = g[7] + g[14], d7 = g[7] - g[14];
-  const int64_t s8 = g[8] + g[13], d8 = g[8] - g[13];
-  const int64_t s9 = g[9] + g[12], d9 = g[9] - g[12];
-  const int64_t sA = g[10] + g[11], dA = g[10] - g[11];
-  const int64_t Q1 = s7 + s8, Q2 = s9 + sA, Q3 = s7 - s8, Q4 = s9 - sA;
-  const int64_t D = Q1 + Q2, A = s1 + s3 + s5, rho = g[0] + A + D;
-  const int64_t P1 = d7 + d8, P2 = d9 + dA, P3 = d7 - d8, P4 = d9 - dA;
-  const int64_t jx = d1 + P1 + P2, jy = d3 + P1 - P2, jz = d5 + P3 + P4;
+  for (int q = 0; q < NV; ++q) g[q] = fx_unit(h[q], l[q], base);
+  const FxSums m = fx_sums(g);
+  const int64_t s1 = m.s1, s3 = m.s3, s5 = m.s5, D = m.D, A = m.A, rho = m.rho;
+  const int64_t jx = m.jx, jy = m.jy, jz = m.jz;
+  const int64_t Q1 = m.Q1, Q2 = m.Q2, Q3 = m.Q3, Q4 = m.Q4;
   const int64_t sxy = Q1 - Q2, sxz = Q3 + Q4, syz = Q3 - Q4;
   const int64_t TrS = fx_dbl(D) - g[0];  // trace of the stress: 3 D + A - rho
   {
@@ -263,6 +298,97 @@ __host__ __device__ __forceinline__ bool collide_fx(double* f, const FxRates& r)
     for (int q = 0; q < NV; ++q) f[q] = fx_to_f64_any(g[q], q < 7 ? xa : xd);
   }
   return true;
+}
+
+// Density and velocity of one cell's FP64 populations (src/AmrSim.cpp:957-971)
+// from the exact sums: the density is rounded once, u_a = j_a / rho from j_a
+// rounded once and the series' inverse (relative error below 2^-56), rounded.
+// The FP64 form's 45 additions and its division take 40 clocks of an SM per
+// cell, against 6 for its memory traffic.
+// Cells left to the caller: as the collision, with the density alone in range.
+__host__ __device__ __forceinline__ bool hydro_fx(const double* f, double* rho, double* u) {
+  uint32_t h[NV], l[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) d_words(f[q], &h[q], &l[q]);
+  const uint32_t top = fx_top(h), base = fx_base(top >> 20);
+  int64_t g[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) g[q] = fx_unit(h[q], l[q], base);
+  const FxSums m = fx_sums(g);
+  // rho in [2^58, 2^61): the range of the inverse
+  const bool ok = fx_top_ok(top) & ((uint32_t)(m.rho >> 32) - 0x04000000u < 0x1c000000u);
+  if (!ok) return false;
+  *rho = fx_to_f64(m.rho, (int)(top >> 20) - 26);
+  const int one = 1054;  // exponent field of 2^32 less 1: whole units
+  const double inv = fx_to_f64(fx_inverse(m.rho), one - 121);
+  u[0] = fx_to_f64_any(m.jx, one) * inv;
+  u[1] = fx_to_f64_any(m.jy, one) * inv;
+  u[2] = fx_to_f64_any(m.jz, one) * inv;
+  return true;
+}
+
+// |u| below 1/4 in units of 2^-62
+__host__ __device__ __forceinline__ int64_t fx_velocity(uint32_t h, uint32_t l) {
+  const uint64_t m = ((uint64_t)((h << 11) | (l >> 21) | 0x80000000u) << 32) | (l << 11);
+  const int64_t v = (int64_t)fx_shr(m, 1024u - ((h >> 20) & 2047u));
+  return (int)h < 0 ? -v : v;
+}
+
+// The equilibrium of d3q15.cuh (src/AmrSim.cpp:873-927) in fixed point: the
+// velocity polynomial of each population in units of 2^-60 (exact but for the
+// six products' half units), times 4/9 of the density's significand, every
+// weight being 4/9 times a power of two; one rounding to FP64 follows.  Its
+// FP64 form's 90 instructions take 47 clocks of an SM per cell.  Left to the
+// caller: densities that are not positive and ordinary, |u_a| of 1/4 and more.
+__host__ __device__ __forceinline__ bool equilibrium_fx(double rho, double ux, double uy, double uz,
+                                                        double* out) {
+  uint32_t hr, lr, h[3], l[3];
+  d_words(rho, &hr, &lr);
+  d_words(ux, &h[0], &l[0]);
+  d_words(uy, &h[1], &l[1]);
+  d_words(uz, &h[2], &l[2]);
+  bool ok = hr - (73u << 20) < (1950u << 20);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) ok = ok & ((h[a] & 0x7fffffffu) < (1021u << 20));
+  if (!ok) return false;
+  const int64_t x = fx_velocity(h[0], l[0]), y = fx_velocity(h[1], l[1]), z = fx_velocity(h[2], l[2]);
+  const FxDigits dx = fx_digits(x), dy = fx_digits(y), dz = fx_digits(z);
+  const int64_t xx = fx_mul(dx, dx), yy = fx_mul(dy, dy), zz = fx_mul(dz, dz);
+  const int64_t xy9 = fx_mul(dx, dy) * 9, xz9 = fx_mul(dx, dz) * 9, yz9 = fx_mul(dy, dz) * 9;
+  const int64_t ax = (x * 3) >> 2, ay = (y * 3) >> 2, az = (z * 3) >> 2;  // 3 u_a
+  const int64_t m2 = (xx + yy + zz) * 3;                                // 3 u^2
+  const int64_t one = int64_t(1) << 60;
+  const int64_t r0 = one - (m2 >> 1), d0 = one + m2;
+  const int64_t bx = r0 + ((xx * 9) >> 1), by = r0 + ((yy * 9) >> 1), bz = r0 + ((zz * 9) >> 1);
+  // 4/9 of the significand at 2^61
+  const int64_t sig = (int64_t)(((uint64_t)((hr & 0xfffffu) | 0x100000u) << 41) | ((uint64_t)lr << 9));
+  const FxDigits four_ninths{0x71c71c72, (int)0xc71c71c7u};  // 8/9 of 2^63
+  const FxDigits w = fx_digits(fx_mul(sig, four_ninths));
+  const int e = (int)(hr >> 20);
+  out[0] = fx_to_f64(fx_mul(r0, w), e - 27);
+  out[1] = fx_to_f64(fx_mul(bx + ax, w), e - 28);
+  out[2] = fx_to_f64(fx_mul(bx - ax, w), e - 28);
+  out[3] = fx_to_f64(fx_mul(by + ay, w), e - 28);
+  out[4] = fx_to_f64(fx_mul(by - ay, w), e - 28);
+  out[5] = fx_to_f64(fx_mul(bz + az, w), e - 28);
+  out[6] = fx_to_f64(fx_mul(bz - az, w), e - 28);
+  const int64_t e7 = d0 + xy9 + (xz9 + yz9), e8 = d0 + xy9 - (xz9 + yz9);
+  const int64_t e9 = d0 - xy9 + (xz9 - yz9), eA = d0 - xy9 - (xz9 - yz9);
+  const int64_t o7 = ax + ay + az, o8 = ax + ay - az, o9 = ax - ay + az, oA = ax - ay - az;
+  out[7] = fx_to_f64(fx_mul(e7 + o7, w), e - 31);
+  out[14] = fx_to_f64(fx_mul(e7 - o7, w), e - 31);
+  out[8] = fx_to_f64(fx_mul(e8 + o8, w), e - 31);
+  out[13] = fx_to_f64(fx_mul(e8 - o8, w), e - 31);
+  out[9] = fx_to_f64(fx_mul(e9 + o9, w), e - 31);
+  out[12] = fx_to_f64(fx_mul(e9 - o9, w), e - 31);
+  out[10] = fx_to_f64(fx_mul(eA + oA, w), e - 31);
+  out[11] = fx_to_f64(fx_mul(eA - oA, w), e - 31);
+  return true;
+}
+// in fixed point, or in FP64 where that does not hold the cell
+__host__ __device__ __forceinline__ void equilibrium_f64(double rho, double ux, double uy, double uz,
+                                                         double* out) {
+  if (!equilibrium_fx(rho, ux, uy, uz, out)) equilibrium(rho, ux, uy, uz, out);
 }
 
 // The FP64 collision of one cell: in fixed point, or with FP64 instructions

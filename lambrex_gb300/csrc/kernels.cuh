@@ -124,7 +124,7 @@ cudaError_t launch_copy_in(const double* in, T* f, const Box3& b, double rho0, c
 // Compensated FP64 sums over the valid region minus `skip`:
 // out4 = {sum f, sum cx f, sum cy f, sum cz f}.  `partials` must hold
 // reduce_partials_doubles() doubles; the kernels write every entry they read.
-constexpr int kReduceBlocks = 512;
+constexpr int kReduceBlocks = 512;  // at most; the launches use three per SM
 constexpr int kReduceThreads = 256;
 inline size_t reduce_partials_doubles() { return (size_t)kReduceBlocks * 8; }
 template <typename T>

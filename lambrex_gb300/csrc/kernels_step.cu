@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "cells.cuh"
+#include "sums.cuh"
 
 namespace lbx {
 
@@ -96,7 +97,7 @@ __global__ void k_equilibrium(const double* __restrict__ rho, const double* __re
     for (int q = 0; q < NV; ++q) st_pop(f, q * b.sq + c, b, g[q]);
   } else {
     double e[NV];
-    equilibrium(r, ux, uy, uz, e);
+    equilibrium_f64(r, ux, uy, uz, e);
 #pragma unroll
     for (int q = 0; q < NV; ++q) st_pop(f, q * b.sq + c, b, (T)(e[q] - W(q) * rho0));
   }
@@ -119,7 +120,7 @@ __global__ void k_init_pulse(T* __restrict__ f, Box3 b, int axis, int index, dou
     for (int q = 0; q < NV; ++q) st_pop(f, q * b.sq + s, b, g[q]);
   } else {
     double e[NV];
-    equilibrium(rho, 0.0, 0.0, 0.0, e);
+    equilibrium_f64(rho, 0.0, 0.0, 0.0, e);
 #pragma unroll
     for (int q = 0; q < NV; ++q) st_pop(f, q * b.sq + s, b, (T)(e[q] - W(q) * rho0));
   }
@@ -190,156 +191,229 @@ __global__ void k_unpack(const T* __restrict__ in, T* __restrict__ f, Box3 b) {
   for (int q = 0; q < NV; ++q) st_pop(f, q * b.sq + c, b, ld_cell(in, q * n + v, NV * n));
 }
 
-// Neumaier-compensated pair (s, e): value = s + e.
-struct Comp {
-  double s, e;
+// Mass and momentum sums.  What bounds them is the bytes of the store as long
+// as the FP64 pipe is kept out of it (sums.cuh): with FP64 additions per
+// population 161x128x95 FP64 took 348 us and its second pass 24.6 us, against
+// 35 us for the store's 235 MB.
+//
+// FP64 store: a cell's populations are brought to one exponent, that of the
+// block's first cell, summed exactly in 64-bit integers (fx64.cuh) and added
+// to the thread's 128-bit sums.  Cells of another scale (largest population
+// more than a factor of two away), or with a negative one, are summed with
+// FP64 instructions, compensated; a block that met any adds both sums.
+template <bool FLAT>
+__device__ __forceinline__ bool reduce_cell(const Box3& b, const IBox& skip, unsigned v,
+                                            long long* c) {
+  if (FLAT) {  // no ghost cells, nothing left out: the store in order
+    *c = v;
+    return true;
+  }
+  const unsigned n0 = (unsigned)b.n[0], n1 = (unsigned)b.n[1], r = v / n0;
+  const int x = (int)(v - r * n0), y = (int)(r % n1), z = (int)(r / n1);
+  *c = b.at(x, y, z);
+  return !skip.contains(x, y, z);
+}
+
+template <bool FLAT>
+__device__ __forceinline__ void reduce_cells(const double* __restrict__ f, const Box3& b,
+                                             const IBox& skip, unsigned n, double rho0,
+                                             Sum4Shared& sh, double* __restrict__ out8) {
+  uint32_t E;  // of the block's first cell (b.at(0, 0, 0) + its place, ghost or left out or not)
+  {
+    uint32_t h[NV], l[NV];
+    long long c;
+    reduce_cell<FLAT>(b, skip, min(blockIdx.x * blockDim.x, n - 1u), &c);
+#pragma unroll
+    for (int q = 0; q < NV; ++q) d_words(ld_pop(f, q * b.sq + c, b), &h[q], &l[q]);
+    const uint32_t top = fx_top(h);
+    E = fx_top_ok(top) ? top >> 20 : 1020u;
+  }
+  const uint32_t base = fx_base(E);
+  i128 t[4] = {0, 0, 0, 0};
+  Comp acc[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+  bool odd = false;
+  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    long long c;
+    if (!reduce_cell<FLAT>(b, skip, v, &c)) continue;
+    double p[NV];
+    uint32_t h[NV], l[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      p[q] = ld_pop(f, q * b.sq + c, b);
+      d_words(p[q], &h[q], &l[q]);
+    }
+    const uint32_t top = fx_top(h);
+    // exponent E - 1, E or E + 1: units of E hold the sums (below 2^63)
+    if (fx_top_ok(top) & ((top >> 20) + 1u - E < 3u)) {
+      int64_t g[NV];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) g[q] = fx_unit(h[q], l[q], base);
+      const FxSums m = fx_sums(g);
+      t[0] += m.rho;
+      t[1] += m.jx;
+      t[2] += m.jy;
+      t[3] += m.jz;
+    } else {
+      odd = true;
+      double m = rho0, j[3] = {0, 0, 0};
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        m += p[q];
+        if (CX(q)) j[0] += CX(q) * p[q];
+        if (CY(q)) j[1] += CY(q) * p[q];
+        if (CZ(q)) j[2] += CZ(q) * p[q];
+      }
+      comp_add(acc[0], m);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) comp_add(acc[1 + a], j[a]);
+    }
+  }
+  const bool any = __syncthreads_or(odd);
+  Comp s = sum_pair(block_sum4(t, sh), (int)E - 1023 - 57);
+  if (any) {
+    __syncthreads();
+    const Comp o = block_sum4(acc, sh);
+    comp_add(s, o.s);
+    s.e += o.e;
+  }
+  if (threadIdx.x < 32 && (threadIdx.x & 7) == 0) {
+    out8[2 * (threadIdx.x >> 3)] = s.s;
+    out8[2 * (threadIdx.x >> 3) + 1] = s.e;
+  }
+}
+
+// FP32 store: the shifted populations are small; each cell's sums in FP32
+// (rounding ~1e-9 of the fluctuations), a thread's cells summed with two
+// levels of FP32 compensation (error of order 2^-72; one FP64 addition and
+// one conversion per value took 34 clocks of an SM per warp, four of them
+// more than the 15 loads), the threads' sums exactly; the mass is rho0 per
+// cell plus the fluctuations.
+struct Comp3 {
+  float s, c, cc;
 };
-__device__ __forceinline__ void comp_add(Comp& a, double v) {
-  const double t = a.s + v;
-  if (fabs(a.s) >= fabs(v))
-    a.e += (a.s - t) + v;
-  else
-    a.e += (v - t) + a.s;
-  a.s = t;
+__device__ __forceinline__ void comp_add(Comp3& a, float v) {
+  const dfl t = two_sum(a.s, v);
+  const dfl w = two_sum(a.c, t.lo);
+  a.s = t.hi;
+  a.c = w.hi;
+  a.cc = add_f(a.cc, w.lo);
 }
-__device__ __forceinline__ void comp_merge(Comp& a, const Comp& b) {
-  comp_add(a, b.s);
-  a.e += b.e;
+__device__ __forceinline__ Comp comp_of(const Comp3& a) {
+  return Comp{(double)a.s, (double)a.c + (double)a.cc};
 }
-
-// Block-level reduction of four compensated sums with warp shuffles.
-__device__ __forceinline__ void block_reduce4(Comp* acc, double* out8) {
-  __shared__ double sh[8][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+template <bool FLAT>
+__device__ __forceinline__ void reduce_cells(const float* __restrict__ f, const Box3& b,
+                                             const IBox& skip, unsigned n, double rho0,
+                                             Sum4Shared& sh, double* __restrict__ out8) {
+  Comp3 t[4] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+  unsigned cells = 0;
+  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    long long c;
+    if (!reduce_cell<FLAT>(b, skip, v, &c)) continue;
+    float s = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      Comp other{__shfl_down_sync(0xffffffffu, acc[k].s, o),
-                 __shfl_down_sync(0xffffffffu, acc[k].e, o)};
-      comp_merge(acc[k], other);
+    for (int q = 0; q < NV; ++q) {
+      const float fq = ld_pop(f, q * b.sq + c, b);
+      s += fq;
+      if (CX(q)) sx += CX(q) * fq;
+      if (CY(q)) sy += CY(q) * fq;
+      if (CZ(q)) sz += CZ(q) * fq;
     }
+    comp_add(t[0], s);
+    comp_add(t[1], sx);
+    comp_add(t[2], sy);
+    comp_add(t[3], sz);
+    ++cells;
   }
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      sh[2 * k][warp] = acc[k].s;
-      sh[2 * k + 1][warp] = acc[k].e;
-    }
-  }
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      Comp c{lane < nw ? sh[2 * k][lane] : 0.0, lane < nw ? sh[2 * k + 1][lane] : 0.0};
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        Comp other{__shfl_down_sync(0xffffffffu, c.s, o), __shfl_down_sync(0xffffffffu, c.e, o)};
-        comp_merge(c, other);
-      }
-      if (lane == 0) {
-        out8[2 * k] = c.s;
-        out8[2 * k + 1] = c.e;
-      }
-    }
+  Comp acc[4] = {comp_of(t[0]), comp_of(t[1]), comp_of(t[2]), comp_of(t[3])};
+  comp_add(acc[0], rho0 * (double)cells);
+  const Comp s = block_sum4(acc, sh);
+  if (threadIdx.x < 32 && (threadIdx.x & 7) == 0) {
+    out8[2 * (threadIdx.x >> 3)] = s.s;
+    out8[2 * (threadIdx.x >> 3) + 1] = s.e;
   }
 }
 
-template <typename T>
+template <typename T, bool FLAT>
 __global__ void __launch_bounds__(kReduceThreads) k_reduce(const T* __restrict__ f, Box3 b,
                                                            IBox skip, double rho0,
                                                            double* __restrict__ partials) {
   if (!idx_ok(blockIdx.x, kReduceBlocks)) return;  // partials hold kReduceBlocks blocks
-  Comp acc[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+  __shared__ Sum4Shared sh;
   // cell counts of every caller are below 2^31 (checked on the host), so the
   // index arithmetic stays in 32 bits
   const unsigned n = (unsigned)((long long)b.n[0] * b.n[1] * b.n[2]);
-  const unsigned n0 = (unsigned)b.n[0], n1 = (unsigned)b.n[1];
-  if constexpr (sizeof(T) == 4) {
-    // the FP32 store's shifted populations are small: each cell's sums in
-    // FP32 (rounding ~1e-9 of the fluctuations), a thread's few hundred
-    // cells summed plainly in FP64 (~1e-14), the threads' and blocks' sums
-    // merged compensated; the mass is rho0 per cell plus the fluctuations
-    double t[4] = {0.0, 0.0, 0.0, 0.0};
-    unsigned cells = 0;
-    for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-      const unsigned r = v / n0;
-      const int x = (int)(v - r * n0);
-      const int y = (int)(r % n1);
-      const int z = (int)(r / n1);
-      if (skip.contains(x, y, z)) continue;
-      const long long c = b.at(x, y, z);
-      float s = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
-#pragma unroll
-      for (int q = 0; q < NV; ++q) {
-        const float fq = (float)ld_pop(f, q * b.sq + c, b);
-        s += fq;
-        if (CX(q)) sx += CX(q) * fq;
-        if (CY(q)) sy += CY(q) * fq;
-        if (CZ(q)) sz += CZ(q) * fq;
-      }
-      t[0] += (double)s;
-      t[1] += (double)sx;
-      t[2] += (double)sy;
-      t[3] += (double)sz;
-      ++cells;
-    }
-    acc[0].s = rho0 * (double)cells;
-    comp_add(acc[0], t[0]);
-    for (int k = 1; k < 4; ++k) acc[k].s = t[k];
-  } else {
-    for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-      const unsigned r = v / n0;
-      const int x = (int)(v - r * n0);
-      const int y = (int)(r % n1);
-      const int z = (int)(r / n1);
-      if (skip.contains(x, y, z)) continue;
-      const long long c = b.at(x, y, z);
-      double m = rho0, jx = 0, jy = 0, jz = 0;
-#pragma unroll
-      for (int q = 0; q < NV; ++q) {
-        const double fq = (double)ld_pop(f, q * b.sq + c, b);
-        m += fq;
-        if (CX(q)) jx += CX(q) * fq;
-        if (CY(q)) jy += CY(q) * fq;
-        if (CZ(q)) jz += CZ(q) * fq;
-      }
-      comp_add(acc[0], m);
-      comp_add(acc[1], jx);
-      comp_add(acc[2], jy);
-      comp_add(acc[3], jz);
-    }
-  }
-  block_reduce4(acc, partials + 8 * blockIdx.x);
+  reduce_cells<FLAT>(f, b, skip, n, rho0, sh, partials + 8 * blockIdx.x);
 }
 
-__global__ void k_reduce_final(const double* __restrict__ partials, int nblocks,
-                               double* __restrict__ out4) {
-  Comp acc[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-  for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
+// the blocks' pairs: one block, a chain of latencies (24.6 us as compensated
+// FP64 additions)
+__global__ void __launch_bounds__(kReduceThreads) k_reduce_final(const double* __restrict__ partials,
+                                                                int nblocks,
+                                                                double* __restrict__ out4) {
+  __shared__ Sum4Shared sh;
+  static_assert(kReduceBlocks <= 2 * kReduceThreads, "two pairs a thread");
+  const int i = threadIdx.x, j = i + kReduceThreads;
+  Comp acc[4], more[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) comp_merge(acc[k], Comp{partials[8 * i + 2 * k], partials[8 * i + 2 * k + 1]});
+  for (int k = 0; k < 4; ++k) {
+    acc[k] = i < nblocks ? Comp{partials[8 * i + 2 * k], partials[8 * i + 2 * k + 1]} : Comp{0, 0};
+    more[k] = j < nblocks ? Comp{partials[8 * j + 2 * k], partials[8 * j + 2 * k + 1]} : Comp{0, 0};
   }
-  __shared__ double res[8];
-  block_reduce4(acc, res);
-  __syncthreads();
-  if (threadIdx.x < 4) out4[threadIdx.x] = res[2 * threadIdx.x] + res[2 * threadIdx.x + 1];
+  Comp s = block_sum4(acc, sh);
+  if (nblocks > kReduceThreads) {
+    __syncthreads();
+    const Comp o = block_sum4(more, sh);
+    comp_add(s, o.s);
+    s.e += o.e;
+  }
+  if (threadIdx.x < 32 && (threadIdx.x & 7) == 0) out4[threadIdx.x >> 3] = s.s + s.e;
 }
 
-// sum of n doubles (the mean density that shifts an FP32 store): each
-// thread adds its strided values with one FP64 addition each (n / 131,072
-// values, ~1e-13 relative), the threads' and blocks' sums merge compensated;
-// the order is fixed, so the sum is the same on every run
+// sum of n doubles (the mean density that shifts an FP32 store): values
+// within a factor of two of the block's first in 128-bit integers, others
+// compensated in FP64; the order of the blocks is fixed and each block's sum
+// exact, so the sum is the same on every run
 __global__ void __launch_bounds__(kReduceThreads) k_sum(const double* __restrict__ x, size_t n,
                                                        double* __restrict__ partials) {
   if (!idx_ok(blockIdx.x, kReduceBlocks)) return;
-  double t = 0.0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    t += ld_cell(x, (long long)i, (long long)n);
-  Comp acc[4] = {{t, 0}, {0, 0}, {0, 0}, {0, 0}};
-  block_reduce4(acc, partials + 8 * blockIdx.x);
+  __shared__ Sum4Shared sh;
+  const size_t first = blockIdx.x * (size_t)blockDim.x, step = (size_t)gridDim.x * blockDim.x;
+  uint32_t h, l;
+  d_words(ld_cell(x, (long long)(first < n ? first : n - 1), (long long)n), &h, &l);
+  const uint32_t E = fx_top_ok(h) ? h >> 20 : 1023u, base = fx_base(E);
+  i128 t[4] = {0, 0, 0, 0};
+  Comp acc[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+  bool odd = false;
+  constexpr int kAhead = 4;  // loads in flight per thread
+  for (size_t i = first + threadIdx.x; i < n; i += kAhead * step) {
+    double v[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      v[k] = i + k * step < n ? ld_cell(x, (long long)(i + k * step), (long long)n) : 0.0;
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      d_words(v[k], &h, &l);
+      if (fx_top_ok(h) & ((h >> 20) + 1u - E < 3u)) {
+        t[0] += fx_unit(h, l, base);
+      } else if (h | l) {
+        odd = true;
+        comp_add(acc[0], v[k]);
+      }
+    }
+  }
+  const bool any = __syncthreads_or(odd);
+  Comp s = sum_pair(block_sum4(t, sh), (int)E - 1023 - 57);
+  if (any) {
+    __syncthreads();
+    const Comp o = block_sum4(acc, sh);
+    comp_add(s, o.s);
+    s.e += o.e;
+  }
+  if (threadIdx.x < 32 && (threadIdx.x & 7) == 0) {
+    partials[8 * blockIdx.x + 2 * (threadIdx.x >> 3)] = s.s;
+    partials[8 * blockIdx.x + 2 * (threadIdx.x >> 3) + 1] = s.e;
+  }
 }
 
 __global__ void k_fill(double* __restrict__ p, size_t n, double v) {
@@ -396,9 +470,17 @@ cudaError_t launch_c_to_fab(const double* rho_c, const double* u_c, double* rho,
   return cudaGetLastError();
 }
 
+// blocks of a sum over n values: three to each of the 152 SMs, fewer where a
+// thread would have no value
+static int reduce_grid(long long n) {
+  const long long blocks = (n + kReduceThreads - 1) / kReduceThreads;
+  return (int)std::min<long long>(std::max<long long>(blocks, 1), 152 * 3);
+}
+
 cudaError_t launch_sum(const double* x, size_t n, double* partials, double* out4, cudaStream_t st) {
-  k_sum<<<kReduceBlocks, kReduceThreads, 0, st>>>(x, n, partials);
-  k_reduce_final<<<1, kReduceThreads, 0, st>>>(partials, kReduceBlocks, out4);
+  const int grid = reduce_grid((long long)n);
+  k_sum<<<grid, kReduceThreads, 0, st>>>(x, n, partials);
+  k_reduce_final<<<1, kReduceThreads, 0, st>>>(partials, grid, out4);
   return cudaGetLastError();
 }
 
@@ -620,8 +702,13 @@ cudaError_t launch_unpack(const T* in, T* f, const Box3& b, cudaStream_t st) {
 template <typename T>
 cudaError_t launch_reduce(const T* f, const Box3& b, IBox skip, double rho0, double* partials,
                           double* out4, cudaStream_t st) {
-  k_reduce<T><<<kReduceBlocks, kReduceThreads, 0, st>>>(f, b, skip, rho0, partials);
-  k_reduce_final<<<1, kReduceThreads, 0, st>>>(partials, kReduceBlocks, out4);
+  const int grid = reduce_grid((long long)b.n[0] * b.n[1] * b.n[2]);
+  const bool none = skip.hi[0] < skip.lo[0] || skip.hi[1] < skip.lo[1] || skip.hi[2] < skip.lo[2];
+  if (b.g == 0 && none)
+    k_reduce<T, true><<<grid, kReduceThreads, 0, st>>>(f, b, skip, rho0, partials);
+  else
+    k_reduce<T, false><<<grid, kReduceThreads, 0, st>>>(f, b, skip, rho0, partials);
+  k_reduce_final<<<1, kReduceThreads, 0, st>>>(partials, grid, out4);
   return cudaGetLastError();
 }
 
