@@ -41,10 +41,10 @@ extern "C" {
 /* precision of the distribution store */
 #define LBX_F64 0              /* FP64 drop-in                              */
 #define LBX_F32_SHIFTED 1      /* FP32 populations f_i - w_i rho0           */
-#define LBX_F64_PAIRED 2       /* FP64 store; every collision is carried in
-                                  pairs of FP32 values (48-bit significand)
-                                  on the FP32 pipe, within the same 1e-12 of
-                                  the reference order as LBX_F64             */
+#define LBX_F64_PAIRED 2       /* FP64 store, within the same 1e-12 of the
+                                  reference order as LBX_F64: refined runs
+                                  collide in pairs of FP32 values (48-bit
+                                  significand), single levels in fixed point */
 
 /* multi-level coupling */
 #define LBX_AMR_FAITHFUL 0     /* the reference's Rohde cycle, quirks kept;
@@ -173,9 +173,7 @@ int lbx_get_device_f(lbx_sim* sim, int level, void** ptr, int* storage_dims3, in
  * (src/AmrSim.cpp:25-135, include/component.h:22-29). */
 int lbx_step_periodic_f64(const double* f_in, double* f_out, int nx, int ny, int nz,
                           double tau_s, double tau_b, void* stream);
-/* FP64 store, collision in paired FP32 arithmetic (LBX_F64_PAIRED) in its
- * one-cell scalar form, which the simulation's packed form reproduces bit
- * for bit */
+/* the same with the collision of LBX_F64_PAIRED */
 int lbx_step_periodic_f64p(const double* f_in, double* f_out, int nx, int ny, int nz,
                            double tau_s, double tau_b, void* stream);
 /* FP32 shifted populations g = f - w rho0 */

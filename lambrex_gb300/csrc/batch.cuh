@@ -112,10 +112,10 @@ cudaError_t launch_b_step(const BBox* boxes, const BTile* tiles, int ntiles, int
 // AMR levels of the batch engine in the pull form: a box's store `f` into
 // it in place (after initialisation in the streamed state), and back (the
 // streamed state gathered from the store before the last step into the
-// latest one)
+// latest one); refined: a level of several (collide_f64)
 template <typename T>
 cudaError_t launch_b_to_qform(T* f, const Box3& b, const IBox& cov, double om_s, double om_b,
-                              double rho0, cudaStream_t st);
+                              double rho0, bool refined, cudaStream_t st);
 template <typename T>
 cudaError_t launch_b_to_rform(const T* qprev, T* r, const Box3& b, cudaStream_t st);
 // explode / coalesce over coupling tiles; flip_c / flip_f select

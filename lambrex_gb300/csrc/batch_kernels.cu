@@ -158,9 +158,10 @@ int conversion_blocks(const Box3& b) {
 
 template <typename T>
 cudaError_t launch_b_to_qform(T* f, const Box3& b, const IBox& cov, double om_s, double om_b,
-                              double rho0, cudaStream_t st) {
+                              double rho0, bool refined, cudaStream_t st) {
+  const DfRates r = rates_of<T>(om_s, om_b);
   k_b_to_qform<T><<<conversion_blocks(b), 256, 0, st>>>(f, b, cov, (T)om_s, (T)om_b, (T)rho0,
-                                                       rates_of<T>(om_s, om_b));
+                                                       refined ? quiet(r) : r);
   return cudaGetLastError();
 }
 
@@ -219,7 +220,7 @@ cudaError_t launch_b_coalesce(const BBox* boxes, const BCoupling* cps, const BTi
   template cudaError_t launch_b_coalesce<T>(const BBox*, const BCoupling*, const BTile*, int,   \
                                             int, int, cudaStream_t);                            \
   template cudaError_t launch_b_to_qform<T>(T*, const Box3&, const IBox&, double, double, double,\
-                                            cudaStream_t);                                      \
+                                            bool, cudaStream_t);                                      \
   template cudaError_t launch_b_to_rform<T>(const T*, T*, const Box3&, cudaStream_t);
 LBX_INST(double)
 LBX_INST(float)

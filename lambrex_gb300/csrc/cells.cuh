@@ -18,15 +18,15 @@ __host__ __device__ __forceinline__ T zero_pop(int q, T rho0) {
   return rho0 == T(0) ? T(0) : T(-W(q)) * rho0;
 }
 // collision of one cell: the FP32 store's in FP32; an FP64 store's (rho0 is 0
-// there) in 64-bit fixed point (fx64.cuh; with FP64 instructions where r.fx
-// was not given), or in paired FP32 arithmetic with its twin operations
-// packed (df32.cuh)
-template <typename T, bool PAIRED>
+// there) in 64-bit fixed point (fx64.cuh), or in paired FP32 arithmetic with
+// its twin operations packed (df32.cuh, see collides_in_pairs)
+// (QUIET: on the levels of refined runs, see collide_f64)
+template <typename T, bool PAIRED, bool QUIET = false>
 __host__ __device__ __forceinline__ void collide_cell(T* f, T om_s, T om_b, T rho0, const DfRates& r) {
   if constexpr (PAIRED)
     collide_f64_via_df_w(f, r);
   else if constexpr (sizeof(T) == 8)
-    collide_f64(f, om_s, om_b, r.fx);
+    collide_f64<QUIET>(f, om_s, om_b, r.fx);
   else
     collide<T>(f, om_s, om_b, rho0);
 }
@@ -93,7 +93,7 @@ __host__ __device__ __forceinline__ void cell_step_periodic(const T* __restrict_
     const I c = sidx_i<I>(b, x + b.g, y + b.g, z + b.g), sq = (I)b.sq;
 #pragma unroll
     for (int q = 0; q < NV; ++q) f[q] = ld_pop(fin, (I)q * sq + c, b);
-    collide_cell<T, PAIRED>(f, om_s, om_b, rho0, r);
+    collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);
   }
   push_periodic<T, I>(fout, b, x, y, z, f);
 }
@@ -124,13 +124,13 @@ __host__ __device__ __forceinline__ void gather_periodic(const T* __restrict__ f
     f[q] = ld_pop(fin, (I)q * sq + oz[CZ(q) + 1] + oy[CY(q) + 1] + ox[CX(q) + 1], b);
 }
 
-template <typename T, bool PAIRED, typename I = long long>
+template <typename T, bool PAIRED, typename I = long long, bool QUIET = false>
 __host__ __device__ __forceinline__ void cell_step_pull(const T* __restrict__ fin, T* __restrict__ fout,
                                                const Box3& b, int x, int y, int z, T om_s, T om_b,
                                                T rho0, const DfRates& r) {
   T f[NV];
   gather_periodic<T, 1, I>(fin, b, x, y, z, f);
-  collide_cell<T, PAIRED>(f, om_s, om_b, rho0, r);
+  collide_cell<T, PAIRED, QUIET>(f, om_s, om_b, rho0, r);
   const I c = sidx_i<I>(b, x + b.g, y + b.g, z + b.g), sq = (I)b.sq;
 #pragma unroll
   for (int q = 0; q < NV; ++q) st_pop(fout, (I)q * sq + c, b, f[q]);
@@ -262,7 +262,7 @@ __host__ __device__ __forceinline__ void cell_step_patch(const T* __restrict__ f
   } else {
 #pragma unroll
     for (int q = 0; q < NV; ++q) f[q] = ld_pop(fin, (I)q * sq + c, b);
-    if (valid) collide_cell<T, PAIRED>(f, om_s, om_b, rho0, r);
+    if (valid) collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);
   }
   const int SX = b.n[0] + 2 * g, SY = b.n[1] + 2 * g, SZ = b.n[2] + 2 * g;
   if (sx > 0 && sx < SX - 1 && sy > 0 && sy < SY - 1 && sz > 0 && sz < SZ - 1) {
@@ -305,7 +305,7 @@ __host__ __device__ __forceinline__ void cell_step_periodic_pull(const T* __rest
     for (int q = 0; q < NV; ++q) st_pop(fout, (I)q * sq + c, b, zero_pop<T>(q, rho0));
     return;
   }
-  cell_step_pull<T, false, I>(fin, fout, b, x, y, z, om_s, om_b, rho0, r);
+  cell_step_pull<T, false, I, true>(fin, fout, b, x, y, z, om_s, om_b, rho0, r);
 }
 
 // AMR patch, storage cell (sx,sy,sz) of the grown box: sources outside the
@@ -341,7 +341,7 @@ __host__ __device__ __forceinline__ void cell_step_patch_pull(const T* __restric
                  : zero_pop<T>(q, rho0);
     }
   }
-  if (valid) collide_cell<T, false>(f, om_s, om_b, rho0, r);
+  if (valid) collide_cell<T, false, true>(f, om_s, om_b, rho0, r);
 #pragma unroll
   for (int q = 0; q < NV; ++q) st_pop(fout, (I)q * sq + c, b, f[q]);
 }
@@ -363,7 +363,7 @@ __host__ __device__ __forceinline__ void cell_to_qform(T* __restrict__ f, const 
   } else {
 #pragma unroll
     for (int q = 0; q < NV; ++q) p[q] = ld_pop(f, (I)q * sq + c, b);
-    collide_cell<T, false>(p, om_s, om_b, rho0, r);
+    collide_cell<T, false, true>(p, om_s, om_b, rho0, r);
   }
 #pragma unroll
   for (int q = 0; q < NV; ++q) st_pop(f, (I)q * sq + c, b, p[q]);
@@ -409,7 +409,7 @@ __host__ __device__ __forceinline__ void cell_explode(const T* __restrict__ coar
   T f[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q) f[q] = ld_pop(coarse, (I)q * csq + cc, c.cb);
-  if (!QFORM) collide_cell<T, PAIRED>(f, om_s, om_b, rho0, r);
+  if (!QFORM) collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);
   const I fc = sidx_i<I>(c.fb, sx, sy, sz);
 #pragma unroll
   for (int q = 0; q < NV; ++q) {
@@ -447,14 +447,14 @@ __host__ __device__ __forceinline__ void cell_explode_resc(const T* __restrict__
   T a[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q) a[q] = ld_pop(cprev, (I)q * csq + cc, c.cb);
-  collide_cell<T, PAIRED>(a, om_s, om_b, rho0, r);
+  collide_cell<T, PAIRED, true>(a, om_s, om_b, rho0, r);
   if (wn != T(0)) {
     T b[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) b[q] = ld_pop(cnow, (I)q * csq + cc, c.cb);
-    collide_cell<T, PAIRED>(b, om_s, om_b, rho0, r);
+    collide_cell<T, PAIRED, true>(b, om_s, om_b, rho0, r);
 #pragma unroll
-    for (int q = 0; q < NV; ++q) a[q] = wp * a[q] + wn * b[q];
+    for (int q = 0; q < NV; ++q) a[q] = weighted(wp, a[q], wn, b[q]);
   }
   const I fc = sidx_i<I>(c.fb, sx, sy, sz);
 #pragma unroll
@@ -485,9 +485,9 @@ __host__ __device__ __forceinline__ void cell_restrict_resc(const T* __restrict_
                     (I)q * fsq + sidx_i<I>(c.fb, 2 * rx + (m & 1) + g, 2 * ry + ((m >> 1) & 1) + g,
                                            2 * rz + (m >> 2) + g),
                     c.fb);
-    f[q] = T(0.125) * (((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+    f[q] = mean8(v);
   }
-  collide_cell<T, PAIRED>(f, om_s, om_b, rho0, r);
+  collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);
 #pragma unroll
   for (int q = 0; q < NV; ++q) st_pop(coarse, (I)q * csq + cc, c.cb, f[q]);
 }
@@ -619,8 +619,7 @@ __host__ __device__ __forceinline__ void cell_restrict(const T* __restrict__ fin
                     (I)q * fsq + sidx_i<I>(c.fb, 2 * rx + (m & 1) + g, 2 * ry + ((m >> 1) & 1) + g,
                                            2 * rz + (m >> 2) + g),
                     c.fb);
-    st_pop(coarse, (I)q * csq + cc, c.cb,
-           T(0.125) * (((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]))));
+    st_pop(coarse, (I)q * csq + cc, c.cb, mean8(v));
   }
 }
 

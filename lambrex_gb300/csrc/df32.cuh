@@ -260,6 +260,11 @@ struct DfRates {
 inline DfRates df_rates(double om_s, double om_b) {
   return DfRates{om_s, om_b, dconst(om_s), dconst(om_b), fx_rates(om_s, om_b)};
 }
+// rates of a level of a refined run (collide_f64)
+inline DfRates quiet(DfRates r) {
+  r.fx.quiet = 1;
+  return r;
+}
 // what a kernel over a store of T needs of them (the FP32 store nothing)
 template <typename T>
 inline DfRates rates_of(double om_s, double om_b) {
@@ -485,5 +490,15 @@ __host__ __device__ __forceinline__ void collide_f64_via_df_w(double* f, const D
     for (int q = 0; q < NV; ++q) f[q] = join(g[q]);
   }
 }
+
+// Whether a single level of LBX_F64_PAIRED collides in pairs at these rates:
+// the fixed point (fx64.cuh) takes fewer instructions (1,090 against 1,340 per
+// cell; 251x190x133: 253 us a step against 289) and rounds less, so the pairs
+// keep only the rates that it cannot hold, where they are the faster ones.
+// Chosen per launch: with the pairs as the fallback of single cells the step
+// took 270 us, the registers of both forms being needed at once.  The levels of
+// a refined run collide in pairs (a rescaled 104x88x72 step: 173 us against
+// 150), for the reason that collide_f64 gives for cells at rest.
+inline bool collides_in_pairs(bool paired, const DfRates& r) { return paired && !r.fx.ok; }
 
 }  // namespace lbx

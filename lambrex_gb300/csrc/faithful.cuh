@@ -74,7 +74,7 @@ __host__ __device__ __forceinline__ void f_cell_collide(double* __restrict__ f, 
   }
 #pragma unroll
   for (int q = 0; q < NV; ++q) v[q] = ld_pop_rw(f, q * b.sq + c, b);
-  collide_cell<double, PAIRED>(v, om_s, om_b, 0.0, r);
+  collide_cell<double, PAIRED, true>(v, om_s, om_b, 0.0, r);
 #pragma unroll
   for (int q = 0; q < NV; ++q) st_pop(f, q * b.sq + c, b, v[q]);
 }

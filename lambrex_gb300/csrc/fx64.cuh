@@ -44,10 +44,11 @@ struct FxDigits {
 };
 
 // (omega - 1) / 2 of the two rates in units of 2^-63; ok = 0: the rates are
-// outside the range of the fixed-point collision (or were not given)
+// outside the range of the fixed-point collision (or were not given); quiet:
+// cells at rest are left to the FP64 instructions (collide_f64)
 struct FxRates {
   FxDigits s, b;
-  int ok;
+  int ok, quiet;
 };
 
 inline FxDigits fx_digits_host(int64_t v) {
@@ -55,7 +56,7 @@ inline FxDigits fx_digits_host(int64_t v) {
   return FxDigits{(int)((v - lo) / (int64_t(1) << 32)), lo};
 }
 inline FxRates fx_rates(double om_s, double om_b) {
-  FxRates r{{0, 0}, {0, 0}, 0};
+  FxRates r{{0, 0}, {0, 0}, 0, 0};
   const double om[2] = {om_s, om_b};
   FxDigits d[2];
   for (int k = 0; k < 2; ++k) {
@@ -203,8 +204,19 @@ __host__ __device__ __forceinline__ FxSums fx_sums(const int64_t* g) {
   return m;
 }
 
+// |momenta| and |differences of the stresses| all below 2^15 units (2^-44 of
+// the density): a fluid at rest but for the last bits
+__host__ __device__ __forceinline__ bool fx_at_rest(const FxSums& m) {
+  const int64_t v[8] = {m.jx, m.jy, m.jz, m.s1 - m.s3, m.s3 - m.s5, m.Q1 - m.Q2, m.Q3 + m.Q4, m.Q3 - m.Q4};
+  uint64_t any = 0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) any |= (uint64_t)(v[k] + 0x8000) >> 16;
+  return any == 0;
+}
+
 // In-place collision; returns false, f untouched, where the cell is left to
 // collide<double>.
+template <bool QUIET = false>
 __host__ __device__ __forceinline__ bool collide_fx(double* f, const FxRates& r) {
   uint32_t h[NV], l[NV];
 #pragma unroll
@@ -233,6 +245,7 @@ __host__ __device__ __forceinline__ bool collide_fx(double* f, const FxRates& r)
     for (int a = 0; a < 3; ++a) ok = ok & ((uint32_t)(jh[a] + q4) < (uint32_t)(2 * q4));
     ok = ok & ((int)(D >> 32) < 2 * q4);
   }
+  if (QUIET) ok = ok & !(r.quiet != 0 && fx_at_rest(m));
   if (!ok) return false;
 
   // u_a in units of 2^-63: j_a 2^63 / rho
@@ -327,6 +340,51 @@ __host__ __device__ __forceinline__ bool hydro_fx(const double* f, double* rho, 
   return true;
 }
 
+// Mean of eight populations (a coarse cell's children): summed exactly and
+// rounded once where all are of ordinary size and not negative.  As FP64
+// additions the 15 means take 2,000 clocks of an SM per warp, more than their
+// loads.  Children within 2^9 units in the last place of each other (a fluid
+// at rest, see collide_f64) keep the additions, equal ones are their mean.
+__host__ __device__ __forceinline__ double mean8(const double* v) {
+  uint32_t h[8], l[8], top = 0, far = 0, differ = 0;
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    d_words(v[m], &h[m], &l[m]);
+    top = fx_umax(top, h[m]);
+    differ |= (h[m] ^ h[0]) | (l[m] ^ l[0]);
+    const uint64_t d = ((uint64_t)h[m] << 32 | l[m]) - ((uint64_t)h[0] << 32 | l[0]) + 512u;
+    far |= (uint32_t)(d >> 32) | ((uint32_t)d >> 10);
+  }
+  if (differ == 0) return v[0];
+  if (fx_top_ok(top) & (far != 0)) {
+    const uint32_t base = fx_base(top >> 20);
+    int64_t g = 0;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) g += fx_unit(h[m], l[m], base);
+    return fx_to_f64(g, (int)(top >> 20) - 29);  // an eighth of it
+  }
+  return 0.125 * (((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+}
+__host__ __device__ __forceinline__ float mean8(const float* v) {
+  return 0.125f * (((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+}
+
+// wp a + wn b: halves as one addition and the sum's exponent lowered (the
+// bits of the general form), one FP64 instruction instead of two
+template <typename T>
+__host__ __device__ __forceinline__ T weighted(T wp, T a, T wn, T b) {
+  if constexpr (sizeof(T) == 8) {
+    if (wp == T(0.5) && wn == T(0.5)) {
+      const double s = a + b;
+      uint32_t h, l;
+      d_words(s, &h, &l);
+      const uint32_t e = (h >> 20) & 2047u;
+      return e - 2u < 2044u ? d_from_words(h - 0x100000u, l) : 0.5 * s;
+    }
+  }
+  return wp * a + wn * b;
+}
+
 // |u| below 1/4 in units of 2^-62
 __host__ __device__ __forceinline__ int64_t fx_velocity(uint32_t h, uint32_t l) {
   const uint64_t m = ((uint64_t)((h << 11) | (l >> 21) | 0x80000000u) << 32) | (l << 11);
@@ -391,16 +449,60 @@ __host__ __device__ __forceinline__ void equilibrium_f64(double rho, double ux, 
   if (!equilibrium_fx(rho, ux, uy, uz, out)) equilibrium(rho, ux, uy, uz, out);
 }
 
+// collide<double> of a cell whose six axis populations are equal and whose
+// eight diagonal ones are: the operations that are left, in the same order, so
+// that the bits are its own (19 FP64 instructions instead of 128)
+__host__ __device__ __forceinline__ void collide_rest(double* f, double om_s, double om_b) {
+  const double s1 = f[1] + f[1], s7 = f[7] + f[7];
+  const double Q = s7 + s7, D = Q + Q, A = s1 + s1 + s1;
+  const double drho = f[0] + A + D;
+  const double A3 = A * (1.0 / 3.0);
+  const double d = s1 - A3;
+  const double TrS = fma(3.0, D, A) - drho;
+  const double TrS3 = fma(om_b, 0.0 - TrS, TrS) * (1.0 / 3.0);
+  const double m = fma(om_s, 0.0 - d, d) + TrS3;
+  const double Tp = m + m + m;
+  const double ba = fma(-1.0 / 6.0, Tp, (1.0 / 9.0) * drho);
+  const double ex = fma(0.5, m, ba);
+  const double bd = fma(1.0 / 24.0, Tp, (1.0 / 72.0) * drho);
+  f[0] = fma(-1.0 / 3.0, Tp, (2.0 / 9.0) * drho);
+#pragma unroll
+  for (int q = 1; q < NV; ++q) f[q] = q < 7 ? ex : bd;
+}
+__host__ __device__ __forceinline__ bool is_rest(const double* f) {
+  uint32_t h[NV], l[NV], d = 0;
+#pragma unroll
+  for (int q = 1; q < NV; ++q) d_words(f[q], &h[q], &l[q]);
+#pragma unroll
+  for (int q = 2; q < NV; ++q) {
+    const int t = q < 7 ? 1 : 7;
+    d |= (h[q] ^ h[t]) | (l[q] ^ l[t]);
+  }
+  return d == 0;
+}
+
 // The FP64 collision of one cell: in fixed point, or with FP64 instructions
 // where the cell or the rates are outside its range.  A host build forms the
 // digits of rates that were not given here; the kernels' launchers give them.
+//
+// QUIET, on the levels of a refined run: a cell at rest takes the FP64
+// instructions too.  The levels collide at different rates, whose roundings of
+// the one rest state differ in the last bit, so that a patch which no wave has
+// reached holds velocities of a few 1e-17 that are rounding alone; they stay
+// what they are with FP64 instructions.  An exactly uniform cell needs 19 of
+// those (323 clocks of an SM per warp, less than the fixed point's 450).
+template <bool QUIET = false>
 __host__ __device__ __forceinline__ void collide_f64(double* f, double om_s, double om_b,
                                                      const FxRates& r) {
 #ifdef __CUDA_ARCH__
-  if (!collide_fx(f, r)) collide<double>(f, om_s, om_b, 0.0);
+  if (collide_fx<QUIET>(f, r)) return;
 #else
-  if (!collide_fx(f, r.ok ? r : fx_rates(om_s, om_b))) collide<double>(f, om_s, om_b, 0.0);
+  if (collide_fx<QUIET>(f, r.ok ? r : fx_rates(om_s, om_b))) return;
 #endif
+  if (QUIET && is_rest(f))
+    collide_rest(f, om_s, om_b);
+  else
+    collide<double>(f, om_s, om_b, 0.0);
 }
 
 }  // namespace lbx

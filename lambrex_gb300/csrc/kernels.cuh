@@ -19,20 +19,23 @@ struct IBox {
 };
 inline IBox empty_ibox() { return IBox{{0, 0, 0}, {-1, -1, -1}}; }
 
-// Launch shape of a kernel over rows of x: blocks of `threads` threads laid
-// out as bx x by, bx = the row length rounded up to a warp (at most
-// `threads`) and by = threads / bx rows, so that short rows (AMR patches,
-// small boxes) do not leave most of a block idle.
+// Launch shape of a kernel over rows of x: blocks of at most `threads` threads
+// laid out as bx x by.  A row takes the fewest blocks that cover it, of equal
+// length rounded up to a warp (192 cells at 128 threads: 96 + 96, not
+// 128 + 64 of 128), and by = threads / bx rows, so that short rows (AMR
+// patches, small boxes) do not leave most of a block idle.
 struct RowLaunch {
   dim3 grid, block;
 };
 inline RowLaunch row_launch(int nx, int ny, int nz, int threads) {
-  int bx = (nx + 31) / 32 * 32;
-  if (bx > threads) bx = threads;
+  const int k = (nx + threads - 1) / threads;
+  const int bx = ((nx + k - 1) / k + 31) / 32 * 32;
   const int by = threads / bx;
   return RowLaunch{dim3((unsigned)((nx + bx - 1) / bx), (unsigned)((ny + by - 1) / by), (unsigned)nz),
                    dim3((unsigned)bx, (unsigned)by, 1)};
 }
+// whether every element index of a store fits in 31 bits (512^3 does)
+inline bool index32(const Box3& b) { return (long long)NV * b.sq < (1ll << 31); }
 #ifdef __CUDACC__
 // (x, y, z) of this thread under row_launch
 __device__ __forceinline__ void row_xyz(int& x, int& y, int& z) {
@@ -46,16 +49,12 @@ __device__ __forceinline__ void row_xyz(int& x, int& y, int& z) {
 // One fused collide + push-stream step (now <- S(C(now))).  Cells inside
 // `covered` are inactive: they emit zero populations (f = 0).
 // paired: FP64 store with the collision carried in pairs of FP32 values
-// (df32.cuh); ignored for the FP32 store.
+// (df32.cuh); ignored for the FP32 store.  refined: the level of a refined run
+// (collide_f64 and collides_in_pairs say what differs).
 template <typename T>
 cudaError_t launch_step_periodic(const T* fin, T* fout, const Box3& b, IBox covered, double om_s,
-                                 double om_b, double rho0, cudaStream_t st, int block = 128,
-                                 bool paired = false);
-
-// FP64 store, periodic push step with the paired collision in its one-cell
-// scalar form (the device-pointer entry lbx_step_periodic_f64p)
-cudaError_t launch_step_periodic_pairs_scalar(const double* fin, double* fout, const Box3& b,
-                                              double om_s, double om_b, cudaStream_t st);
+                                 double om_b, double rho0, cudaStream_t st, bool paired = false,
+                                 bool refined = false);
 
 // compensated sum of x[0..n) into out4[0] (out4[1..3] = 0); partials holds
 // kReduceBlocks x 8 doubles

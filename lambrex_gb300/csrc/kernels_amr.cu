@@ -42,31 +42,33 @@ inline RowLaunch grown_launch(const Box3& b, int threads) {
 }
 // ------------------------------------------------------------------ conservative
 
-template <typename T, bool PAIRED>
+template <typename T, bool PAIRED, typename I>
 __global__ void k_explode(const T* __restrict__ coarse, T* __restrict__ fine, Coupling c, T om_s,
                           T om_b, T rho0, DfRates r) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   int s[3];
   if (t >= ghost_cells_of(c.fb) || !ghost_coords(c.fb, (int)t, s)) return;
-  cell_explode<T, PAIRED>(coarse, fine, c, s[0], s[1], s[2], om_s, om_b, rho0, r);
+  cell_explode<T, PAIRED, I>(coarse, fine, c, s[0], s[1], s[2], om_s, om_b, rho0, r);
 }
 
-template <typename T, bool COVER, bool PAIRED>
-__global__ void k_step_patch(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov,
+// FP64: eight blocks an SM (64 registers): a rescaled two-level coarse step of
+// 104x88x72 took 158 us, against 162, 164 and 169 with six, five and four
+template <typename T, bool COVER, bool PAIRED, typename I>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 1) k_step_patch(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov,
                              T om_s, T om_b, T rho0, DfRates r) {
   GIdx s;
   if (!grown_index(b, s)) return;
-  cell_step_patch<T, COVER, PAIRED>(fin, fout, b, cov, s.x, s.y, s.z, om_s, om_b, rho0, r);
+  cell_step_patch<T, COVER, PAIRED, I>(fin, fout, b, cov, s.x, s.y, s.z, om_s, om_b, rho0, r);
 }
 
-template <typename T>
+template <typename T, typename I>
 __global__ void k_coalesce(const T* __restrict__ fine, T* __restrict__ coarse, Coupling c, T rho0) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;  // (ring cell, q)
-  const long long cell = t / NV;
-  const int q = (int)(t - cell * NV);
+  // (ring cell, population), neighbouring ring cells of one population per
+  // warp: their children and coarse entries lie side by side
+  const int cell = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
   int r[3];
-  if (cell >= ring_cells_of(c) || !ring_coords(c, (int)cell, r)) return;
-  cell_coalesce_q<T>(fine, coarse, c, r[0], r[1], r[2], q, rho0);
+  if (cell >= ring_cells_of(c) || !ring_coords(c, cell, r)) return;
+  cell_coalesce_q<T, I>(fine, coarse, c, r[0], r[1], r[2], q, rho0);
 }
 
 template <typename T>
@@ -78,24 +80,24 @@ __global__ void k_restrict(const T* __restrict__ fine, T* __restrict__ coarse, C
   cell_restrict<T>(fine, coarse, c, rx, ry, rz);
 }
 
-template <typename T, bool PAIRED>
+template <typename T, bool PAIRED, typename I>
 __global__ void k_explode_resc(const T* __restrict__ cprev, const T* __restrict__ cnow,
                                T* __restrict__ fine, Coupling c, T om_s, T om_b, T rho0, T wp, T wn,
                                DfRates r) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   int s[3];
   if (t >= ghost_cells_of(c.fb) || !ghost_coords(c.fb, (int)t, s)) return;
-  cell_explode_resc<T, PAIRED>(cprev, cnow, fine, c, s[0], s[1], s[2], om_s, om_b, rho0, wp, wn, r);
+  cell_explode_resc<T, PAIRED, I>(cprev, cnow, fine, c, s[0], s[1], s[2], om_s, om_b, rho0, wp, wn, r);
 }
 
-template <typename T, bool PAIRED>
+template <typename T, bool PAIRED, typename I>
 __global__ void k_restrict_resc(const T* __restrict__ fine, T* __restrict__ coarse, Coupling c,
                                 T om_s, T om_b, T rho0, DfRates r) {
   const int ex = c.fb.n[0] / 2, ey = c.fb.n[1] / 2, ez = c.fb.n[2] / 2;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)ex * ey * ez) return;
   const int rx = (int)(t % ex), ry = (int)((t / ex) % ey), rz = (int)(t / ((long long)ex * ey));
-  cell_restrict_resc<T, PAIRED>(fine, coarse, c, rx, ry, rz, om_s, om_b, rho0, r);
+  cell_restrict_resc<T, PAIRED, I>(fine, coarse, c, rx, ry, rz, om_s, om_b, rho0, r);
 }
 
 template <typename T>
@@ -172,18 +174,29 @@ inline long long grown_coarse_cells(const Box3& fb) {
 
 }  // namespace
 
+// f(index type) with int where every element index of the boxes fits in 31
+// bits: the kernels here are bound by instructions and latency, and 64-bit
+// element offsets took a third of the instructions of a patch step
+template <typename F>
+static void with_index(bool narrow, F f) {
+  if (narrow)
+    f(int{});
+  else
+    f((long long)0);
+}
+
 template <typename T>
 cudaError_t launch_explode(const T* coarse, T* fine, const Coupling& c, double om_s, double om_b,
                            double rho0, cudaStream_t st, bool paired) {
   const unsigned grid = blocks_for(ghost_cells_of(c.fb), 128);
-  if constexpr (sizeof(T) == 8) {
-    if (paired) {
-      k_explode<double, true><<<grid, 128, 0, st>>>(coarse, fine, c, om_s, om_b, 0.0,
-                                                    df_rates(om_s, om_b));
-      return cudaGetLastError();
-    }
-  }
-  k_explode<T, false><<<grid, 128, 0, st>>>(coarse, fine, c, (T)om_s, (T)om_b, (T)rho0, rates_of<T>(om_s, om_b));
+  const DfRates r = quiet(rates_of<T>(om_s, om_b));
+  with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
+    using I = decltype(i);
+    if (sizeof(T) == 8 && paired)
+      k_explode<T, sizeof(T) == 8, I><<<grid, 128, 0, st>>>(coarse, fine, c, (T)om_s, (T)om_b, (T)rho0, r);
+    else
+      k_explode<T, false, I><<<grid, 128, 0, st>>>(coarse, fine, c, (T)om_s, (T)om_b, (T)rho0, r);
+  });
   return cudaGetLastError();
 }
 
@@ -193,31 +206,30 @@ cudaError_t launch_step_patch(const T* fin, T* fout, const Box3& b, IBox covered
   const bool cov = covered.hi[0] >= covered.lo[0] && covered.hi[1] >= covered.lo[1] &&
                    covered.hi[2] >= covered.lo[2];
   const RowLaunch rl = grown_launch(b, 128);
-  if constexpr (sizeof(T) == 8) {
-    if (paired) {
-      const DfRates r = df_rates(om_s, om_b);
-      if (cov)
-        k_step_patch<double, true, true><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, om_s, om_b,
-                                                               0.0, r);
-      else
-        k_step_patch<double, false, true><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, om_s, om_b,
-                                                                0.0, r);
-      return cudaGetLastError();
-    }
-  }
-  if (cov)
-    k_step_patch<T, true, false><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, (T)om_s, (T)om_b,
-                                                       (T)rho0, rates_of<T>(om_s, om_b));
-  else
-    k_step_patch<T, false, false><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, (T)om_s, (T)om_b,
-                                                        (T)rho0, rates_of<T>(om_s, om_b));
+  const DfRates r = quiet(rates_of<T>(om_s, om_b));
+  with_index(index32(b), [&](auto i) {
+    using I = decltype(i);
+    constexpr bool P = sizeof(T) == 8;
+    const T ts = (T)om_s, tb = (T)om_b, t0 = (T)rho0;
+    if (P && paired && cov)
+      k_step_patch<T, true, P, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, ts, tb, t0, r);
+    else if (P && paired)
+      k_step_patch<T, false, P, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, ts, tb, t0, r);
+    else if (cov)
+      k_step_patch<T, true, false, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, ts, tb, t0, r);
+    else
+      k_step_patch<T, false, false, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, ts, tb, t0, r);
+  });
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_coalesce(const T* fine, T* coarse, const Coupling& c, double rho0,
                             cudaStream_t st) {
-  k_coalesce<T><<<blocks_for(ring_cells_of(c) * NV, 128), 128, 0, st>>>(fine, coarse, c, (T)rho0);
+  const dim3 grid(blocks_for(ring_cells_of(c), 128), NV);
+  with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
+    k_coalesce<T, decltype(i)><<<grid, 128, 0, st>>>(fine, coarse, c, (T)rho0);
+  });
   return cudaGetLastError();
 }
 
@@ -233,15 +245,16 @@ cudaError_t launch_explode_resc(const T* cprev, const T* cnow, T* fine, const Co
                                 double om_s, double om_b, double rho0, double wp, double wn,
                                 cudaStream_t st, bool paired) {
   const unsigned grid = blocks_for(ghost_cells_of(c.fb), 128);
-  if constexpr (sizeof(T) == 8) {
-    if (paired) {
-      k_explode_resc<double, true><<<grid, 128, 0, st>>>(cprev, cnow, fine, c, om_s, om_b, 0.0, wp,
-                                                         wn, df_rates(om_s, om_b));
-      return cudaGetLastError();
-    }
-  }
-  k_explode_resc<T, false><<<grid, 128, 0, st>>>(cprev, cnow, fine, c, (T)om_s, (T)om_b, (T)rho0,
-                                                 (T)wp, (T)wn, rates_of<T>(om_s, om_b));
+  const DfRates r = quiet(rates_of<T>(om_s, om_b));
+  with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
+    using I = decltype(i);
+    if (sizeof(T) == 8 && paired)
+      k_explode_resc<T, sizeof(T) == 8, I><<<grid, 128, 0, st>>>(
+          cprev, cnow, fine, c, (T)om_s, (T)om_b, (T)rho0, (T)wp, (T)wn, r);
+    else
+      k_explode_resc<T, false, I><<<grid, 128, 0, st>>>(cprev, cnow, fine, c, (T)om_s, (T)om_b,
+                                                        (T)rho0, (T)wp, (T)wn, r);
+  });
   return cudaGetLastError();
 }
 
@@ -249,15 +262,16 @@ template <typename T>
 cudaError_t launch_restrict_resc(const T* fine, T* coarse, const Coupling& c, double om_s,
                                  double om_b, double rho0, cudaStream_t st, bool paired) {
   const long long n = (long long)(c.fb.n[0] / 2) * (c.fb.n[1] / 2) * (c.fb.n[2] / 2);
-  if constexpr (sizeof(T) == 8) {
-    if (paired) {
-      k_restrict_resc<double, true><<<blocks_for(n, 128), 128, 0, st>>>(fine, coarse, c, om_s, om_b,
-                                                                       0.0, df_rates(om_s, om_b));
-      return cudaGetLastError();
-    }
-  }
-  k_restrict_resc<T, false><<<blocks_for(n, 128), 128, 0, st>>>(fine, coarse, c, (T)om_s, (T)om_b,
-                                                               (T)rho0, rates_of<T>(om_s, om_b));
+  const DfRates r = quiet(rates_of<T>(om_s, om_b));
+  with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
+    using I = decltype(i);
+    if (sizeof(T) == 8 && paired)
+      k_restrict_resc<T, sizeof(T) == 8, I><<<blocks_for(n, 128), 128, 0, st>>>(
+          fine, coarse, c, (T)om_s, (T)om_b, (T)rho0, r);
+    else
+      k_restrict_resc<T, false, I><<<blocks_for(n, 128), 128, 0, st>>>(fine, coarse, c, (T)om_s,
+                                                                       (T)om_b, (T)rho0, r);
+  });
   return cudaGetLastError();
 }
 
@@ -306,10 +320,11 @@ cudaError_t launch_f_collide(double* f, const Box3& b, IBox covered, double om_s
                              cudaStream_t st, bool paired) {
   const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
   if (paired)
-    k_f_collide<true><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b, df_rates(om_s, om_b));
+    k_f_collide<true><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b,
+                                                    quiet(df_rates(om_s, om_b)));
   else
     k_f_collide<false><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b,
-                                                     df_rates(om_s, om_b));
+                                                     quiet(df_rates(om_s, om_b)));
   return cudaGetLastError();
 }
 cudaError_t launch_f_stream(const double* src, double* dst, const Box3& b, cudaStream_t st) {

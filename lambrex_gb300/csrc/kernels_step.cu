@@ -9,24 +9,35 @@ namespace lbx {
 
 namespace {
 
+// Launch shape of the FP64 steps: they want instructions in flight as much as
+// bytes (1,090 a cell at 128 integer lanes), so blocks of 128 threads are held
+// to 64 registers, eight to an SM.  192^3: 277 us a step, against 297 in blocks
+// of 256 at 78 registers and 300 and 314 held to 56 and 48 (spills);
+// 251x190x133: 253 against 290, 264 and 301.
+constexpr int kF64Threads = 128, kF64Blocks = 8;
+constexpr int kPushThreads = 128;
+#define LBX_STEP_BOUNDS(T)                              \
+  __launch_bounds__(sizeof(T) == 8 ? kF64Threads : 256, \
+                    sizeof(T) == 8 ? kF64Blocks : 1)
+
 // Fused collide + push-stream over a periodic valid region
 // (src/AmrSim.cpp:25-135; include/component.h:22-29 written as a push:
 // f_new(x + c_q, q) = C(f)(x, q) is the same map as the reference's pull
 // f_new(x, q) = C(f)(x - c_q, q)).
-template <typename T, bool COVER, bool PAIRED>
-__global__ void __launch_bounds__(256) k_step_periodic(const T* __restrict__ fin,
-                                                       T* __restrict__ fout, Box3 b, IBox cov,
-                                                       T om_s, T om_b, T rho0, DfRates r) {
+template <typename T, bool COVER, bool PAIRED, typename I>
+__global__ void LBX_STEP_BOUNDS(T)
+    k_step_periodic(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov, T om_s,
+                    T om_b, T rho0, DfRates r) {
   int x, y, z;
   row_xyz(x, y, z);
   if (x >= b.n[0] || y >= b.n[1]) return;
-  cell_step_periodic<T, COVER, PAIRED>(fin, fout, b, cov, x, y, z, om_s, om_b, rho0, r);
+  cell_step_periodic<T, COVER, PAIRED, I>(fin, fout, b, cov, x, y, z, om_s, om_b, rho0, r);
 }
 
 // pull-form step P -> C(S(P)) (see cells.cuh); I = int when every element
 // index of the store fits in 31 bits (up to 15 x 2^27 elements: 512^3)
 template <typename T, bool PAIRED, typename I>
-__global__ void __launch_bounds__(256) k_step_pull(const T* __restrict__ fin, T* __restrict__ fout,
+__global__ void LBX_STEP_BOUNDS(T) k_step_pull(const T* __restrict__ fin, T* __restrict__ fout,
                                                    Box3 b, T om_s, T om_b, T rho0, DfRates r) {
   int x, y, z;
   row_xyz(x, y, z);
@@ -36,7 +47,7 @@ __global__ void __launch_bounds__(256) k_step_pull(const T* __restrict__ fin, T*
 
 // the pull-form step with CalcHydroVars fused in (cell_step_pull_hydro)
 template <typename T, bool PAIRED, typename I>
-__global__ void __launch_bounds__(256) k_step_pull_hydro(const T* __restrict__ fin,
+__global__ void LBX_STEP_BOUNDS(T) k_step_pull_hydro(const T* __restrict__ fin,
                                                          T* __restrict__ fout, Box3 b, T om_s,
                                                          T om_b, T rho0, DfRates r, double rho0_d,
                                                          double* __restrict__ rho,
@@ -45,24 +56,6 @@ __global__ void __launch_bounds__(256) k_step_pull_hydro(const T* __restrict__ f
   row_xyz(x, y, z);
   if (x >= b.n[0] || y >= b.n[1]) return;
   cell_step_pull_hydro<T, PAIRED, I>(fin, fout, b, x, y, z, om_s, om_b, rho0, r, rho0_d, rho, u);
-}
-
-// FP64 store, periodic push step with the paired collision in its one-cell
-// scalar form (collide_f64_via_df, no packed instructions): the form the
-// packed collision reproduces bit for bit, kept for the device-pointer entry
-// lbx_step_periodic_f64p so that the two can be compared.
-__global__ void __launch_bounds__(256) k_step_periodic_pairs_scalar(const double* __restrict__ fin,
-                                                                    double* __restrict__ fout,
-                                                                    Box3 b, DfRates r) {
-  int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
-  const long long c = b.at(x, y, z);
-  double f[NV];
-#pragma unroll
-  for (int q = 0; q < NV; ++q) f[q] = ld_pop(fin, q * b.sq + c, b);
-  collide_f64_via_df(f, r);
-  push_periodic<double>(fout, b, x, y, z, f);
 }
 
 // Q -> R = S(Q) (SIGN = +1, leaving the pull form) or R -> Q = S^-1(R)
@@ -491,32 +484,38 @@ cudaError_t launch_fill(double* p, size_t n, double v, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+template <typename T, bool COVER, bool PAIRED>
+static void step_periodic(const T* fin, T* fout, const Box3& b, const IBox& covered, double om_s,
+                          double om_b, double rho0, const DfRates& r, cudaStream_t st) {
+  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], kPushThreads);
+  if (index32(b))
+    k_step_periodic<T, COVER, PAIRED, int><<<rl.grid, rl.block, 0, st>>>(
+        fin, fout, b, covered, (T)om_s, (T)om_b, (T)rho0, r);
+  else
+    k_step_periodic<T, COVER, PAIRED, long long><<<rl.grid, rl.block, 0, st>>>(
+        fin, fout, b, covered, (T)om_s, (T)om_b, (T)rho0, r);
+}
+
 template <typename T>
 cudaError_t launch_step_periodic(const T* fin, T* fout, const Box3& b, IBox covered, double om_s,
-                                 double om_b, double rho0, cudaStream_t st, int block,
-                                 bool paired) {
+                                 double om_b, double rho0, cudaStream_t st, bool paired,
+                                 bool refined) {
   const bool cov = covered.hi[0] >= covered.lo[0] && covered.hi[1] >= covered.lo[1] &&
                    covered.hi[2] >= covered.lo[2];
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], block);
-  const dim3 grid = rl.grid;
+  const DfRates r = refined ? quiet(rates_of<T>(om_s, om_b)) : rates_of<T>(om_s, om_b);
   if constexpr (sizeof(T) == 8) {
-    if (paired) {
-      const DfRates r = df_rates(om_s, om_b);
+    if (refined ? paired : collides_in_pairs(paired, r)) {
       if (cov)
-        k_step_periodic<double, true, true><<<grid, rl.block, 0, st>>>(fin, fout, b, covered, om_s,
-                                                                    om_b, 0.0, r);
+        step_periodic<T, true, true>(fin, fout, b, covered, om_s, om_b, 0.0, r, st);
       else
-        k_step_periodic<double, false, true><<<grid, rl.block, 0, st>>>(fin, fout, b, covered, om_s,
-                                                                     om_b, 0.0, r);
+        step_periodic<T, false, true>(fin, fout, b, covered, om_s, om_b, 0.0, r, st);
       return cudaGetLastError();
     }
   }
   if (cov)
-    k_step_periodic<T, true, false><<<grid, rl.block, 0, st>>>(fin, fout, b, covered, (T)om_s,
-                                                            (T)om_b, (T)rho0, rates_of<T>(om_s, om_b));
+    step_periodic<T, true, false>(fin, fout, b, covered, om_s, om_b, rho0, r, st);
   else
-    k_step_periodic<T, false, false><<<grid, rl.block, 0, st>>>(fin, fout, b, covered, (T)om_s,
-                                                             (T)om_b, (T)rho0, rates_of<T>(om_s, om_b));
+    step_periodic<T, false, false>(fin, fout, b, covered, om_s, om_b, rho0, r, st);
   return cudaGetLastError();
 }
 
@@ -596,13 +595,10 @@ cudaError_t launch_copy_out(const T* f, const Box3& b, double rho0, double* out,
 template <typename T, typename I>
 cudaError_t launch_step_pull_i(const T* fin, T* fout, const Box3& b, double om_s, double om_b,
                                double rho0, bool paired, cudaStream_t st, int block) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], block);
+  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], sizeof(T) == 8 ? kF64Threads : block);
   if constexpr (sizeof(T) == 8) {
-    if (paired) {
-      // 52 registers: blocks of 128 threads fit nine per SM (36 warps)
-      // against four of 256 (32 warps); measured 1 % faster at 512^3
-      const RowLaunch rp = row_launch(b.n[0], b.n[1], b.n[2], block < 128 ? block : 128);
-      k_step_pull<double, true, I><<<rp.grid, rp.block, 0, st>>>(fin, fout, b, om_s, om_b, 0.0,
+    if (collides_in_pairs(paired, df_rates(om_s, om_b))) {
+      k_step_pull<double, true, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, om_s, om_b, 0.0,
                                                                  df_rates(om_s, om_b));
       return cudaGetLastError();
     }
@@ -627,15 +623,14 @@ template <typename T, typename I>
 cudaError_t launch_step_pull_hydro_i(const T* fin, T* fout, const Box3& b, double om_s,
                                      double om_b, double rho0, bool paired, double* rho,
                                      double* u, cudaStream_t st) {
+  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], sizeof(T) == 8 ? kF64Threads : 256);
   if constexpr (sizeof(T) == 8) {
-    if (paired) {
-      const RowLaunch rp = row_launch(b.n[0], b.n[1], b.n[2], 128);
-      k_step_pull_hydro<double, true, I><<<rp.grid, rp.block, 0, st>>>(
+    if (collides_in_pairs(paired, df_rates(om_s, om_b))) {
+      k_step_pull_hydro<double, true, I><<<rl.grid, rl.block, 0, st>>>(
           fin, fout, b, om_s, om_b, 0.0, df_rates(om_s, om_b), rho0, rho, u);
       return cudaGetLastError();
     }
   }
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 256);
   k_step_pull_hydro<T, false, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, (T)om_s, (T)om_b,
                                                                (T)rho0, rates_of<T>(om_s, om_b), rho0, rho, u);
   return cudaGetLastError();
@@ -648,13 +643,6 @@ cudaError_t launch_step_pull_hydro(const T* fin, T* fout, const Box3& b, double 
   if (sizeof(T) == 8 && (long long)NV * b.sq < (1ll << 31))
     return launch_step_pull_hydro_i<T, int>(fin, fout, b, om_s, om_b, rho0, paired, rho, u, st);
   return launch_step_pull_hydro_i<T, long long>(fin, fout, b, om_s, om_b, rho0, paired, rho, u, st);
-}
-
-cudaError_t launch_step_periodic_pairs_scalar(const double* fin, double* fout, const Box3& b,
-                                              double om_s, double om_b, cudaStream_t st) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
-  k_step_periodic_pairs_scalar<<<rl.grid, rl.block, 0, st>>>(fin, fout, b, df_rates(om_s, om_b));
-  return cudaGetLastError();
 }
 
 template <typename T>
@@ -714,7 +702,7 @@ cudaError_t launch_reduce(const T* f, const Box3& b, IBox skip, double rho0, dou
 
 #define LBX_INST(T)                                                                             \
   template cudaError_t launch_step_periodic<T>(const T*, T*, const Box3&, IBox, double, double, \
-                                               double, cudaStream_t, int, bool);                \
+                                               double, cudaStream_t, bool, bool);               \
   template cudaError_t launch_equilibrium<T>(const double*, const double*, T*, const Box3&,     \
                                              double, cudaStream_t);                             \
   template cudaError_t launch_hydro<T>(const T*, const Box3&, double, double*, double*,         \

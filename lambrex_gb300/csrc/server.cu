@@ -193,6 +193,7 @@ int admit(lbx_server* s, Req& q) {
     lv.box.om_s = lv.box.om_b = 1.0 / (tau + 0.5);
     lv.box.rho0 = rho0;
     lv.box.fx = lbx::fx_rates(lv.box.om_s, lv.box.om_b);
+    lv.box.fx.quiet = q.nlev > 1;
     tau *= 2.0;  // conservative scheme: viscosity-preserving tau_{l+1} = 2 tau_l
     lv.box.cov = lbx::empty_ibox();
     if (!lbx::set_iteration_space(lv.box)) return LBX_ERR_UNSUPPORTED;
@@ -236,9 +237,9 @@ int admit(lbx_server* s, Req& q) {
     const BBox& B = q.lev[L].box;
     cudaError_t e = s->precision == LBX_F64
                         ? lbx::launch_b_to_qform<double>(static_cast<double*>(B.buf[0]), B.b, B.cov, B.om_s,
-                                                         B.om_b, B.rho0, s->stream)
+                                                         B.om_b, B.rho0, q.nlev > 1, s->stream)
                         : lbx::launch_b_to_qform<float>(static_cast<float*>(B.buf[0]), B.b, B.cov, B.om_s,
-                                                        B.om_b, B.rho0, s->stream);
+                                                        B.om_b, B.rho0, q.nlev > 1, s->stream);
     CK(e);
   }
   q.state = 1;

@@ -461,8 +461,7 @@ int c_advance(lbx_sim* s, int L) {
   s->launches += (L < s->finest) ? 3 : 1;  // explode, step, coalesce
   if (L == 0)
     CK(lbx::launch_step_periodic<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box, cov,
-                                    omega(l.tau_s), omega(l.tau_b), s->rho0, s->stream, 128,
-                                    paired));
+                                    omega(l.tau_s), omega(l.tau_b), s->rho0, s->stream, paired, true));
   else
     CK(lbx::launch_step_patch<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box, cov,
                                  omega(l.tau_s), omega(l.tau_b), s->rho0, s->stream, paired));
@@ -516,7 +515,7 @@ int r_advance(lbx_sim* s, int L) {
   if (L == 0)
     CK(lbx::launch_step_periodic<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box,
                                     lbx::empty_ibox(), omega(l.tau_s), omega(l.tau_b), s->rho0,
-                                    s->stream, 128, paired));
+                                    s->stream, paired, true));
   else
     CK(lbx::launch_step_patch<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box,
                                  lbx::empty_ibox(), omega(l.tau_s), omega(l.tau_b), s->rho0,
@@ -1459,8 +1458,8 @@ int lbx_step_periodic_f64(const double* fin, double* fout, int nx, int ny, int n
 int lbx_step_periodic_f64p(const double* fin, double* fout, int nx, int ny, int nz, double tau_s,
                            double tau_b, void* stream) {
   if (!fin || !fout || fin == fout || nx <= 0 || ny <= 0 || nz <= 0) return LBX_ERR_ARG;
-  CK(lbx::launch_step_periodic_pairs_scalar(fin, fout, lbx::make_box(nx, ny, nz, 0), omega(tau_s),
-                                             omega(tau_b), (cudaStream_t)stream));
+  CK(lbx::launch_step_periodic<double>(fin, fout, lbx::make_box(nx, ny, nz, 0), lbx::empty_ibox(),
+                                       omega(tau_s), omega(tau_b), 0.0, (cudaStream_t)stream, true, false));
   return LBX_OK;
 }
 
