@@ -2,6 +2,9 @@
 // walks a tile work-list (box, first cell, cell count) with a grid sized to
 // the SM count; tiles of all boxes of a phase (independent simulations,
 // AMR levels of several requests) share the launch.
+// Launched the ordinary way: chained (launch.cuh) the served kernels took 14.6
+// ms instead of 13.8 for ten requests, as a grid that fills the GPU leaves the
+// next kernel's blocks no room to come up in.
 #include "batch.cuh"
 #include "cells.cuh"
 

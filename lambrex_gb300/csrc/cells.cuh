@@ -239,7 +239,7 @@ __host__ __device__ __forceinline__ void cell_fill_from_coarse(const T* __restri
   const long long cc = c.cb.at(px, py, pz), fc = sidx(c.fb, sx, sy, sz);
 #pragma unroll
   for (int q = 0; q < NV; ++q)
-    st_pop(fine, q * c.fb.sq + fc, c.fb, ld_pop(coarse, q * c.cb.sq + cc, c.cb));
+    st_pop(fine, q * c.fb.sq + fc, c.fb, ld_pop_ro(coarse, q * c.cb.sq + cc, c.cb));
 }
 
 // AMR patch, storage cell (sx,sy,sz) of the grown box: valid cells collide
@@ -615,7 +615,7 @@ __host__ __device__ __forceinline__ void cell_restrict(const T* __restrict__ fin
     T v[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m)
-      v[m] = ld_pop(fine,
+      v[m] = ld_pop_ro(fine,
                     (I)q * fsq + sidx_i<I>(c.fb, 2 * rx + (m & 1) + g, 2 * ry + ((m >> 1) & 1) + g,
                                            2 * rz + (m >> 2) + g),
                     c.fb);

@@ -3,7 +3,7 @@
 //
 // Every kernel reads and writes population stores and per-cell fields
 // through ld_pop / st_pop / ld_cell / st_cell.  In the release library they
-// are plain (read-only cached) loads and stores.  Built with LBX_CHECKED
+// are plain loads and stores.  Built with LBX_CHECKED
 // (liblbx_cuda_checked.so) each access first tests its element index against
 // the extent of the array it addresses -- NV * sq elements for a population
 // store of box b, the cell count for a per-cell field -- and on a miss counts
@@ -50,12 +50,32 @@ static const int g_oob_unit_registered = register_oob_reader(&read_unit_oob);
 __host__ __device__ __forceinline__ constexpr bool idx_ok(long long, long long) { return true; }
 #endif
 
-// read-only cached load on the device (a plain load in a host build, which
-// runs the per-cell code off the GPU in the tests)
+// read-only cached load on the device (a plain load in a host build)
 template <typename T>
 __host__ __device__ __forceinline__ T ld_ro(const T* p) {
 #ifdef __CUDA_ARCH__
   return __ldg(p);
+#else
+  return *p;
+#endif
+}
+// plain load of what an earlier kernel wrote: not through the read-only cache
+// and not moved ahead of chain_begin() (launch.cuh); on the host a plain load,
+// as the tests run the per-cell code off the GPU
+__host__ __device__ __forceinline__ double ld_plain(const double* p) {
+#ifdef __CUDA_ARCH__
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+#else
+  return *p;
+#endif
+}
+__host__ __device__ __forceinline__ float ld_plain(const float* p) {
+#ifdef __CUDA_ARCH__
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
 #else
   return *p;
 #endif
@@ -66,6 +86,12 @@ __host__ __device__ __forceinline__ T ld_ro(const T* p) {
 // 32-bit)
 template <typename T, typename I>
 __host__ __device__ __forceinline__ T ld_pop(const T* __restrict__ p, I i, const Box3& b) {
+  return idx_ok((long long)i, NV * b.sq) ? ld_plain(p + i) : T(0);
+}
+// the same through the read-only cache, for kernels that are not chained: a
+// compiler may move these ahead of the kernel's stores
+template <typename T, typename I>
+__host__ __device__ __forceinline__ T ld_pop_ro(const T* __restrict__ p, I i, const Box3& b) {
   return idx_ok((long long)i, NV * b.sq) ? ld_ro(p + i) : T(0);
 }
 // load of an entry the same kernel may also write (no read-only cache)

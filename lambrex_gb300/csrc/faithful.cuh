@@ -18,7 +18,7 @@ __host__ __device__ __forceinline__ void f_cell_fill_single(const double* __rest
   const long long d = sidx(b, sx, sy, sz);
   const long long c = b.at(wrapi(sx - g, b.n[0]), wrapi(sy - g, b.n[1]), wrapi(sz - g, b.n[2]));
 #pragma unroll
-  for (int q = 0; q < NV; ++q) st_pop(dst, q * b.sq + d, b, ld_pop(src, q * b.sq + c, b));
+  for (int q = 0; q < NV; ++q) st_pop(dst, q * b.sq + d, b, ld_pop_ro(src, q * b.sq + c, b));
 }
 
 // FillPatchTwoLevels + PCInterp (src/AmrSim.cpp:373-388), single time level:
@@ -37,7 +37,7 @@ __host__ __device__ __forceinline__ void f_cell_fill_two(const double* __restric
     const long long f = c.fb.at(wx, wy, wz);
 #pragma unroll
     for (int q = 0; q < NV; ++q)
-      st_pop(dst, q * c.fb.sq + d, c.fb, ld_pop(fnow, q * c.fb.sq + f, c.fb));
+      st_pop(dst, q * c.fb.sq + d, c.fb, ld_pop_ro(fnow, q * c.fb.sq + f, c.fb));
     return;
   }
   const int px = wrapi(floordiv2(X), c.cdom[0]) - c.clo[0];
@@ -47,7 +47,7 @@ __host__ __device__ __forceinline__ void f_cell_fill_two(const double* __restric
   const long long cc = c.cb.at(px, py, pz);
 #pragma unroll
   for (int q = 0; q < NV; ++q)
-    st_pop(dst, q * c.fb.sq + d, c.fb, ld_pop(cnow, q * c.cb.sq + cc, c.cb));
+    st_pop(dst, q * c.fb.sq + d, c.fb, ld_pop_ro(cnow, q * c.cb.sq + cc, c.cb));
 }
 
 // the outermost ghost layer, component 0 only (src/AmrSim.cpp:479-481)
@@ -90,7 +90,7 @@ __host__ __device__ __forceinline__ void f_cell_stream(const double* __restrict_
   const long long d = sidx(b, sx, sy, sz);
 #pragma unroll
   for (int q = 0; q < NV; ++q)
-    st_pop(dst, q * b.sq + d, b, ld_pop(src, q * b.sq + sidx(b, sx - CX(q), sy - CY(q), sz - CZ(q)), b));
+    st_pop(dst, q * b.sq + d, b, ld_pop_ro(src, q * b.sq + sidx(b, sx - CX(q), sy - CY(q), sz - CZ(q)), b));
 }
 
 // FillBoundary(periodicity) of level 0 (src/AmrSim.cpp:19-23, 132): ghost
@@ -144,7 +144,7 @@ __host__ __device__ __forceinline__ void f_cell_sum_from_fine(const double* __re
     for (int kr = 0; kr < 2; ++kr)
       for (int jr = 0; jr < 2; ++jr)
         for (int ir = 0; ir < 2; ++ir)
-          s += ld_pop(fnow, q * c.fb.sq + c.fb.at(fx0 + ir, fy0 + jr, fz0 + kr), c.fb);
+          s += ld_pop_ro(fnow, q * c.fb.sq + c.fb.at(fx0 + ir, fy0 + jr, fz0 + kr), c.fb);
     const double avg = 0.125 * s;
     for (int sz = -1; sz <= 1; ++sz)
       for (int sy = -1; sy <= 1; ++sy)

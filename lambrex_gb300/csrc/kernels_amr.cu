@@ -13,6 +13,7 @@
 // interpolated in time, with the non-equilibrium part rescaled between the
 // levels, and restricts the covered cells after the two sub-steps.
 #include "cells.cuh"
+#include "launch.cuh"
 #include "faithful.cuh"
 
 namespace lbx {
@@ -45,6 +46,7 @@ inline RowLaunch grown_launch(const Box3& b, int threads) {
 template <typename T, bool PAIRED, typename I>
 __global__ void k_explode(const T* __restrict__ coarse, T* __restrict__ fine, Coupling c, T om_s,
                           T om_b, T rho0, DfRates r) {
+  chain_begin();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   int s[3];
   if (t >= ghost_cells_of(c.fb) || !ghost_coords(c.fb, (int)t, s)) return;
@@ -56,6 +58,7 @@ __global__ void k_explode(const T* __restrict__ coarse, T* __restrict__ fine, Co
 template <typename T, bool COVER, bool PAIRED, typename I>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 1) k_step_patch(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov,
                              T om_s, T om_b, T rho0, DfRates r) {
+  chain_begin();
   GIdx s;
   if (!grown_index(b, s)) return;
   cell_step_patch<T, COVER, PAIRED, I>(fin, fout, b, cov, s.x, s.y, s.z, om_s, om_b, rho0, r);
@@ -63,6 +66,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 1) k_step_patch(cons
 
 template <typename T, typename I>
 __global__ void k_coalesce(const T* __restrict__ fine, T* __restrict__ coarse, Coupling c, T rho0) {
+  chain_begin();
   // (ring cell, population), neighbouring ring cells of one population per
   // warp: their children and coarse entries lie side by side
   const int cell = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
@@ -84,6 +88,7 @@ template <typename T, bool PAIRED, typename I>
 __global__ void k_explode_resc(const T* __restrict__ cprev, const T* __restrict__ cnow,
                                T* __restrict__ fine, Coupling c, T om_s, T om_b, T rho0, T wp, T wn,
                                DfRates r) {
+  chain_begin();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   int s[3];
   if (t >= ghost_cells_of(c.fb) || !ghost_coords(c.fb, (int)t, s)) return;
@@ -93,6 +98,7 @@ __global__ void k_explode_resc(const T* __restrict__ cprev, const T* __restrict_
 template <typename T, bool PAIRED, typename I>
 __global__ void k_restrict_resc(const T* __restrict__ fine, T* __restrict__ coarse, Coupling c,
                                 T om_s, T om_b, T rho0, DfRates r) {
+  chain_begin();
   const int ex = c.fb.n[0] / 2, ey = c.fb.n[1] / 2, ez = c.fb.n[2] / 2;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)ex * ey * ez) return;
@@ -193,9 +199,9 @@ cudaError_t launch_explode(const T* coarse, T* fine, const Coupling& c, double o
   with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
     using I = decltype(i);
     if (sizeof(T) == 8 && paired)
-      k_explode<T, sizeof(T) == 8, I><<<grid, 128, 0, st>>>(coarse, fine, c, (T)om_s, (T)om_b, (T)rho0, r);
+      chained(k_explode<T, sizeof(T) == 8, I>, grid, 128, st, coarse, fine, c, (T)om_s, (T)om_b, (T)rho0, r);
     else
-      k_explode<T, false, I><<<grid, 128, 0, st>>>(coarse, fine, c, (T)om_s, (T)om_b, (T)rho0, r);
+      chained(k_explode<T, false, I>, grid, 128, st, coarse, fine, c, (T)om_s, (T)om_b, (T)rho0, r);
   });
   return cudaGetLastError();
 }
@@ -212,13 +218,13 @@ cudaError_t launch_step_patch(const T* fin, T* fout, const Box3& b, IBox covered
     constexpr bool P = sizeof(T) == 8;
     const T ts = (T)om_s, tb = (T)om_b, t0 = (T)rho0;
     if (P && paired && cov)
-      k_step_patch<T, true, P, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, ts, tb, t0, r);
+      chained(k_step_patch<T, true, P, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r);
     else if (P && paired)
-      k_step_patch<T, false, P, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, ts, tb, t0, r);
+      chained(k_step_patch<T, false, P, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r);
     else if (cov)
-      k_step_patch<T, true, false, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, ts, tb, t0, r);
+      chained(k_step_patch<T, true, false, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r);
     else
-      k_step_patch<T, false, false, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, covered, ts, tb, t0, r);
+      chained(k_step_patch<T, false, false, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r);
   });
   return cudaGetLastError();
 }
@@ -228,7 +234,7 @@ cudaError_t launch_coalesce(const T* fine, T* coarse, const Coupling& c, double 
                             cudaStream_t st) {
   const dim3 grid(blocks_for(ring_cells_of(c), 128), NV);
   with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
-    k_coalesce<T, decltype(i)><<<grid, 128, 0, st>>>(fine, coarse, c, (T)rho0);
+    chained(k_coalesce<T, decltype(i)>, grid, 128, st, fine, coarse, c, (T)rho0);
   });
   return cudaGetLastError();
 }
@@ -249,10 +255,9 @@ cudaError_t launch_explode_resc(const T* cprev, const T* cnow, T* fine, const Co
   with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
     using I = decltype(i);
     if (sizeof(T) == 8 && paired)
-      k_explode_resc<T, sizeof(T) == 8, I><<<grid, 128, 0, st>>>(
-          cprev, cnow, fine, c, (T)om_s, (T)om_b, (T)rho0, (T)wp, (T)wn, r);
+      chained(k_explode_resc<T, sizeof(T) == 8, I>, grid, 128, st, cprev, cnow, fine, c, (T)om_s, (T)om_b, (T)rho0, (T)wp, (T)wn, r);
     else
-      k_explode_resc<T, false, I><<<grid, 128, 0, st>>>(cprev, cnow, fine, c, (T)om_s, (T)om_b,
+      chained(k_explode_resc<T, false, I>, grid, 128, st, cprev, cnow, fine, c, (T)om_s, (T)om_b,
                                                         (T)rho0, (T)wp, (T)wn, r);
   });
   return cudaGetLastError();
@@ -266,10 +271,9 @@ cudaError_t launch_restrict_resc(const T* fine, T* coarse, const Coupling& c, do
   with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
     using I = decltype(i);
     if (sizeof(T) == 8 && paired)
-      k_restrict_resc<T, sizeof(T) == 8, I><<<blocks_for(n, 128), 128, 0, st>>>(
-          fine, coarse, c, (T)om_s, (T)om_b, (T)rho0, r);
+      chained(k_restrict_resc<T, sizeof(T) == 8, I>, blocks_for(n, 128), 128, st, fine, coarse, c, (T)om_s, (T)om_b, (T)rho0, r);
     else
-      k_restrict_resc<T, false, I><<<blocks_for(n, 128), 128, 0, st>>>(fine, coarse, c, (T)om_s,
+      chained(k_restrict_resc<T, false, I>, blocks_for(n, 128), 128, st, fine, coarse, c, (T)om_s,
                                                                        (T)om_b, (T)rho0, r);
   });
   return cudaGetLastError();

@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "cells.cuh"
+#include "launch.cuh"
 #include "sums.cuh"
 
 namespace lbx {
@@ -28,6 +29,7 @@ template <typename T, bool COVER, bool PAIRED, typename I>
 __global__ void LBX_STEP_BOUNDS(T)
     k_step_periodic(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov, T om_s,
                     T om_b, T rho0, DfRates r) {
+  chain_begin();
   int x, y, z;
   row_xyz(x, y, z);
   if (x >= b.n[0] || y >= b.n[1]) return;
@@ -39,6 +41,7 @@ __global__ void LBX_STEP_BOUNDS(T)
 template <typename T, bool PAIRED, typename I>
 __global__ void LBX_STEP_BOUNDS(T) k_step_pull(const T* __restrict__ fin, T* __restrict__ fout,
                                                    Box3 b, T om_s, T om_b, T rho0, DfRates r) {
+  chain_begin();
   int x, y, z;
   row_xyz(x, y, z);
   if (x >= b.n[0] || y >= b.n[1]) return;
@@ -52,6 +55,7 @@ __global__ void LBX_STEP_BOUNDS(T) k_step_pull_hydro(const T* __restrict__ fin,
                                                          T om_b, T rho0, DfRates r, double rho0_d,
                                                          double* __restrict__ rho,
                                                          double* __restrict__ u) {
+  chain_begin();
   int x, y, z;
   row_xyz(x, y, z);
   if (x >= b.n[0] || y >= b.n[1]) return;
@@ -122,6 +126,7 @@ __global__ void k_init_pulse(T* __restrict__ f, Box3 b, int axis, int index, dou
 template <typename T, bool GATHER>
 __global__ void k_hydro(const T* __restrict__ f, Box3 b, double rho0, double* __restrict__ rho,
                         double* __restrict__ u) {
+  chain_begin();
   int x, y, z;
   row_xyz(x, y, z);
   if (x >= b.n[0] || y >= b.n[1]) return;
@@ -141,7 +146,7 @@ __global__ void k_copy_out(const T* __restrict__ f, Box3 b, double rho0, double*
     gather_periodic<T>(f, b, x, y, z, p);
   } else {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) p[q] = ld_pop(f, q * b.sq + c, b);
+    for (int q = 0; q < NV; ++q) p[q] = ld_pop_ro(f, q * b.sq + c, b);
   }
 #pragma unroll
   for (int q = 0; q < NV; ++q) st_cell(out, q * n + v, NV * n, (double)p[q] + W(q) * rho0);
@@ -170,7 +175,7 @@ __global__ void k_pack(const T* __restrict__ f, Box3 b, T* __restrict__ out) {
   const long long v = ((long long)z * b.n[1] + y) * b.n[0] + x;
   const long long c = b.at(x, y, z);
 #pragma unroll
-  for (int q = 0; q < NV; ++q) st_cell(out, q * n + v, NV * n, ld_pop(f, q * b.sq + c, b));
+  for (int q = 0; q < NV; ++q) st_cell(out, q * n + v, NV * n, ld_pop_ro(f, q * b.sq + c, b));
 }
 template <typename T>
 __global__ void k_unpack(const T* __restrict__ in, T* __restrict__ f, Box3 b) {
@@ -331,6 +336,7 @@ template <typename T, bool FLAT>
 __global__ void __launch_bounds__(kReduceThreads) k_reduce(const T* __restrict__ f, Box3 b,
                                                            IBox skip, double rho0,
                                                            double* __restrict__ partials) {
+  chain_begin();
   if (!idx_ok(blockIdx.x, kReduceBlocks)) return;  // partials hold kReduceBlocks blocks
   __shared__ Sum4Shared sh;
   // cell counts of every caller are below 2^31 (checked on the host), so the
@@ -489,11 +495,9 @@ static void step_periodic(const T* fin, T* fout, const Box3& b, const IBox& cove
                           double om_b, double rho0, const DfRates& r, cudaStream_t st) {
   const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], kPushThreads);
   if (index32(b))
-    k_step_periodic<T, COVER, PAIRED, int><<<rl.grid, rl.block, 0, st>>>(
-        fin, fout, b, covered, (T)om_s, (T)om_b, (T)rho0, r);
+    chained(k_step_periodic<T, COVER, PAIRED, int>, rl.grid, rl.block, st, fin, fout, b, covered, (T)om_s, (T)om_b, (T)rho0, r);
   else
-    k_step_periodic<T, COVER, PAIRED, long long><<<rl.grid, rl.block, 0, st>>>(
-        fin, fout, b, covered, (T)om_s, (T)om_b, (T)rho0, r);
+    chained(k_step_periodic<T, COVER, PAIRED, long long>, rl.grid, rl.block, st, fin, fout, b, covered, (T)om_s, (T)om_b, (T)rho0, r);
 }
 
 template <typename T>
@@ -575,9 +579,9 @@ cudaError_t launch_hydro(const T* f, const Box3& b, double rho0, double* rho, do
                          cudaStream_t st, bool gather) {
   const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
   if (gather)
-    k_hydro<T, true><<<rl.grid, rl.block, 0, st>>>(f, b, rho0, rho, u);
+    chained(k_hydro<T, true>, rl.grid, rl.block, st, f, b, rho0, rho, u);
   else
-    k_hydro<T, false><<<rl.grid, rl.block, 0, st>>>(f, b, rho0, rho, u);
+    chained(k_hydro<T, false>, rl.grid, rl.block, st, f, b, rho0, rho, u);
   return cudaGetLastError();
 }
 
@@ -598,12 +602,12 @@ cudaError_t launch_step_pull_i(const T* fin, T* fout, const Box3& b, double om_s
   const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], sizeof(T) == 8 ? kF64Threads : block);
   if constexpr (sizeof(T) == 8) {
     if (collides_in_pairs(paired, df_rates(om_s, om_b))) {
-      k_step_pull<double, true, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, om_s, om_b, 0.0,
+      chained(k_step_pull<double, true, I>, rl.grid, rl.block, st, fin, fout, b, om_s, om_b, 0.0,
                                                                  df_rates(om_s, om_b));
       return cudaGetLastError();
     }
   }
-  k_step_pull<T, false, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, (T)om_s, (T)om_b, (T)rho0,
+  chained(k_step_pull<T, false, I>, rl.grid, rl.block, st, fin, fout, b, (T)om_s, (T)om_b, (T)rho0,
                                                           rates_of<T>(om_s, om_b));
   return cudaGetLastError();
 }
@@ -626,12 +630,11 @@ cudaError_t launch_step_pull_hydro_i(const T* fin, T* fout, const Box3& b, doubl
   const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], sizeof(T) == 8 ? kF64Threads : 256);
   if constexpr (sizeof(T) == 8) {
     if (collides_in_pairs(paired, df_rates(om_s, om_b))) {
-      k_step_pull_hydro<double, true, I><<<rl.grid, rl.block, 0, st>>>(
-          fin, fout, b, om_s, om_b, 0.0, df_rates(om_s, om_b), rho0, rho, u);
+      chained(k_step_pull_hydro<double, true, I>, rl.grid, rl.block, st, fin, fout, b, om_s, om_b, 0.0, df_rates(om_s, om_b), rho0, rho, u);
       return cudaGetLastError();
     }
   }
-  k_step_pull_hydro<T, false, I><<<rl.grid, rl.block, 0, st>>>(fin, fout, b, (T)om_s, (T)om_b,
+  chained(k_step_pull_hydro<T, false, I>, rl.grid, rl.block, st, fin, fout, b, (T)om_s, (T)om_b,
                                                                (T)rho0, rates_of<T>(om_s, om_b), rho0, rho, u);
   return cudaGetLastError();
 }
@@ -693,9 +696,9 @@ cudaError_t launch_reduce(const T* f, const Box3& b, IBox skip, double rho0, dou
   const int grid = reduce_grid((long long)b.n[0] * b.n[1] * b.n[2]);
   const bool none = skip.hi[0] < skip.lo[0] || skip.hi[1] < skip.lo[1] || skip.hi[2] < skip.lo[2];
   if (b.g == 0 && none)
-    k_reduce<T, true><<<grid, kReduceThreads, 0, st>>>(f, b, skip, rho0, partials);
+    chained(k_reduce<T, true>, grid, kReduceThreads, st, f, b, skip, rho0, partials);
   else
-    k_reduce<T, false><<<grid, kReduceThreads, 0, st>>>(f, b, skip, rho0, partials);
+    chained(k_reduce<T, false>, grid, kReduceThreads, st, f, b, skip, rho0, partials);
   k_reduce_final<<<1, kReduceThreads, 0, st>>>(partials, grid, out4);
   return cudaGetLastError();
 }

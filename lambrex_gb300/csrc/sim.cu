@@ -119,6 +119,7 @@ struct StepGraph {
   double rho0 = 0.0;
   std::vector<double> dtime;    // per-level bookkeeping of one replay
   std::vector<int> dstep;
+  unsigned long long used = 0;  // when it was last replayed or captured
 };
 }  // namespace
 
@@ -145,10 +146,12 @@ struct lbx_sim {
   double* d_out4 = nullptr;
   double* h_out4 = nullptr;
   long long launches = 0;  // kernels issued by lbx_iterate (counted per launch)
-  // replayable macro steps (lbx_iterate): the two most recent captures, since
-  // a step taken ahead by CalcHydroVars swaps the store roles between calls
-  StepGraph graphs[2];
+  // replayable macro steps (lbx_iterate): a short and a long graph for each of
+  // the two store roles, since a step taken ahead by CalcHydroVars swaps them
+  // between calls
+  StepGraph graphs[4];
   int gcur = 0;            // the slot that matched or was captured last
+  unsigned long long gclock = 0;
   // CalcHydroVars on a single pull-form level runs the next step with the
   // fields as its epilogue once the program has shown that it steps on after
   // reading fields (an Iterate after a CalcHydroVars); until then it runs the
@@ -615,16 +618,28 @@ std::vector<LevelSig> signature(const lbx_sim* s) {
   return v;
 }
 
-bool graph_matches(lbx_sim* s) {
+// the longest graph of the present state that makes at most `left` steps
+bool graph_matches(lbx_sim* s, int left) {
   const std::vector<LevelSig> sig = signature(s);
-  for (int i = 0; i < 2; ++i) {
+  int best = 0;
+  for (int i = 0; i < 4; ++i) {
     const StepGraph& G = s->graphs[i];
-    if (G.exec && G.finest == s->finest && G.rho0 == s->rho0 && sig == G.sig) {
+    if (G.exec && G.finest == s->finest && G.rho0 == s->rho0 && sig == G.sig && G.period <= left &&
+        G.period > best) {
       s->gcur = i;
-      return true;
+      best = G.period;
     }
   }
-  return false;
+  return best > 0;
+}
+// Launches of a long graph: between the kernels of one graph there is no gap
+// (chained, launch.cuh), between two replays there is, so a run of
+// kGraphLongRun launches or more is replayed in long graphs; what is left, and
+// shorter runs, in graphs of one period.
+constexpr int kGraphLong = 32, kGraphLongRun = 2 * kGraphLong;
+int graph_steps(const lbx_sim* s, int left) {
+  const int per_step = std::max(1, s->finest == 0 ? 1 : 4 << (s->finest - 1));  // launches, about
+  return (long long)left * per_step >= kGraphLongRun ? std::max(2, kGraphLong / per_step) : 1;
 }
 
 // Capture macro steps from the simulation's own launches until every level's
@@ -632,8 +647,12 @@ bool graph_matches(lbx_sim* s) {
 // host-side bookkeeping already advanced while capturing).  Keeps the graph
 // for replay when the roles did return.
 int capture_graph(lbx_sim* s, int* left) {
-  s->gcur ^= 1;  // replaces the older of the two captures
+  const int atleast = std::min(graph_steps(s, *left), *left);
+  s->gcur = 0;  // replaces the one not used for longest
+  for (int i = 1; i < 4; ++i)
+    if (s->graphs[i].used < s->graphs[s->gcur].used) s->gcur = i;
   StepGraph& G = s->graphs[s->gcur];
+  G.used = ++s->gclock;
   if (G.exec) {
     CK(cudaStreamSynchronize(s->stream));
     cudaGraphExecDestroy(G.exec);
@@ -652,7 +671,8 @@ int capture_graph(lbx_sim* s, int* left) {
   do {
     rc = macro_step(s);
     ++m;
-  } while (rc == LBX_OK && m < std::min(kGraphMaxPeriod, *left) && !(signature(s) == sig0));
+  } while (rc == LBX_OK && m < std::min(kGraphMaxPeriod + atleast - 1, *left) &&
+           (m < atleast || !(signature(s) == sig0)));
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(s->stream, &g);
   if (rc != LBX_OK || e != cudaSuccess) {
@@ -688,6 +708,7 @@ int capture_graph(lbx_sim* s, int* left) {
 
 int replay_graph(lbx_sim* s) {
   StepGraph& G = s->graphs[s->gcur];
+  G.used = ++s->gclock;
   CK(cudaGraphLaunch(G.exec, s->stream));
   for (size_t L = 0; L < s->lev.size() && L < G.dtime.size(); ++L) {
     s->lev[L].time += G.dtime[L];
@@ -1142,11 +1163,14 @@ int lbx_iterate(lbx_sim* s, int nsteps) {
     --left;
   }
   if (left >= kGraphMinSteps) {
-    if (!graph_matches(s)) RET(capture_graph(s, &left));
-    const StepGraph& G = s->graphs[s->gcur];
-    while (G.exec && left >= G.period) {
-      RET(replay_graph(s));
-      left -= G.period;
+    while (left >= kGraphMinSteps) {
+      if (!graph_matches(s, left) || s->graphs[s->gcur].period < graph_steps(s, left)) {
+        RET(capture_graph(s, &left));  // runs what it captures
+        if (!s->graphs[s->gcur].exec) break;
+        continue;
+      }
+      for (const int period = s->graphs[s->gcur].period; left >= period; left -= period)
+        RET(replay_graph(s));
     }
   }
   for (; left > 0; --left) RET(macro_step(s));
