@@ -39,8 +39,11 @@ struct BTile {
 // coarse/fine pair of boxes inside the batch (AMR coupling of one request)
 struct BCoupling {
   Coupling c;
-  int cbox, fbox;  // box-table indices of the coarse and the fine level
-  int nring;       // coarse ring cells (grown coarsened patch minus interior)
+  void* cbuf[2];   // the stores of the coarse and the fine level, their index
+  void* fbuf[2];   // when the level's flip is 0, and the shift: a block needs
+  int cpar, fpar;  // this one descriptor and not the boxes' too
+  int clev;        // the coarse level
+  double rho0;
 };
 
 // Division by an iteration-space extent d: q = (x * m) >> 40 with
@@ -94,6 +97,17 @@ inline long long box_cells(const BBox& b) {
   return b.periodic ? (long long)b.dxy * b.b.n[2] : b.b.sq;
 }
 
+// Cells per tile of a launch over `cells` cells: as large as leaves two tiles to
+// each of `blocks` resident blocks, between lo and hi (each lo times a power of
+// two).  Ten served requests, levels 0, 1 and 2 of 1.8, 1.3 and 0.8 M cells:
+// tiles of 1024 left the finest level at 0.6 waves, 22 us a launch for the 10 us
+// that its instructions take.
+inline int fitting_tile(long long cells, long long blocks, int lo, int hi) {
+  int tile = lo;
+  while (tile * 2 <= hi && cells >= 2 * blocks * tile * 2) tile *= 2;
+  return tile;
+}
+
 // split the iteration space of each listed box into tiles of tile_cells
 inline std::vector<BTile> make_tiles(const std::vector<BBox>& boxes, const std::vector<int>& ids,
                                      int tile_cells) {
@@ -118,14 +132,16 @@ cudaError_t launch_b_to_qform(T* f, const Box3& b, const IBox& cov, double om_s,
                               double rho0, bool refined, cudaStream_t st);
 template <typename T>
 cudaError_t launch_b_to_rform(const T* qprev, T* r, const Box3& b, cudaStream_t st);
-// explode / coalesce over coupling tiles; flip_c / flip_f select
-// the coarse and fine "now" stores at the time of the call (explosion and
-// coalescence in the pull form)
+// explode / coalesce over coupling tiles; flips[L] selects the "now" store of
+// level L at the time of the call (explosion and coalescence in the pull form)
+struct BFlips {
+  int f[3];
+};
 template <typename T>
-cudaError_t launch_b_explode(const BBox* boxes, const BCoupling* cps, const BTile* tiles,
-                             int ntiles, int flip_c, int flip_f, cudaStream_t st);
+cudaError_t launch_b_explode(const BCoupling* cps, const BTile* tiles, int ntiles, BFlips flips,
+                             cudaStream_t st);
 template <typename T>
-cudaError_t launch_b_coalesce(const BBox* boxes, const BCoupling* cps, const BTile* tiles,
-                              int ntiles, int flip_c, int flip_f, cudaStream_t st);
+cudaError_t launch_b_coalesce(const BCoupling* cps, const BTile* tiles, int ntiles, BFlips flips,
+                              cudaStream_t st);
 
 }  // namespace lbx

@@ -12,10 +12,21 @@ namespace lbx {
 
 namespace {
 
+// a descriptor into shared memory, word by word over the block's threads: one
+// latency, where a single thread's copy waits for several
+template <typename D>
+__device__ __forceinline__ void stage(D& to, const D& from) {
+  static_assert(sizeof(D) % 4 == 0, "copied in words");
+  const int* s = reinterpret_cast<const int*>(&from);
+  int* d = reinterpret_cast<int*>(&to);
+  for (int i = threadIdx.x; i < (int)(sizeof(D) / 4); i += blockDim.x) d[i] = s[i];
+}
+
 // One kernel per box kind (every launch covers boxes of one kind), so each
 // instantiation carries only its own cell body.  The tile's box descriptor
 // is staged in shared memory: the cell code reads its geometry from there
-// instead of holding it in registers, which keeps occupancy high.
+// instead of holding it in registers, which keeps occupancy high.  (FP64 held
+// to 64 registers spills and is no faster: 109.2 us a step against 107.9.)
 template <typename T, int KIND, int CPT>
 __global__ void __launch_bounds__(512) k_b_step(const BBox* __restrict__ boxes,
                                                 const BTile* __restrict__ tiles, int ntiles,
@@ -24,7 +35,7 @@ __global__ void __launch_bounds__(512) k_b_step(const BBox* __restrict__ boxes,
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const BTile tl = tiles[t];
     __syncthreads();  // the previous tile is done with sbox
-    if (threadIdx.x == 0) sbox = boxes[tl.box];
+    stage(sbox, boxes[tl.box]);
     __syncthreads();
     const BBox& B = sbox;
     const int par = B.par ^ flip;
@@ -79,38 +90,38 @@ void launch_kind(const BBox* boxes, const BTile* tiles, int ntiles, int flip, in
 }
 
 template <typename T>
-__global__ void k_b_explode(const BBox* __restrict__ boxes, const BCoupling* __restrict__ cps,
-                            const BTile* __restrict__ tiles, int ntiles, int flip_c, int flip_f) {
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const BTile tl = tiles[t];
-    const BCoupling& cp = cps[tl.box];
-    const BBox& C = boxes[cp.cbox];
-    const BBox& F = boxes[cp.fbox];
-    const T* coarse = static_cast<const T*>(C.buf[C.par ^ flip_c]);
-    T* fine = static_cast<T*>(F.buf[F.par ^ flip_f]);
-    for (int i = threadIdx.x; i < tl.count; i += blockDim.x) {
-      int s[3];
-      if (ghost_coords(cp.c.fb, tl.start + i, s))  // the ghost shell only
-        cell_explode<T, false, int, true>(coarse, fine, cp.c, s[0], s[1], s[2], (T)C.om_s,
-                                          (T)C.om_b, (T)C.rho0);
-    }
+__global__ void __launch_bounds__(128) k_b_explode(const BCoupling* __restrict__ cps,
+                                                   const BTile* __restrict__ tiles, BFlips flips) {
+  __shared__ BCoupling cp;
+  const BTile tl = tiles[blockIdx.x];
+  stage(cp, cps[tl.box]);
+  __syncthreads();
+  const T* coarse = static_cast<const T*>(cp.cbuf[cp.cpar ^ flips.f[cp.clev]]);
+  T* fine = static_cast<T*>(cp.fbuf[cp.fpar ^ flips.f[cp.clev + 1]]);
+  const T rho0 = (T)cp.rho0;
+  for (int i = threadIdx.x; i < tl.count; i += blockDim.x) {
+    int s[3];
+    if (ghost_coords(cp.c.fb, tl.start + i, s))  // the ghost shell only
+      cell_explode<T, false, int, true>(coarse, fine, cp.c, s[0], s[1], s[2], T(0), T(0), rho0);
   }
 }
 
+constexpr int kCoalesceThreads = 256;
 template <typename T>
-__global__ void k_b_coalesce(const BBox* __restrict__ boxes, const BCoupling* __restrict__ cps,
-                             const BTile* __restrict__ tiles, int ntiles, int flip_c, int flip_f) {
+__global__ void __launch_bounds__(kCoalesceThreads)
+    k_b_coalesce(const BCoupling* __restrict__ cps, const BTile* __restrict__ tiles, BFlips flips) {
   // ring-cell coordinates are decoded once per cell into shared memory, then
   // the block's threads take the (ring cell, population) items
   constexpr int kChunk = 256;
   __shared__ int sr[kChunk][3];
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const BTile tl = tiles[t];
-    const BCoupling& cp = cps[tl.box];
-    const BBox& C = boxes[cp.cbox];
-    const BBox& F = boxes[cp.fbox];
-    T* coarse = static_cast<T*>(C.buf[C.par ^ flip_c]);
-    const T* fine = static_cast<const T*>(F.buf[F.par ^ flip_f]);
+  __shared__ BCoupling cp;
+  {
+    const BTile tl = tiles[blockIdx.x];
+    stage(cp, cps[tl.box]);
+    __syncthreads();
+    T* coarse = static_cast<T*>(cp.cbuf[cp.cpar ^ flips.f[cp.clev]]);
+    const T* fine = static_cast<const T*>(cp.fbuf[cp.fpar ^ flips.f[cp.clev + 1]]);
+    const T rho0 = (T)cp.rho0;
     for (int c0 = 0; c0 < tl.count; c0 += kChunk) {
       const int nc = min(kChunk, tl.count - c0);
       __syncthreads();  // the previous chunk is done with sr
@@ -128,7 +139,7 @@ __global__ void k_b_coalesce(const BBox* __restrict__ boxes, const BCoupling* __
         const int q = i / nc, cell = i - q * nc;
         if (sr[cell][0] >= 0)
           cell_coalesce_q<T, int, true>(fine, coarse, cp.c, sr[cell][0], sr[cell][1], sr[cell][2],
-                                        q, (T)C.rho0);
+                                        q, rho0);
       }
     }
   }
@@ -200,28 +211,28 @@ cudaError_t launch_b_step(const BBox* boxes, const BTile* tiles, int ntiles, int
 }
 
 template <typename T>
-cudaError_t launch_b_explode(const BBox* boxes, const BCoupling* cps, const BTile* tiles,
-                             int ntiles, int flip_c, int flip_f, cudaStream_t st) {
+cudaError_t launch_b_explode(const BCoupling* cps, const BTile* tiles, int ntiles, BFlips flips,
+                             cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
-  k_b_explode<T><<<ntiles, 128, 0, st>>>(boxes, cps, tiles, ntiles, flip_c, flip_f);
+  k_b_explode<T><<<ntiles, 128, 0, st>>>(cps, tiles, flips);
   return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t launch_b_coalesce(const BBox* boxes, const BCoupling* cps, const BTile* tiles,
-                              int ntiles, int flip_c, int flip_f, cudaStream_t st) {
+cudaError_t launch_b_coalesce(const BCoupling* cps, const BTile* tiles, int ntiles, BFlips flips,
+                              cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
-  k_b_coalesce<T><<<ntiles, 128, 0, st>>>(boxes, cps, tiles, ntiles, flip_c, flip_f);
+  k_b_coalesce<T><<<ntiles, kCoalesceThreads, 0, st>>>(cps, tiles, flips);
   return cudaGetLastError();
 }
 
 #define LBX_INST(T)                                                                             \
   template cudaError_t launch_b_step<T>(const BBox*, const BTile*, int, int, int, int, int, int,\
                                         cudaStream_t);                                          \
-  template cudaError_t launch_b_explode<T>(const BBox*, const BCoupling*, const BTile*, int,    \
-                                           int, int, cudaStream_t);                             \
-  template cudaError_t launch_b_coalesce<T>(const BBox*, const BCoupling*, const BTile*, int,   \
-                                            int, int, cudaStream_t);                            \
+  template cudaError_t launch_b_explode<T>(const BCoupling*, const BTile*, int, BFlips,         \
+                                           cudaStream_t);                                       \
+  template cudaError_t launch_b_coalesce<T>(const BCoupling*, const BTile*, int, BFlips,        \
+                                            cudaStream_t);                                      \
   template cudaError_t launch_b_to_qform<T>(T*, const Box3&, const IBox&, double, double, double,\
                                             bool, cudaStream_t);                                      \
   template cudaError_t launch_b_to_rform<T>(const T*, T*, const Box3&, cudaStream_t);

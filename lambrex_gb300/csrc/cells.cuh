@@ -407,13 +407,18 @@ __host__ __device__ __forceinline__ void cell_explode(const T* __restrict__ coar
                          P[2] - c.clo[2] + c.cb.g);
   const I csq = (I)c.cb.sq, fsq = (I)c.fb.sq;
   T f[NV];
+  // post-collision populations are taken as they are, so those that do not
+  // enter (two thirds of a face's) are not loaded
 #pragma unroll
-  for (int q = 0; q < NV; ++q) f[q] = ld_pop(coarse, (I)q * csq + cc, c.cb);
+  for (int q = 0; q < NV; ++q) {
+    const bool in = in_valid(c.fb, vx + 2 * CX(q), vy + 2 * CY(q), vz + 2 * CZ(q));
+    f[q] = !QFORM || in ? ld_pop(coarse, (I)q * csq + cc, c.cb) : zero_pop<T>(q, rho0);
+  }
   if (!QFORM) collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);
   const I fc = sidx_i<I>(c.fb, sx, sy, sz);
 #pragma unroll
   for (int q = 0; q < NV; ++q) {
-    const bool in = in_valid(c.fb, vx + 2 * CX(q), vy + 2 * CY(q), vz + 2 * CZ(q));
+    const bool in = QFORM || in_valid(c.fb, vx + 2 * CX(q), vy + 2 * CY(q), vz + 2 * CZ(q));
     st_pop(fine, (I)q * fsq + fc, c.fb, in ? f[q] : zero_pop<T>(q, rho0));
   }
 }
@@ -566,6 +571,12 @@ __host__ __device__ __forceinline__ void cell_coalesce_q(const T* __restrict__ f
                                                 T rho0) {
   const int cgx = c.flo[0] / 2 + rx - 1, cgy = c.flo[1] / 2 + ry - 1, cgz = c.flo[2] / 2 + rz - 1;
   const int cx = CX(q), cy = CY(q), cz = CZ(q);
+  // a cell beyond a face receives from the patch only what moves out of it
+  // through that face (a third of the populations; the others end here)
+  const int mx = c.fb.n[0] / 2 + 1, my = c.fb.n[1] / 2 + 1, mz = c.fb.n[2] / 2 + 1;
+  if ((rx == 0 && cx >= 0) || (rx == mx && cx <= 0) || (ry == 0 && cy >= 0) ||
+      (ry == my && cy <= 0) || (rz == 0 && cz >= 0) || (rz == mz && cz <= 0))
+    return;
   int P[3] = {cgx, cgy, cgz};
   if (QFORM) {
     P[0] -= cx;

@@ -67,7 +67,7 @@ struct lbx_ensemble {
   BBox* d_boxes = nullptr;
   std::vector<BTile> ht;
   BTile* d_tiles = nullptr;
-  int tile_cells = 8192, block = 256, cpt = 1, grid = 0;
+  int tile_cells = 1024, block = 256, cpt = 1, grid = 0;  // see default_shape
   int flip = 0;  // all boxes step together: store "now" is par ^ flip
   int num_sms = 0;
   cudaStream_t stream = nullptr;
@@ -77,6 +77,23 @@ struct lbx_ensemble {
 };
 
 namespace {
+
+// Launch shape until the caller sets or tunes it: blocks of 256 threads (FP64
+// 128, for its registers) and as many tiles as keep the blocks of the persistent
+// grid even at their end, and no more.  us a step with tiles of 256, 1024 and
+// 8192 cells: 24 boxes of 9.9 M cells FP32 200, 184, 214 (in blocks of 128: 185,
+// 199, 240); 8 boxes of 0.33 M cells 8.2, 9.2, 24.6; 16 boxes of 2.0 M cells
+// FP64 in blocks of 128 108, 104, 152 (of 256: 122, 114, 121).
+void default_shape(lbx_ensemble* e) {
+  const bool f64 = e->precision == LBX_F64;
+  e->block = f64 ? 128 : 256;
+  e->cpt = 1;
+  long long cells = 0;
+  for (const BBox& b : e->hb) cells += lbx::box_cells(b);
+  const int per_sm = f64 ? lbx::b_step_blocks_per_sm<double>(e->block, e->cpt, lbx::kBoxPull)
+                         : lbx::b_step_blocks_per_sm<float>(e->block, e->cpt, lbx::kBoxPull);
+  e->tile_cells = lbx::fitting_tile(cells, (long long)e->num_sms * per_sm, 256, 1024);
+}
 
 int upload_tiles(lbx_ensemble* e) {
   std::vector<int> ids(e->nbox);
@@ -193,6 +210,7 @@ int lbx_ensemble_create(int nbox, const int* dims, const double* tau, int precis
     lbx_ensemble_destroy(e);
     return lbx::status_from_cuda(err);
   }
+  default_shape(e);
   int rc = upload_tiles(e);
   if (rc != LBX_OK) {
     lbx_ensemble_destroy(e);
@@ -262,7 +280,7 @@ int lbx_ensemble_autotune(lbx_ensemble* e, int trial_steps, int* chosen3) {
     CK(cudaMallocAsync(&saved[b], bytes, e->stream));
     CK(cudaMemcpyAsync(saved[b], e->hb[b].buf[box_now(e, b)], bytes, cudaMemcpyDeviceToDevice, e->stream));
   }
-  const int tiles[] = {2048, 8192, 32768};
+  const int tiles[] = {512, 1024, 2048};
   const int blocks[] = {128, 256, 512};
   const int cpts[] = {1, 2};
   float best = 1e30f;

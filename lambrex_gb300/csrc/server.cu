@@ -49,11 +49,15 @@ using lbx::Range;
 namespace {
 
 constexpr int kMaxLevels = 3;
-// cells per tile of the coupling kernels (128-thread blocks).  Explosion:
-// one ghost cell per thread.  Coalescence: each ring cell is fifteen
-// (cell, population) items of eight loads; 32 ring cells per block spread a
-// launch over enough blocks to fill the GPU (256 per block left a launch of
-// a few requests at 0.1 waves and 6 % of the warp slots, latency-bound).
+// cells per tile of the coupling kernels.  Explosion: one ghost cell per thread
+// of 128.  Coalescence: each ring cell is fifteen (cell, population) items of
+// eight loads for 256 threads; 32 ring cells per block spread a launch over
+// enough blocks to fill the GPU (256 per block left a launch of a few requests
+// at 0.1 waves and 6 % of the warp slots, latency-bound; 64: 10.97 ms instead of
+// 10.78 for the steps of ten requests).  What bounds both is a chain of
+// latencies, tile, descriptor, values: one descriptor staged by the whole block
+// and the populations that cannot cross left out took the explosions from 3 x
+// 11 to 2 x 14 us a coarse step and the coalescences from 3 x 17.4 to 3 x 7.8.
 constexpr int kExplodeTile = 128;
 constexpr int kCoalesceTile = 32;
 
@@ -108,7 +112,9 @@ struct lbx_server {
   long long graph_launches = 0;
   cudaStream_t stream = nullptr;
   cudaMemPool_t pool = nullptr;  // request stores (release threshold = budget)
-  int num_sms = 0, block = 128, cpt = 1, tile_cells = 1024;  // measured best on GB300
+  int num_sms = 0, block = 128, cpt = 1;  // measured best on GB300
+  int tile_cells = 1024;  // at most (fitting_tile), or as the caller set it
+  bool tuned = false;
   int grid[3] = {0, 0, 0};  // persistent grid per box kind (SMs x resident blocks)
   long long cell_updates = 0, launches = 0;
   long long updates_per_macro = 0;
@@ -270,19 +276,34 @@ int rebuild_tables(lbx_server* s) {
     }
     for (int L = 1; L < q.nlev; ++L) {
       BCoupling c;
+      std::memset(&c, 0, sizeof c);
       c.c = coupling_of(q, L);
-      c.cbox = bidx[L - 1];
-      c.fbox = bidx[L];
-      c.nring = 0;
+      c.clev = L - 1;
+      const BBox &cb = q.lev[L - 1].box, &fb = q.lev[L].box;
+      for (int k = 0; k < 2; ++k) {
+        c.cbuf[k] = cb.buf[k];
+        c.fbuf[k] = fb.buf[k];
+      }
+      c.cpar = cb.par;
+      c.fpar = fb.par;
+      c.rho0 = fb.rho0;
       cids[L - 1].push_back((int)s->hc.size());
       s->hc.push_back(c);
     }
   }
   std::vector<BTile> all;
   for (int L = 0; L < kMaxLevels; ++L) {
-    s->tiles_step[L] = lbx::make_tiles(s->hb, ids[L], s->tile_cells);
+    long long cells = 0;
+    for (int id : ids[L]) cells += lbx::box_cells(s->hb[id]);
+    const int tile = s->tuned ? s->tile_cells
+                              : lbx::fitting_tile(cells, s->grid[L ? lbx::kBoxPatch : lbx::kBoxPeriodic],
+                                                  s->block, s->tile_cells);
+    s->tiles_step[L] = lbx::make_tiles(s->hb, ids[L], tile);
     append(all, s->off_step[L], s->tiles_step[L]);
   }
+  // the explosions' tiles of the two level pairs side by side (advance_level
+  // launches them together), then the coalescences'
+  std::vector<BTile> all_co;
   for (int k = 0; k < 2; ++k) {
     std::vector<BTile> ex, co;
     for (int ci : cids[k]) {
@@ -299,8 +320,10 @@ int rebuild_tables(lbx_server* s) {
     s->tiles_ex[k] = ex;
     s->tiles_co[k] = co;
     append(all, s->off_ex[k], ex);
-    append(all, s->off_co[k], co);
+    append(all_co, s->off_co[k], co);
   }
+  for (int k = 0; k < 2; ++k) s->off_co[k] += all.size();
+  all.insert(all.end(), all_co.begin(), all_co.end());
   auto align = [](size_t n) { return (n + 255) & ~size_t(255); };
   const size_t nb = s->hb.size() * sizeof(BBox), nc = s->hc.size() * sizeof(BCoupling),
                nt = all.size() * sizeof(BTile);
@@ -351,26 +374,34 @@ cudaError_t phase_step(lbx_server* s, int L) {
 // L+1, coalesce into the streamed coarse state) becomes: explode from the
 // coarse post-collision store, two steps of L+1, coalesce into the entries
 // the coarse cells will gather, step L.
+//
+// Level 0's explosion and the first of level 1 are one launch: the one writes
+// level 1's ghost shell, the other reads the ring around level 2's centred
+// box, which keeps a quarter of level 1's extent from that shell.
 template <typename T>
-cudaError_t advance_level(lbx_server* s, int L) {
+cudaError_t advance_level(lbx_server* s, int L, bool exploded = false) {
   cudaError_t e = cudaSuccess;
   const bool has_fine = L + 1 < kMaxLevels && !s->tiles_step[L + 1].empty();
+  const lbx::BFlips flips{{s->F[0], s->F[1], s->F[2]}};
   if (has_fine) {
-    if (!s->tiles_ex[L].empty()) {
+    const bool both = L == 0 && !s->tiles_ex[1].empty();
+    if (!exploded && !s->tiles_ex[L].empty()) {
       ++s->launches;
-      e = lbx::launch_b_explode<T>(s->d_boxes, s->d_cps, s->d_tiles + s->off_ex[L],
-                                   (int)s->tiles_ex[L].size(), s->F[L], s->F[L + 1], s->stream);
+      e = lbx::launch_b_explode<T>(s->d_cps, s->d_tiles + s->off_ex[L],
+                                   (int)(s->tiles_ex[L].size() + (both ? s->tiles_ex[1].size() : 0)),
+                                   flips, s->stream);
       if (e != cudaSuccess) return e;
     }
     for (int k = 0; k < 2; ++k) {
-      e = advance_level<T>(s, L + 1);
+      e = advance_level<T>(s, L + 1, both && k == 0);
       if (e != cudaSuccess) return e;
     }
     if (!s->tiles_co[L].empty()) {
       // covered coarse cells are restricted only when a request finishes
       ++s->launches;
-      e = lbx::launch_b_coalesce<T>(s->d_boxes, s->d_cps, s->d_tiles + s->off_co[L],
-                                    (int)s->tiles_co[L].size(), s->F[L], s->F[L + 1], s->stream);
+      const lbx::BFlips now{{s->F[0], s->F[1], s->F[2]}};
+      e = lbx::launch_b_coalesce<T>(s->d_cps, s->d_tiles + s->off_co[L],
+                                    (int)s->tiles_co[L].size(), now, s->stream);
       if (e != cudaSuccess) return e;
     }
   }
@@ -529,6 +560,7 @@ int lbx_server_set_config(lbx_server* s, int tile_cells, int block, int cells_pe
       cells_per_thread > 2 || tile_cells < block)
     return LBX_ERR_ARG;
   s->tile_cells = tile_cells;
+  s->tuned = true;
   s->block = block;
   s->cpt = cells_per_thread;
   for (int kind = 0; kind < 3; ++kind) {
