@@ -221,9 +221,30 @@ __host__ __device__ __forceinline__ void equilibrium_shifted(double rho, double 
   out[14] = w2 * (dr + r * (-ax - ay - az + uv + vw + uw + m2));
 }
 
+// Division of numbers below 2^31 by a fixed d >= 1 (round-up method, Granlund
+// and Montgomery 1994): with 2^(l-1) < d <= 2^l and m = floor(2^32 (2^l - d) / d)
+// + 1, x / d = (floor(x m / 2^32) + x) >> l; the sum stays below 2^32.
+struct Divisor {
+  uint32_t m;
+  int l;
+};
+inline Divisor make_divisor(uint32_t d) {
+  int l = 0;
+  while ((uint64_t(1) << l) < d) ++l;
+  return Divisor{(uint32_t)(((uint64_t(1) << 32) * ((uint64_t(1) << l) - d)) / d + 1), l};
+}
+__host__ __device__ __forceinline__ uint32_t divide(uint32_t x, const Divisor& d) {
+#ifdef __CUDA_ARCH__
+  return (__umulhi(x, d.m) + x) >> d.l;
+#else
+  return (uint32_t)((((uint64_t)x * d.m) >> 32) + x) >> d.l;
+#endif
+}
+
 // Storage description of one box: valid extents n, ghost width g, strides.
 struct Box3 {
   int n[3];        // valid extents
+  Divisor row, plane;  // of valid cells in order, by n[0] and by n[0] n[1]
   int g;           // ghost layers in storage
   long long sx;    // row length  = n[0] + 2g
   long long sxy;   // plane size  = (n[1] + 2g) * sx
@@ -238,6 +259,8 @@ inline Box3 make_box(int nx, int ny, int nz, int g) {
   b.n[0] = nx;
   b.n[1] = ny;
   b.n[2] = nz;
+  b.row = make_divisor((uint32_t)nx);
+  b.plane = make_divisor((uint32_t)((long long)nx * ny));
   b.g = g;
   b.sx = nx + 2 * g;
   b.sxy = (long long)(ny + 2 * g) * b.sx;

@@ -19,29 +19,32 @@ struct IBox {
 };
 inline IBox empty_ibox() { return IBox{{0, 0, 0}, {-1, -1, -1}}; }
 
-// Launch shape of a kernel over rows of x: blocks of at most `threads` threads
-// laid out as bx x by.  A row takes the fewest blocks that cover it, of equal
-// length rounded up to a warp (192 cells at 128 threads: 96 + 96, not
-// 128 + 64 of 128), and by = threads / bx rows, so that short rows (AMR
-// patches, small boxes) do not leave most of a block idle.
-struct RowLaunch {
+// Launch shape of a kernel over the valid cells of a box in storage order: one
+// thread a cell, whatever the extents (rows padded to warps left 22 % of the
+// lanes idle at 100 or 104 cells, 16 % at 161).  Neighbouring threads have
+// neighbouring addresses across the ends of rows too, as the cells do.  A box
+// that would not give every other SM a block gets smaller blocks (10x10x50 in
+// blocks of 32: FP64 2.38 us a step against 2.46, FP32 1.60 against 1.79; with
+// the line at 152 or 304 blocks 32^3 FP32 took 2.06 us instead of 1.85).
+struct CellLaunch {
   dim3 grid, block;
 };
-inline RowLaunch row_launch(int nx, int ny, int nz, int threads) {
-  const int k = (nx + threads - 1) / threads;
-  const int bx = ((nx + k - 1) / k + 31) / 32 * 32;
-  const int by = threads / bx;
-  return RowLaunch{dim3((unsigned)((nx + bx - 1) / bx), (unsigned)((ny + by - 1) / by), (unsigned)nz),
-                   dim3((unsigned)bx, (unsigned)by, 1)};
+inline CellLaunch cell_launch(const Box3& b, int threads) {
+  const long long n = (long long)b.n[0] * b.n[1] * b.n[2];
+  while (threads > 32 && n < 76ll * threads) threads /= 2;
+  return CellLaunch{dim3((unsigned)((n + threads - 1) / threads)), dim3((unsigned)threads)};
 }
 // whether every element index of a store fits in 31 bits (512^3 does)
 inline bool index32(const Box3& b) { return (long long)NV * b.sq < (1ll << 31); }
 #ifdef __CUDACC__
-// (x, y, z) of this thread under row_launch
-__device__ __forceinline__ void row_xyz(int& x, int& y, int& z) {
-  x = blockIdx.x * blockDim.x + threadIdx.x;
-  y = blockIdx.y * blockDim.y + threadIdx.y;
-  z = blockIdx.z;
+// (x, y, z) of this thread's cell under cell_launch; false beyond the last one
+__device__ __forceinline__ bool cell_xyz(const Box3& b, int& x, int& y, int& z) {
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  z = (int)divide(c, b.plane);
+  const uint32_t p = c - (uint32_t)z * (uint32_t)(b.n[0] * b.n[1]);
+  y = (int)divide(p, b.row);
+  x = (int)(p - (uint32_t)y * (uint32_t)b.n[0]);
+  return z < b.n[2];
 }
 #endif
 

@@ -36,9 +36,9 @@ __device__ __forceinline__ bool grown_index(const Box3& b, GIdx& s) {
   s.z = blockIdx.y;
   return true;
 }
-inline RowLaunch grown_launch(const Box3& b, int threads) {
+inline CellLaunch grown_launch(const Box3& b, int threads) {
   const int plane = (b.n[0] + 2 * b.g) * (b.n[1] + 2 * b.g);
-  return RowLaunch{dim3((unsigned)((plane + threads - 1) / threads), (unsigned)(b.n[2] + 2 * b.g), 1),
+  return CellLaunch{dim3((unsigned)((plane + threads - 1) / threads), (unsigned)(b.n[2] + 2 * b.g), 1),
                    dim3((unsigned)threads, 1, 1)};
 }
 // ------------------------------------------------------------------ conservative
@@ -139,8 +139,7 @@ template <bool PAIRED>
 __global__ void k_f_collide(double* __restrict__ f, Box3 b, IBox cov, double om_s, double om_b,
                             DfRates r) {
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   f_cell_collide<PAIRED>(f, b, cov, x, y, z, om_s, om_b, r);
 }
 
@@ -211,7 +210,7 @@ cudaError_t launch_step_patch(const T* fin, T* fout, const Box3& b, IBox covered
                               double om_b, double rho0, cudaStream_t st, bool paired) {
   const bool cov = covered.hi[0] >= covered.lo[0] && covered.hi[1] >= covered.lo[1] &&
                    covered.hi[2] >= covered.lo[2];
-  const RowLaunch rl = grown_launch(b, 128);
+  const CellLaunch rl = grown_launch(b, 128);
   const DfRates r = quiet(rates_of<T>(om_s, om_b));
   with_index(index32(b), [&](auto i) {
     using I = decltype(i);
@@ -281,7 +280,7 @@ cudaError_t launch_restrict_resc(const T* fine, T* coarse, const Coupling& c, do
 
 template <typename T>
 cudaError_t launch_fill_from_coarse(const T* coarse, T* fine, const Coupling& c, cudaStream_t st) {
-  const RowLaunch rl = grown_launch(c.fb, 128);
+  const CellLaunch rl = grown_launch(c.fb, 128);
   k_fill_from_coarse<T><<<rl.grid, rl.block, 0, st>>>(coarse, fine, c);
   return cudaGetLastError();
 }
@@ -304,25 +303,25 @@ LBX_INST(float)
 #undef LBX_INST
 
 cudaError_t launch_f_fill_single(const double* src, double* dst, const Box3& b, cudaStream_t st) {
-  const RowLaunch rl = grown_launch(b, 128);
+  const CellLaunch rl = grown_launch(b, 128);
   k_f_fill_single<<<rl.grid, rl.block, 0, st>>>(src, dst, b);
   return cudaGetLastError();
 }
 cudaError_t launch_f_fill_two(const double* fine_now, double* dst, const double* coarse_now,
                               const Coupling& c, const int* fdom, cudaStream_t st) {
-  const RowLaunch rl = grown_launch(c.fb, 128);
+  const CellLaunch rl = grown_launch(c.fb, 128);
   k_f_fill_two<<<rl.grid, rl.block, 0, st>>>(fine_now, dst, coarse_now, c, fdom[0],
                                                          fdom[1], fdom[2]);
   return cudaGetLastError();
 }
 cudaError_t launch_f_zero_ring0(double* f, const Box3& b, cudaStream_t st) {
-  const RowLaunch rl = grown_launch(b, 128);
+  const CellLaunch rl = grown_launch(b, 128);
   k_f_zero_ring0<<<rl.grid, rl.block, 0, st>>>(f, b);
   return cudaGetLastError();
 }
 cudaError_t launch_f_collide(double* f, const Box3& b, IBox covered, double om_s, double om_b,
                              cudaStream_t st, bool paired) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
+  const CellLaunch rl = cell_launch(b, 128);
   if (paired)
     k_f_collide<true><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b,
                                                     quiet(df_rates(om_s, om_b)));
@@ -332,17 +331,17 @@ cudaError_t launch_f_collide(double* f, const Box3& b, IBox covered, double om_s
   return cudaGetLastError();
 }
 cudaError_t launch_f_stream(const double* src, double* dst, const Box3& b, cudaStream_t st) {
-  const RowLaunch rl = grown_launch(b, 128);
+  const CellLaunch rl = grown_launch(b, 128);
   k_f_stream<<<rl.grid, rl.block, 0, st>>>(src, dst, b);
   return cudaGetLastError();
 }
 cudaError_t launch_f_fill_boundary(double* f, const Box3& b, cudaStream_t st) {
-  const RowLaunch rl = grown_launch(b, 128);
+  const CellLaunch rl = grown_launch(b, 128);
   k_f_fill_boundary<<<rl.grid, rl.block, 0, st>>>(f, b);
   return cudaGetLastError();
 }
 cudaError_t launch_f_zero_invalid(double* f, const Box3& b, cudaStream_t st) {
-  const RowLaunch rl = grown_launch(b, 128);
+  const CellLaunch rl = grown_launch(b, 128);
   k_f_zero_invalid<<<rl.grid, rl.block, 0, st>>>(f, b);
   return cudaGetLastError();
 }

@@ -12,9 +12,8 @@ namespace {
 
 // Launch shape of the FP64 steps: they want instructions in flight as much as
 // bytes (1,090 a cell at 128 integer lanes), so blocks of 128 threads are held
-// to 64 registers, eight to an SM.  192^3: 277 us a step, against 297 in blocks
-// of 256 at 78 registers and 300 and 314 held to 56 and 48 (spills);
-// 251x190x133: 253 against 290, 264 and 301.
+// to 64 registers, eight to an SM.  251x190x133: 253 us a step, against 290 in
+// blocks of 256 at 78 registers and 264 and 301 held to 56 and 48 (spills).
 constexpr int kF64Threads = 128, kF64Blocks = 8;
 constexpr int kPushThreads = 128;
 #define LBX_STEP_BOUNDS(T)                              \
@@ -31,8 +30,7 @@ __global__ void LBX_STEP_BOUNDS(T)
                     T om_b, T rho0, DfRates r) {
   chain_begin();
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   cell_step_periodic<T, COVER, PAIRED, I>(fin, fout, b, cov, x, y, z, om_s, om_b, rho0, r);
 }
 
@@ -43,8 +41,7 @@ __global__ void LBX_STEP_BOUNDS(T) k_step_pull(const T* __restrict__ fin, T* __r
                                                    Box3 b, T om_s, T om_b, T rho0, DfRates r) {
   chain_begin();
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   cell_step_pull<T, PAIRED, I>(fin, fout, b, x, y, z, om_s, om_b, rho0, r);
 }
 
@@ -57,8 +54,7 @@ __global__ void LBX_STEP_BOUNDS(T) k_step_pull_hydro(const T* __restrict__ fin,
                                                          double* __restrict__ u) {
   chain_begin();
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   cell_step_pull_hydro<T, PAIRED, I>(fin, fout, b, x, y, z, om_s, om_b, rho0, r, rho0_d, rho, u);
 }
 
@@ -67,8 +63,7 @@ __global__ void LBX_STEP_BOUNDS(T) k_step_pull_hydro(const T* __restrict__ fin,
 template <typename T, int SIGN>
 __global__ void k_shift(const T* __restrict__ fin, T* __restrict__ fout, Box3 b) {
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   T v[NV];
   gather_periodic<T, SIGN>(fin, b, x, y, z, v);
   const long long c = b.at(x, y, z);
@@ -80,8 +75,7 @@ template <typename T>
 __global__ void k_equilibrium(const double* __restrict__ rho, const double* __restrict__ u,
                               T* __restrict__ f, Box3 b, double rho0) {
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   const long long n = (long long)b.n[0] * b.n[1] * b.n[2];
   const long long v = ((long long)z * b.n[1] + y) * b.n[0] + x;
   const double r = ld_cell(rho, v, n), ux = ld_cell(u, v, 3 * n), uy = ld_cell(u, n + v, 3 * n),
@@ -105,8 +99,7 @@ template <typename T>
 __global__ void k_init_pulse(T* __restrict__ f, Box3 b, int axis, int index, double amplitude,
                              double rho0) {
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   const int c[3] = {x, y, z};
   const double rho = 1.0 + (c[axis] == index ? amplitude : 0.0);
   const long long s = b.at(x, y, z);
@@ -128,16 +121,14 @@ __global__ void k_hydro(const T* __restrict__ f, Box3 b, double rho0, double* __
                         double* __restrict__ u) {
   chain_begin();
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   cell_hydro<T, GATHER>(f, b, rho0, rho, u, x, y, z);
 }
 
 template <typename T, bool GATHER>
 __global__ void k_copy_out(const T* __restrict__ f, Box3 b, double rho0, double* __restrict__ out) {
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   const long long n = (long long)b.n[0] * b.n[1] * b.n[2];
   const long long v = ((long long)z * b.n[1] + y) * b.n[0] + x;
   const long long c = b.at(x, y, z);
@@ -155,8 +146,7 @@ __global__ void k_copy_out(const T* __restrict__ f, Box3 b, double rho0, double*
 template <typename T>
 __global__ void k_copy_in(const double* __restrict__ in, T* __restrict__ f, Box3 b, double rho0) {
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   const long long n = (long long)b.n[0] * b.n[1] * b.n[2];
   const long long v = ((long long)z * b.n[1] + y) * b.n[0] + x;
   const long long c = b.at(x, y, z);
@@ -169,8 +159,7 @@ __global__ void k_copy_in(const double* __restrict__ in, T* __restrict__ f, Box3
 template <typename T>
 __global__ void k_pack(const T* __restrict__ f, Box3 b, T* __restrict__ out) {
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   const long long n = (long long)b.n[0] * b.n[1] * b.n[2];
   const long long v = ((long long)z * b.n[1] + y) * b.n[0] + x;
   const long long c = b.at(x, y, z);
@@ -180,8 +169,7 @@ __global__ void k_pack(const T* __restrict__ f, Box3 b, T* __restrict__ out) {
 template <typename T>
 __global__ void k_unpack(const T* __restrict__ in, T* __restrict__ f, Box3 b) {
   int x, y, z;
-  row_xyz(x, y, z);
-  if (x >= b.n[0] || y >= b.n[1]) return;
+  if (!cell_xyz(b, x, y, z)) return;
   const long long n = (long long)b.n[0] * b.n[1] * b.n[2];
   const long long v = ((long long)z * b.n[1] + y) * b.n[0] + x;
   const long long c = b.at(x, y, z);
@@ -493,7 +481,7 @@ cudaError_t launch_fill(double* p, size_t n, double v, cudaStream_t st) {
 template <typename T, bool COVER, bool PAIRED>
 static void step_periodic(const T* fin, T* fout, const Box3& b, const IBox& covered, double om_s,
                           double om_b, double rho0, const DfRates& r, cudaStream_t st) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], kPushThreads);
+  const CellLaunch rl = cell_launch(b, kPushThreads);
   if (index32(b))
     chained(k_step_periodic<T, COVER, PAIRED, int>, rl.grid, rl.block, st, fin, fout, b, covered, (T)om_s, (T)om_b, (T)rho0, r);
   else
@@ -526,7 +514,7 @@ cudaError_t launch_step_periodic(const T* fin, T* fout, const Box3& b, IBox cove
 template <typename T>
 cudaError_t launch_equilibrium(const double* rho, const double* u, T* f, const Box3& b,
                                double rho0, cudaStream_t st) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
+  const CellLaunch rl = cell_launch(b, 128);
   k_equilibrium<T><<<rl.grid, rl.block, 0, st>>>(rho, u, f, b, rho0);
   return cudaGetLastError();
 }
@@ -577,7 +565,7 @@ cudaError_t launch_tag_density(const double* rho, const int* n, double ref, doub
 template <typename T>
 cudaError_t launch_hydro(const T* f, const Box3& b, double rho0, double* rho, double* u,
                          cudaStream_t st, bool gather) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
+  const CellLaunch rl = cell_launch(b, 128);
   if (gather)
     chained(k_hydro<T, true>, rl.grid, rl.block, st, f, b, rho0, rho, u);
   else
@@ -588,7 +576,7 @@ cudaError_t launch_hydro(const T* f, const Box3& b, double rho0, double* rho, do
 template <typename T>
 cudaError_t launch_copy_out(const T* f, const Box3& b, double rho0, double* out, cudaStream_t st,
                             bool gather) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
+  const CellLaunch rl = cell_launch(b, 128);
   if (gather)
     k_copy_out<T, true><<<rl.grid, rl.block, 0, st>>>(f, b, rho0, out);
   else
@@ -599,7 +587,7 @@ cudaError_t launch_copy_out(const T* f, const Box3& b, double rho0, double* out,
 template <typename T, typename I>
 cudaError_t launch_step_pull_i(const T* fin, T* fout, const Box3& b, double om_s, double om_b,
                                double rho0, bool paired, cudaStream_t st, int block) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], sizeof(T) == 8 ? kF64Threads : block);
+  const CellLaunch rl = cell_launch(b, sizeof(T) == 8 ? kF64Threads : block);
   if constexpr (sizeof(T) == 8) {
     if (collides_in_pairs(paired, df_rates(om_s, om_b))) {
       chained(k_step_pull<double, true, I>, rl.grid, rl.block, st, fin, fout, b, om_s, om_b, 0.0,
@@ -627,7 +615,7 @@ template <typename T, typename I>
 cudaError_t launch_step_pull_hydro_i(const T* fin, T* fout, const Box3& b, double om_s,
                                      double om_b, double rho0, bool paired, double* rho,
                                      double* u, cudaStream_t st) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], sizeof(T) == 8 ? kF64Threads : 256);
+  const CellLaunch rl = cell_launch(b, sizeof(T) == 8 ? kF64Threads : 256);
   if constexpr (sizeof(T) == 8) {
     if (collides_in_pairs(paired, df_rates(om_s, om_b))) {
       chained(k_step_pull_hydro<double, true, I>, rl.grid, rl.block, st, fin, fout, b, om_s, om_b, 0.0, df_rates(om_s, om_b), rho0, rho, u);
@@ -651,41 +639,41 @@ cudaError_t launch_step_pull_hydro(const T* fin, T* fout, const Box3& b, double 
 template <typename T>
 cudaError_t launch_init_pulse(T* f, const Box3& b, int axis, int index, double amplitude,
                               double rho0, cudaStream_t st) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
+  const CellLaunch rl = cell_launch(b, 128);
   k_init_pulse<T><<<rl.grid, rl.block, 0, st>>>(f, b, axis, index, amplitude, rho0);
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_unstream(const T* fin, T* fout, const Box3& b, cudaStream_t st) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
+  const CellLaunch rl = cell_launch(b, 128);
   k_shift<T, -1><<<rl.grid, rl.block, 0, st>>>(fin, fout, b);
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_stream_gather(const T* fin, T* fout, const Box3& b, cudaStream_t st) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
+  const CellLaunch rl = cell_launch(b, 128);
   k_shift<T, 1><<<rl.grid, rl.block, 0, st>>>(fin, fout, b);
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_copy_in(const double* in, T* f, const Box3& b, double rho0, cudaStream_t st) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
+  const CellLaunch rl = cell_launch(b, 128);
   k_copy_in<T><<<rl.grid, rl.block, 0, st>>>(in, f, b, rho0);
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_pack(const T* f, const Box3& b, T* out, cudaStream_t st) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
+  const CellLaunch rl = cell_launch(b, 128);
   k_pack<T><<<rl.grid, rl.block, 0, st>>>(f, b, out);
   return cudaGetLastError();
 }
 template <typename T>
 cudaError_t launch_unpack(const T* in, T* f, const Box3& b, cudaStream_t st) {
-  const RowLaunch rl = row_launch(b.n[0], b.n[1], b.n[2], 128);
+  const CellLaunch rl = cell_launch(b, 128);
   k_unpack<T><<<rl.grid, rl.block, 0, st>>>(in, f, b);
   return cudaGetLastError();
 }
