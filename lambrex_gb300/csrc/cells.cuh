@@ -389,38 +389,70 @@ __host__ __device__ __forceinline__ void cell_to_rform(const T* __restrict__ qpr
   for (int q = 0; q < NV; ++q) st_pop(r, (I)q * sq + c, b, p[q]);
 }
 
-// Explosion onto the fine ghost cell at storage (sx,sy,sz): the parent's
-// post-collision populations that will enter the patch within two fine
-// sub-steps (x + 2 c_q inside), empty otherwise.  QFORM: the coarse store
-// holds post-collision populations already (pull form).
+// A patch's ghost shell is as thick as a coarse cell, and the patch starts on
+// one, so the shell's cells are the children of the coarse ring around the
+// patch: ring cell (rx,ry,rz), counted from the shell's corner, has the children
+// at storage 2 r and 2 r + 1 of each axis.
+struct Ring {
+  int r[3];
+};
+template <typename I>
+__host__ __device__ __forceinline__ I ring_parent(const Coupling& c, const Ring& g) {
+  int P[3];
+  for (int d = 0; d < 3; ++d) {
+    P[d] = c.flo[d] / 2 + g.r[d] - 1;
+    if (c.cper) P[d] = wrapi(P[d], c.cdom[d]);
+  }
+  return sidx_i<I>(c.cb, P[0] - c.clo[0] + c.cb.g, P[1] - c.clo[1] + c.cb.g, P[2] - c.clo[2] + c.cb.g);
+}
+// whether population q of the ring cell's children enters the patch within two
+// fine sub-steps (x + 2 c_q inside; the same for all eight)
+__host__ __device__ __forceinline__ bool ring_enters(const Coupling& c, const Ring& g, int q) {
+  return in_valid(c.fb, 2 * (g.r[0] - 1 + CX(q)), 2 * (g.r[1] - 1 + CY(q)), 2 * (g.r[2] - 1 + CZ(q)));
+}
+// the eight children's populations, two of a row in one store
+template <typename T, typename I>
+__host__ __device__ __forceinline__ void st_children(T* __restrict__ fine, const Coupling& c,
+                                                     const Ring& g, const T* f) {
+  const I fsq = (I)c.fb.sq;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const I fc = sidx_i<I>(c.fb, 2 * g.r[0], 2 * g.r[1] + (m & 1), 2 * g.r[2] + (m >> 1));
+#pragma unroll
+    for (int q = 0; q < NV; ++q) st_pop2(fine, (I)q * fsq + fc, c.fb, f[q]);
+  }
+}
+
+// Explosion: the parent's post-collision populations that will enter the patch
+// within two fine sub-steps, empty otherwise.  QFORM: the coarse store holds
+// post-collision populations already (pull form); they are taken as they are,
+// so those that do not enter (two thirds of a face's) are not loaded.
+template <typename T, bool PAIRED, typename I, bool QFORM>
+__host__ __device__ __forceinline__ void explode_values(const T* __restrict__ coarse,
+                                                        const Coupling& c, const Ring& g, T om_s,
+                                                        T om_b, T rho0, const DfRates& r, T* f) {
+  const I cc = ring_parent<I>(c, g), csq = (I)c.cb.sq;
+#pragma unroll
+  for (int q = 0; q < NV; ++q)
+    f[q] = !QFORM || ring_enters(c, g, q) ? ld_pop(coarse, (I)q * csq + cc, c.cb) : zero_pop<T>(q, rho0);
+  if (QFORM) return;
+  collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);
+#pragma unroll
+  for (int q = 0; q < NV; ++q)
+    if (!ring_enters(c, g, q)) f[q] = zero_pop<T>(q, rho0);
+}
+// onto the one ghost cell at storage (sx,sy,sz)
 template <typename T, bool PAIRED = false, typename I = long long, bool QFORM = false>
 __host__ __device__ __forceinline__ void cell_explode(const T* __restrict__ coarse, T* __restrict__ fine,
                                              const Coupling& c, int sx, int sy, int sz, T om_s,
                                              T om_b, T rho0, const DfRates& r = DfRates{}) {
-  const int g = c.fb.g;
-  const int vx = sx - g, vy = sy - g, vz = sz - g;
-  if (in_valid(c.fb, vx, vy, vz)) return;
-  int P[3] = {floordiv2(c.flo[0] + vx), floordiv2(c.flo[1] + vy), floordiv2(c.flo[2] + vz)};
-  if (c.cper)
-    for (int d = 0; d < 3; ++d) P[d] = wrapi(P[d], c.cdom[d]);
-  const I cc = sidx_i<I>(c.cb, P[0] - c.clo[0] + c.cb.g, P[1] - c.clo[1] + c.cb.g,
-                         P[2] - c.clo[2] + c.cb.g);
-  const I csq = (I)c.cb.sq, fsq = (I)c.fb.sq;
+  const int w = c.fb.g;
+  if (in_valid(c.fb, sx - w, sy - w, sz - w)) return;
   T f[NV];
-  // post-collision populations are taken as they are, so those that do not
-  // enter (two thirds of a face's) are not loaded
+  explode_values<T, PAIRED, I, QFORM>(coarse, c, Ring{{sx / 2, sy / 2, sz / 2}}, om_s, om_b, rho0, r, f);
+  const I fc = sidx_i<I>(c.fb, sx, sy, sz), fsq = (I)c.fb.sq;
 #pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    const bool in = in_valid(c.fb, vx + 2 * CX(q), vy + 2 * CY(q), vz + 2 * CZ(q));
-    f[q] = !QFORM || in ? ld_pop(coarse, (I)q * csq + cc, c.cb) : zero_pop<T>(q, rho0);
-  }
-  if (!QFORM) collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);
-  const I fc = sidx_i<I>(c.fb, sx, sy, sz);
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    const bool in = QFORM || in_valid(c.fb, vx + 2 * CX(q), vy + 2 * CY(q), vz + 2 * CZ(q));
-    st_pop(fine, (I)q * fsq + fc, c.fb, in ? f[q] : zero_pop<T>(q, rho0));
-  }
+  for (int q = 0; q < NV; ++q) st_pop(fine, (I)q * fsq + fc, c.fb, f[q]);
 }
 
 // ---- rescaled coupling ------------------------------------------------------
@@ -429,31 +461,22 @@ __host__ __device__ __forceinline__ void cell_explode(const T* __restrict__ coar
 // Rescaling the non-equilibrium moments by s is the collision at rate 1 - s,
 // so both transfers are collisions at rates the host derives per coupling.
 //
-// Fine ghost cell at storage (sx,sy,sz) <- its parent's populations collided
-// at the explosion rates (the fine post-collision state, non-equilibrium
-// part rescaled to the fine level), interpolated in time: wp times the
-// parent at the start of the coarse step (cprev) plus wn times the parent at
-// its end (cnow; not read when wn == 0).
-template <typename T, bool PAIRED = false, typename I = long long>
-__host__ __device__ __forceinline__ void cell_explode_resc(const T* __restrict__ cprev,
-                                                  const T* __restrict__ cnow, T* __restrict__ fine,
-                                                  const Coupling& c, int sx, int sy, int sz,
-                                                  T om_s, T om_b, T rho0, T wp, T wn,
-                                                  const DfRates& r = DfRates{}) {
-  const int g = c.fb.g;
-  const int vx = sx - g, vy = sy - g, vz = sz - g;
-  if (in_valid(c.fb, vx, vy, vz)) return;
-  int P[3] = {floordiv2(c.flo[0] + vx), floordiv2(c.flo[1] + vy), floordiv2(c.flo[2] + vz)};
-  if (c.cper)
-    for (int d = 0; d < 3; ++d) P[d] = wrapi(P[d], c.cdom[d]);
-  const I cc = sidx_i<I>(c.cb, P[0] - c.clo[0] + c.cb.g, P[1] - c.clo[1] + c.cb.g,
-                         P[2] - c.clo[2] + c.cb.g);
-  const I csq = (I)c.cb.sq, fsq = (I)c.fb.sq;
-  T a[NV];
+// Fine ghost cell <- its parent's populations collided at the explosion rates
+// (the fine post-collision state, non-equilibrium part rescaled to the fine
+// level), interpolated in time: wp times the parent at the start of the coarse
+// step (cprev) plus wn times the parent at its end (cnow; not read when wn == 0).
+// FIRST: known to be the state before alone.
+template <typename T, bool PAIRED, typename I, bool FIRST = false>
+__host__ __device__ __forceinline__ void explode_resc_values(const T* __restrict__ cprev,
+                                                             const T* __restrict__ cnow,
+                                                             const Coupling& c, const Ring& g,
+                                                             T om_s, T om_b, T rho0, T wp, T wn,
+                                                             const DfRates& r, T* a) {
+  const I cc = ring_parent<I>(c, g), csq = (I)c.cb.sq;
 #pragma unroll
   for (int q = 0; q < NV; ++q) a[q] = ld_pop(cprev, (I)q * csq + cc, c.cb);
   collide_cell<T, PAIRED, true>(a, om_s, om_b, rho0, r);
-  if (wn != T(0)) {
+  if (!FIRST && wn != T(0)) {
     T b[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) b[q] = ld_pop(cnow, (I)q * csq + cc, c.cb);
@@ -461,7 +484,32 @@ __host__ __device__ __forceinline__ void cell_explode_resc(const T* __restrict__
 #pragma unroll
     for (int q = 0; q < NV; ++q) a[q] = weighted(wp, a[q], wn, b[q]);
   }
-  const I fc = sidx_i<I>(c.fb, sx, sy, sz);
+}
+// onto the children of a ring cell, the parent's collisions made once: FP64,
+// where they are what the explosion costs (104x88x72: 158 -> 149 us a coarse
+// step with the means' loads in pairs; FP32 and the conservative explosion are
+// faster with a thread a ghost cell, eight times the loads and stores in flight)
+template <typename T, bool PAIRED = false, typename I = long long>
+__host__ __device__ __forceinline__ void ring_explode_resc(const T* __restrict__ cprev,
+                                                  const T* __restrict__ cnow, T* __restrict__ fine,
+                                                  const Coupling& c, const Ring& g, T om_s, T om_b,
+                                                  T rho0, T wp, T wn, const DfRates& r = DfRates{}) {
+  T a[NV];
+  explode_resc_values<T, PAIRED, I>(cprev, cnow, c, g, om_s, om_b, rho0, wp, wn, r, a);
+  st_children<T, I>(fine, c, g, a);
+}
+template <typename T, bool PAIRED = false, typename I = long long, bool FIRST = false>
+__host__ __device__ __forceinline__ void cell_explode_resc(const T* __restrict__ cprev,
+                                                  const T* __restrict__ cnow, T* __restrict__ fine,
+                                                  const Coupling& c, int sx, int sy, int sz,
+                                                  T om_s, T om_b, T rho0, T wp, T wn,
+                                                  const DfRates& r = DfRates{}) {
+  const int w = c.fb.g;
+  if (in_valid(c.fb, sx - w, sy - w, sz - w)) return;
+  T a[NV];
+  explode_resc_values<T, PAIRED, I, FIRST>(cprev, cnow, c, Ring{{sx / 2, sy / 2, sz / 2}}, om_s, om_b,
+                                           rho0, wp, wn, r, a);
+  const I fc = sidx_i<I>(c.fb, sx, sy, sz), fsq = (I)c.fb.sq;
 #pragma unroll
   for (int q = 0; q < NV; ++q) st_pop(fine, (I)q * fsq + fc, c.fb, a[q]);
 }
@@ -485,11 +533,10 @@ __host__ __device__ __forceinline__ void cell_restrict_resc(const T* __restrict_
   for (int q = 0; q < NV; ++q) {
     T v[8];
 #pragma unroll
-    for (int m = 0; m < 8; ++m)
-      v[m] = ld_pop(fine,
-                    (I)q * fsq + sidx_i<I>(c.fb, 2 * rx + (m & 1) + g, 2 * ry + ((m >> 1) & 1) + g,
-                                           2 * rz + (m >> 2) + g),
-                    c.fb);
+    for (int m = 0; m < 8; m += 2)
+      ld_pop2(fine,
+              (I)q * fsq + sidx_i<I>(c.fb, 2 * rx + g, 2 * ry + ((m >> 1) & 1) + g, 2 * rz + (m >> 2) + g),
+              c.fb, v + m);
     f[q] = mean8(v);
   }
   collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);

@@ -104,6 +104,46 @@ __host__ __device__ __forceinline__ void st_pop(T* __restrict__ p, I i, const Bo
   if (idx_ok((long long)i, NV * b.sq)) p[i] = v;
 }
 
+// two neighbours of a row from an even element on, in one access
+__host__ __device__ __forceinline__ void ld_plain2(const double* p, double* v) {
+#ifdef __CUDA_ARCH__
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "l"(p));
+#else
+  v[0] = p[0], v[1] = p[1];
+#endif
+}
+__host__ __device__ __forceinline__ void ld_plain2(const float* p, float* v) {
+#ifdef __CUDA_ARCH__
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(p));
+#else
+  v[0] = p[0], v[1] = p[1];
+#endif
+}
+template <typename T, typename I>
+__host__ __device__ __forceinline__ void ld_pop2(const T* __restrict__ p, I i, const Box3& b, T* v) {
+  v[0] = v[1] = T(0);
+  if (idx_ok((long long)i, NV * b.sq) && idx_ok((long long)i + 1, NV * b.sq)) ld_plain2(p + i, v);
+}
+__host__ __device__ __forceinline__ void st_plain2(double* p, double v) {
+#ifdef __CUDA_ARCH__
+  *reinterpret_cast<double2*>(p) = make_double2(v, v);
+#else
+  p[0] = p[1] = v;
+#endif
+}
+__host__ __device__ __forceinline__ void st_plain2(float* p, float v) {
+#ifdef __CUDA_ARCH__
+  *reinterpret_cast<float2*>(p) = make_float2(v, v);
+#else
+  p[0] = p[1] = v;
+#endif
+}
+// v into both
+template <typename T, typename I>
+__host__ __device__ __forceinline__ void st_pop2(T* __restrict__ p, I i, const Box3& b, T v) {
+  if (idx_ok((long long)i, NV * b.sq) && idx_ok((long long)i + 1, NV * b.sq)) st_plain2(p + i, v);
+}
+
 // per-cell field of n elements (density, velocity components, partial sums)
 template <typename T>
 __host__ __device__ __forceinline__ T ld_cell(const T* __restrict__ p, long long i, long long n) {

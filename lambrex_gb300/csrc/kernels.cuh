@@ -37,9 +37,10 @@ inline CellLaunch cell_launch(const Box3& b, int threads) {
 // whether every element index of a store fits in 31 bits (512^3 does)
 inline bool index32(const Box3& b) { return (long long)NV * b.sq < (1ll << 31); }
 #ifdef __CUDACC__
-// (x, y, z) of this thread's cell under cell_launch; false beyond the last one
-__device__ __forceinline__ bool cell_xyz(const Box3& b, int& x, int& y, int& z) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+// (x, y, z) of this thread's cell under cell_launch (its first block being
+// block `first` of the grid); false beyond the last one
+__device__ __forceinline__ bool cell_xyz(const Box3& b, int& x, int& y, int& z, unsigned first = 0) {
+  const uint32_t c = (blockIdx.x - first) * blockDim.x + threadIdx.x;
   z = (int)divide(c, b.plane);
   const uint32_t p = c - (uint32_t)z * (uint32_t)(b.n[0] * b.n[1]);
   y = (int)divide(p, b.row);
@@ -168,6 +169,14 @@ template <typename T>
 cudaError_t launch_explode_resc(const T* cprev, const T* cnow, T* fine, const Coupling& c,
                                 double om_s, double om_b, double rho0, double wp, double wn,
                                 cudaStream_t st, bool paired = false);
+// Both at once: the step of a periodic level (launch_step_periodic, refined) and
+// the explosion onto the level above it of the state the step starts from
+// (launch_explode, or with rescaled launch_explode_resc at wp = 1, wn = 0 and
+// the rates es, eb)
+template <typename T>
+cudaError_t launch_step_explode(const T* fin, T* fout, const Box3& b, IBox covered, double om_s,
+                                double om_b, double rho0, T* fine, const Coupling& c, bool rescaled,
+                                double es, double eb, cudaStream_t st, bool paired = false);
 // covered coarse cells <- mean of their children collided at the restriction rates
 template <typename T>
 cudaError_t launch_restrict_resc(const T* fine, T* coarse, const Coupling& c, double om_s,

@@ -47,9 +47,9 @@ template <typename T, bool PAIRED, typename I>
 __global__ void k_explode(const T* __restrict__ coarse, T* __restrict__ fine, Coupling c, T om_s,
                           T om_b, T rho0, DfRates r) {
   chain_begin();
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   int s[3];
-  if (t >= ghost_cells_of(c.fb) || !ghost_coords(c.fb, (int)t, s)) return;
+  if (t >= ghost_cells_of(c.fb) || !ghost_coords(c.fb, t, s)) return;
   cell_explode<T, PAIRED, I>(coarse, fine, c, s[0], s[1], s[2], om_s, om_b, rho0, r);
 }
 
@@ -89,10 +89,42 @@ __global__ void k_explode_resc(const T* __restrict__ cprev, const T* __restrict_
                                T* __restrict__ fine, Coupling c, T om_s, T om_b, T rho0, T wp, T wn,
                                DfRates r) {
   chain_begin();
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  int s[3];
-  if (t >= ghost_cells_of(c.fb) || !ghost_coords(c.fb, (int)t, s)) return;
-  cell_explode_resc<T, PAIRED, I>(cprev, cnow, fine, c, s[0], s[1], s[2], om_s, om_b, rho0, wp, wn, r);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if constexpr (sizeof(T) == 8) {
+    Ring g;
+    if (t >= ring_cells_of(c) || !ring_coords(c, t, g.r)) return;
+    ring_explode_resc<T, PAIRED, I>(cprev, cnow, fine, c, g, om_s, om_b, rho0, wp, wn, r);
+  } else {
+    int s[3];
+    if (t >= ghost_cells_of(c.fb) || !ghost_coords(c.fb, t, s)) return;
+    cell_explode_resc<T, PAIRED, I>(cprev, cnow, fine, c, s[0], s[1], s[2], om_s, om_b, rho0, wp, wn, r);
+  }
+}
+
+// The step of a periodic level and the explosion of the state it starts from in
+// one launch: they read the same store and write different ones.  The explosion
+// alone is a chain of latencies (4 us for the 2 MB of a 32^3 patch, at 15 % of
+// the warp slots); as the first blocks of the step's launch it is done before
+// the step is.  64^3 conservative FP32: 25.4 -> 22.9 us a coarse step.
+template <typename T, bool COVER, bool PAIRED, typename I, bool RESC>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 1)
+    k_step_explode(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov, T om_s, T om_b,
+                   T rho0, DfRates r, T* __restrict__ fine, Coupling c, T es, T eb, DfRates re,
+                   unsigned first) {
+  chain_begin();
+  if (blockIdx.x < first) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    int s[3];
+    if (t >= ghost_cells_of(c.fb) || !ghost_coords(c.fb, t, s)) return;
+    if (RESC)  // the state before the step alone
+      cell_explode_resc<T, PAIRED, I, true>(fin, fin, fine, c, s[0], s[1], s[2], es, eb, rho0, T(1), T(0), re);
+    else
+      cell_explode<T, PAIRED, I>(fin, fine, c, s[0], s[1], s[2], om_s, om_b, rho0, r);
+    return;
+  }
+  int x, y, z;
+  if (!cell_xyz(b, x, y, z, first)) return;
+  cell_step_periodic<T, COVER, PAIRED, I>(fin, fout, b, cov, x, y, z, om_s, om_b, rho0, r);
 }
 
 template <typename T, bool PAIRED, typename I>
@@ -179,6 +211,8 @@ inline long long grown_coarse_cells(const Box3& fb) {
 
 }  // namespace
 
+// threads of a block over ring cells: one warp, to reach every SM
+constexpr int kRingThreads = 32;
 // f(index type) with int where every element index of the boxes fits in 31
 // bits: the kernels here are bound by instructions and latency, and 64-bit
 // element offsets took a third of the instructions of a patch step
@@ -249,16 +283,46 @@ template <typename T>
 cudaError_t launch_explode_resc(const T* cprev, const T* cnow, T* fine, const Coupling& c,
                                 double om_s, double om_b, double rho0, double wp, double wn,
                                 cudaStream_t st, bool paired) {
-  const unsigned grid = blocks_for(ghost_cells_of(c.fb), 128);
+  const int threads = sizeof(T) == 8 ? kRingThreads : 128;
+  const unsigned grid =
+      blocks_for(sizeof(T) == 8 ? ring_cells_of(c) : ghost_cells_of(c.fb), threads);
   const DfRates r = quiet(rates_of<T>(om_s, om_b));
   with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
     using I = decltype(i);
     if (sizeof(T) == 8 && paired)
-      chained(k_explode_resc<T, sizeof(T) == 8, I>, grid, 128, st, cprev, cnow, fine, c, (T)om_s, (T)om_b, (T)rho0, (T)wp, (T)wn, r);
+      chained(k_explode_resc<T, sizeof(T) == 8, I>, grid, threads, st, cprev, cnow, fine, c, (T)om_s, (T)om_b, (T)rho0, (T)wp, (T)wn, r);
     else
-      chained(k_explode_resc<T, false, I>, grid, 128, st, cprev, cnow, fine, c, (T)om_s, (T)om_b,
+      chained(k_explode_resc<T, false, I>, grid, threads, st, cprev, cnow, fine, c, (T)om_s, (T)om_b,
                                                         (T)rho0, (T)wp, (T)wn, r);
   });
+  return cudaGetLastError();
+}
+
+template <typename T, bool COVER, bool PAIRED, bool RESC>
+static void step_explode(const T* fin, T* fout, const Box3& b, const IBox& cov, double om_s,
+                         double om_b, double rho0, T* fine, const Coupling& c, double es, double eb,
+                         cudaStream_t st) {
+  const unsigned first = blocks_for(ghost_cells_of(c.fb), 128);
+  const unsigned cells = blocks_for((long long)b.n[0] * b.n[1] * b.n[2], 128);
+  with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
+    chained(k_step_explode<T, COVER, PAIRED, decltype(i), RESC>, first + cells, 128, st, fin, fout, b,
+            cov, (T)om_s, (T)om_b, (T)rho0, quiet(rates_of<T>(om_s, om_b)), fine, c, (T)es, (T)eb,
+            quiet(rates_of<T>(es, eb)), first);
+  });
+}
+template <typename T>
+cudaError_t launch_step_explode(const T* fin, T* fout, const Box3& b, IBox covered, double om_s,
+                                double om_b, double rho0, T* fine, const Coupling& c, bool rescaled,
+                                double es, double eb, cudaStream_t st, bool paired) {
+  constexpr bool P = sizeof(T) == 8;
+  if (rescaled && P && paired)
+    step_explode<T, false, P, true>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st);
+  else if (rescaled)
+    step_explode<T, false, false, true>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st);
+  else if (P && paired)
+    step_explode<T, true, P, false>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st);
+  else
+    step_explode<T, true, false, false>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st);
   return cudaGetLastError();
 }
 
@@ -290,6 +354,9 @@ cudaError_t launch_fill_from_coarse(const T* coarse, T* fine, const Coupling& c,
                                          cudaStream_t, bool);                                  \
   template cudaError_t launch_step_patch<T>(const T*, T*, const Box3&, IBox, double, double,   \
                                             double, cudaStream_t, bool);                       \
+  template cudaError_t launch_step_explode<T>(const T*, T*, const Box3&, IBox, double, double, \
+                                              double, T*, const Coupling&, bool, double,       \
+                                              double, cudaStream_t, bool);                     \
   template cudaError_t launch_coalesce<T>(const T*, T*, const Coupling&, double, cudaStream_t); \
   template cudaError_t launch_restrict<T>(const T*, T*, const Coupling&, cudaStream_t);        \
   template cudaError_t launch_fill_from_coarse<T>(const T*, T*, const Coupling&, cudaStream_t); \

@@ -455,19 +455,28 @@ template <typename T>
 int c_advance(lbx_sim* s, int L) {
   Level& l = s->lev[L];
   const bool paired = s->precision == LBX_F64_PAIRED;
-  if (L < s->finest) {
-    Level& f = s->lev[L + 1];
-    CK(lbx::launch_explode<T>(P<T>(l.buf[l.now]), P<T>(f.buf[f.now]), coupling(s, L + 1),
-                              omega(l.tau_s), omega(l.tau_b), s->rho0, s->stream, paired));
-  }
   const IBox cov = covered_box(s, L);
-  s->launches += (L < s->finest) ? 3 : 1;  // explode, step, coalesce
-  if (L == 0)
-    CK(lbx::launch_step_periodic<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box, cov,
-                                    omega(l.tau_s), omega(l.tau_b), s->rho0, s->stream, paired, true));
-  else
-    CK(lbx::launch_step_patch<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box, cov,
-                                 omega(l.tau_s), omega(l.tau_b), s->rho0, s->stream, paired));
+  if (L == 0 && s->finest > 0) {
+    Level& f = s->lev[1];
+    s->launches += 2;  // explosion and step, coalescence
+    CK(lbx::launch_step_explode<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box, cov,
+                                   omega(l.tau_s), omega(l.tau_b), s->rho0, P<T>(f.buf[f.now]),
+                                   coupling(s, 1), false, 0.0, 0.0, s->stream, paired));
+  } else {
+    if (L < s->finest) {
+      Level& f = s->lev[L + 1];
+      CK(lbx::launch_explode<T>(P<T>(l.buf[l.now]), P<T>(f.buf[f.now]), coupling(s, L + 1),
+                                omega(l.tau_s), omega(l.tau_b), s->rho0, s->stream, paired));
+    }
+    s->launches += (L < s->finest) ? 3 : 1;  // explosion, step, coalescence
+    if (L == 0)
+      CK(lbx::launch_step_periodic<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box, cov,
+                                      omega(l.tau_s), omega(l.tau_b), s->rho0, s->stream, paired,
+                                      true));
+    else
+      CK(lbx::launch_step_patch<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box, cov,
+                                   omega(l.tau_s), omega(l.tau_b), s->rho0, s->stream, paired));
+  }
   std::swap(l.now, l.next);
   if (L < s->finest) {
     RET(c_advance<T>(s, L + 1));
@@ -514,25 +523,36 @@ template <typename T>
 int r_advance(lbx_sim* s, int L) {
   Level& l = s->lev[L];
   const bool paired = s->precision == LBX_F64_PAIRED;
+  const bool both = L == 0 && s->finest > 0;  // the step and the first explosion at once
   ++s->launches;
-  if (L == 0)
+  if (both) {
+    Level& f = s->lev[1];
+    const ResRates R = resc_rates(s, 1);
+    CK(lbx::launch_step_explode<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box,
+                                   lbx::empty_ibox(), omega(l.tau_s), omega(l.tau_b), s->rho0,
+                                   P<T>(f.buf[f.now]), coupling(s, 1), true, R.es, R.eb, s->stream,
+                                   paired));
+  } else if (L == 0) {
     CK(lbx::launch_step_periodic<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box,
                                     lbx::empty_ibox(), omega(l.tau_s), omega(l.tau_b), s->rho0,
                                     s->stream, paired, true));
-  else
+  } else {
     CK(lbx::launch_step_patch<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box,
                                  lbx::empty_ibox(), omega(l.tau_s), omega(l.tau_b), s->rho0,
                                  s->stream, paired));
+  }
   std::swap(l.now, l.next);
   if (L < s->finest) {
     Level& f = s->lev[L + 1];
     const Coupling cp = coupling(s, L + 1);
     const ResRates R = resc_rates(s, L + 1);
     for (int k = 0; k < 2; ++k) {
-      CK(lbx::launch_explode_resc<T>(P<T>(l.buf[l.next]), P<T>(l.buf[l.now]), P<T>(f.buf[f.now]),
-                                     cp, R.es, R.eb, s->rho0, 1.0 - 0.5 * k, 0.5 * k, s->stream,
-                                     paired));
-      ++s->launches;
+      if (k > 0 || !both) {
+        CK(lbx::launch_explode_resc<T>(P<T>(l.buf[l.next]), P<T>(l.buf[l.now]), P<T>(f.buf[f.now]),
+                                       cp, R.es, R.eb, s->rho0, 1.0 - 0.5 * k, 0.5 * k, s->stream,
+                                       paired));
+        ++s->launches;
+      }
       RET(r_advance<T>(s, L + 1));
     }
     CK(lbx::launch_restrict_resc<T>(P<T>(f.buf[f.now]), P<T>(l.buf[l.now]), cp, R.rs, R.rb,
