@@ -73,10 +73,14 @@ struct lbx_ensemble {
   cudaStream_t stream = nullptr;
   cudaGraphExec_t gexec = nullptr;
   long long launches = 0, last_launches = 0;
+  double* d_fields = nullptr;  // density and velocity of one box (lbx_ensemble_hydro)
+  size_t fields_cap = 0;       // bytes
   size_t esize() const { return precision == LBX_F64 ? 8 : 4; }
 };
 
 namespace {
+
+constexpr size_t kFieldsKept = (size_t)128 << 20;
 
 // Launch shape until the caller sets or tunes it: blocks of 256 threads (FP64
 // 128, for its registers) and as many tiles as keep the blocks of the persistent
@@ -229,6 +233,7 @@ int lbx_ensemble_destroy(lbx_ensemble* e) {
       if (p) cudaFree(p);
   if (e->d_boxes) cudaFree(e->d_boxes);
   if (e->d_tiles) cudaFree(e->d_tiles);
+  if (e->d_fields) cudaFree(e->d_fields);
   if (e->stream) cudaStreamDestroy(e->stream);
   delete e;
   return LBX_OK;
@@ -374,18 +379,33 @@ int lbx_ensemble_copy_f(lbx_ensemble* e, int b, double* out, size_t n) {
 int lbx_ensemble_hydro(lbx_ensemble* e, int b, double* rho, double* u, size_t ncells) {
   if (!e || b < 0 || b >= e->nbox || !rho || !u) return LBX_ERR_ARG;
   const BBox& B = e->hb[b];
-  const size_t N = (size_t)B.b.n[0] * B.b.n[1] * B.b.n[2];
+  const size_t N = (size_t)B.b.n[0] * B.b.n[1] * B.b.n[2], bytes = 4 * N * sizeof(double);
   if (ncells < N) return LBX_ERR_ARG;
+  // the fields' device memory is kept up to kFieldsKept: from the device's pool
+  // it would be mapped and unmapped again at each call
   double* d = nullptr;
-  CK(cudaMallocAsync(&d, 4 * N * sizeof(double), e->stream));
+  if (bytes <= kFieldsKept) {
+    if (bytes > e->fields_cap) {
+      if (e->d_fields) CK(cudaFree(e->d_fields));
+      e->d_fields = nullptr;
+      e->fields_cap = 0;
+      CK(cudaMalloc(&e->d_fields, bytes));
+      e->fields_cap = bytes;
+    }
+    d = e->d_fields;
+  } else {
+    CK(cudaMallocAsync(&d, bytes, e->stream));
+  }
   const int now = box_now(e, b);
   cudaError_t err = e->precision == LBX_F64
                         ? lbx::launch_hydro<double>(static_cast<double*>(B.buf[now]), B.b, 0.0, d, d + N, e->stream, B.pull != 0)
                         : lbx::launch_hydro<float>(static_cast<float*>(B.buf[now]), B.b, B.rho0, d, d + N, e->stream, B.pull != 0);
-  if (err == cudaSuccess) err = cudaMemcpyAsync(rho, d, N * sizeof(double), cudaMemcpyDeviceToHost, e->stream);
-  if (err == cudaSuccess) err = cudaMemcpyAsync(u, d + N, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, e->stream);
-  cudaFreeAsync(d, e->stream);
-  if (err == cudaSuccess) err = cudaStreamSynchronize(e->stream);
+  if (err == cudaSuccess) err = lbx::download_host(rho, d, N * sizeof(double), e->stream);
+  if (err == cudaSuccess) err = lbx::download_host(u, d + N, 3 * N * sizeof(double), e->stream);
+  if (d != e->d_fields) {
+    cudaFreeAsync(d, e->stream);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(e->stream);
+  }
   CK(err);
   return LBX_OK;
 }

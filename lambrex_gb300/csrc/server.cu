@@ -18,6 +18,8 @@
 #include <cstring>
 #include <deque>
 #include <map>
+#include <memory>
+#include <new>
 #include <vector>
 
 #include "batch.cuh"
@@ -75,7 +77,8 @@ struct Req {
   ReqLevel lev[kMaxLevels];
   size_t bytes = 0;
   double mass = 0.0, probe = 0.0;
-  std::vector<double> rho;  // level-0 density at completion (if kept)
+  std::unique_ptr<double[]> rho;  // level-0 density at completion (if kept)
+  size_t nrho = 0;
 };
 
 size_t level_bytes(const int* n, int ghost, int esize) {
@@ -112,6 +115,8 @@ struct lbx_server {
   long long graph_launches = 0;
   cudaStream_t stream = nullptr;
   cudaMemPool_t pool = nullptr;  // request stores (release threshold = budget)
+  double* d_work = nullptr;  // partial sums, then the sums of each level
+  double* h_work = nullptr;  // page-locked: those and the probe
   int num_sms = 0, block = 128, cpt = 1;  // measured best on GB300
   int tile_cells = 1024;  // at most (fitting_tile), or as the caller set it
   bool tuned = false;
@@ -461,27 +466,15 @@ int finish_request(lbx_server* s, Req& q) {
     CK(lbx::launch_b_to_rform<T>(static_cast<const T*>(B.buf[now ^ 1]), static_cast<T*>(B.buf[now]),
                                  B.b, s->stream));
   }
-  // composite mass: uncovered cells of each level weighted by 8^-L
-  double* d = nullptr;
-  CK(cudaMallocAsync(&d, (lbx::reduce_partials_doubles() + 8) * sizeof(double), s->stream));
-  long double mass = 0, vol = 1;
-  double h[4];
+  // composite mass: uncovered cells of each level weighted by 8^-L; the sums
+  // are read with the density below
+  double* sums = s->d_work + lbx::reduce_partials_doubles();
   for (int L = 0; L < q.nlev; ++L) {
     const BBox& B = q.lev[L].box;
     const IBox skip = (L + 1 < q.nlev) ? B.cov : lbx::empty_ibox();
-    cudaError_t e = lbx::launch_reduce<T>(static_cast<const T*>(B.buf[B.par ^ s->F[L]]), B.b, skip, B.rho0, d + 8,
-                                          d, s->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, 4 * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-    if (e != cudaSuccess) {
-      cudaFreeAsync(d, s->stream);
-      CK(e);
-    }
-    mass += vol * (long double)h[0];
-    vol /= 8;
+    CK(lbx::launch_reduce<T>(static_cast<const T*>(B.buf[B.par ^ s->F[L]]), B.b, skip, B.rho0, s->d_work,
+                             sums + 4 * L, s->stream));
   }
-  cudaFreeAsync(d, s->stream);
-  q.mass = (double)mass;
   // covered cells of each level <- mean of their children (finest pair first)
   for (int L = q.nlev - 1; L >= 1; --L) {
     const BBox& F = q.lev[L].box;
@@ -493,22 +486,30 @@ int finish_request(lbx_server* s, Req& q) {
   const BBox& B0 = q.lev[0].box;
   const size_t N = (size_t)q.r.nx * q.r.ny * q.r.nz;
   double* dr = nullptr;
-  CK(cudaMallocAsync(&dr, 4 * N * sizeof(double), s->stream));
+  CK(cudaMallocFromPoolAsync(&dr, 4 * N * sizeof(double), s->pool, s->stream));
   cudaError_t e = lbx::launch_hydro<T>(static_cast<const T*>(B0.buf[B0.par ^ s->F[0]]), B0.b, B0.rho0, dr, dr + N,
                                        s->stream);
   int pc[3] = {q.r.nx / 2, q.r.ny / 2, q.r.nz / 2};
   pc[q.r.pulse_axis] = q.r.pulse_index;
   const size_t probe_at = ((size_t)pc[2] * q.r.ny + pc[1]) * q.r.nx + pc[0];
-  std::vector<double> rho(q.r.keep_field ? N : 0);
   if (e == cudaSuccess)
-    e = q.r.keep_field
-            ? cudaMemcpyAsync(rho.data(), dr, N * sizeof(double), cudaMemcpyDeviceToHost, s->stream)
-            : cudaMemcpyAsync(&q.probe, dr + probe_at, sizeof(double), cudaMemcpyDeviceToHost, s->stream);
+    e = cudaMemcpyAsync(s->h_work, sums, 4 * kMaxLevels * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(s->h_work + 4 * kMaxLevels, dr + probe_at, sizeof(double), cudaMemcpyDeviceToHost,
+                        s->stream);
+  if (e == cudaSuccess && q.r.keep_field) {
+    q.rho.reset(new (std::nothrow) double[N]);
+    q.nrho = N;
+    e = q.rho ? lbx::download_host(q.rho.get(), dr, N * sizeof(double), s->stream)
+              : cudaErrorMemoryAllocation;
+  }
   cudaFreeAsync(dr, s->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   CK(e);
-  if (q.r.keep_field) q.probe = rho[probe_at];
-  q.rho = std::move(rho);
+  long double mass = 0, vol = 1;
+  for (int L = 0; L < q.nlev; ++L, vol /= 8) mass += vol * (long double)s->h_work[4 * L];
+  q.mass = (double)mass;
+  q.probe = s->h_work[4 * kMaxLevels];
   return LBX_OK;
 }
 
@@ -539,8 +540,12 @@ int lbx_server_create(size_t hbm_budget_bytes, int max_active, int precision, lb
       e = cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
   }
+  if (e == cudaSuccess)
+    e = cudaMalloc(&s->d_work, (lbx::reduce_partials_doubles() + 4 * kMaxLevels) * sizeof(double));
+  if (e == cudaSuccess) e = cudaMallocHost(&s->h_work, (4 * kMaxLevels + 1) * sizeof(double));
   if (e != cudaSuccess) {
     lbx::note_error("lbx_server_create", e);
+    if (s->d_work) cudaFree(s->d_work);
     if (s->pool) cudaMemPoolDestroy(s->pool);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -581,6 +586,8 @@ int lbx_server_destroy(lbx_server* s) {
   if (s->gexec) cudaGraphExecDestroy(s->gexec);
   if (s->d_tables) cudaFree(s->d_tables);
   if (s->h_tables) cudaFreeHost(s->h_tables);
+  if (s->d_work) cudaFree(s->d_work);
+  if (s->h_work) cudaFreeHost(s->h_work);
   if (s->stream) {
     cudaStreamSynchronize(s->stream);  // pool frees are stream-ordered
     cudaStreamDestroy(s->stream);
@@ -623,9 +630,9 @@ int lbx_server_submit(lbx_server* s, const lbx_request* r, long long* id) {
   }
   if (request_bytes(q, (int)s->esize()) > s->budget) return LBX_ERR_OOM;
   q.id = s->next_id++;
-  s->reqs[q.id] = q;
-  s->queue.push_back(q.id);
   *id = q.id;
+  s->queue.push_back(q.id);
+  s->reqs[*id] = std::move(q);
   return LBX_OK;
 }
 
@@ -712,8 +719,8 @@ int lbx_server_take(lbx_server* s, long long id, double* rho, size_t n) {
   if (it == s->reqs.end()) return LBX_ERR_NOT_FOUND;
   if (it->second.state != 2) return LBX_ERR_STATE;
   if (rho) {
-    if (n < it->second.rho.size()) return LBX_ERR_ARG;
-    std::copy(it->second.rho.begin(), it->second.rho.end(), rho);
+    if (n < it->second.nrho) return LBX_ERR_ARG;
+    std::copy(it->second.rho.get(), it->second.rho.get() + it->second.nrho, rho);
   }
   s->reqs.erase(it);
   return LBX_OK;

@@ -158,7 +158,9 @@ struct lbx_sim {
   // hydro pass alone, so that a final readout costs no extra step
   bool fuse_hydro = false;
   bool hydro_since_iterate = false;
-  int nbuf() const { return amr_mode == LBX_AMR_FAITHFUL ? 3 : 2; }
+  // the third is the faithful cycle's stream buffer: a run that cannot refine
+  // never enters it
+  int nbuf() const { return amr_mode == LBX_AMR_FAITHFUL && max_level > 0 ? 3 : 2; }
   // FP64 store (LBX_F64 and LBX_F64_PAIRED) or FP32 shifted store
   bool f64() const { return precision != LBX_F32_SHIFTED; }
   size_t esize() const { return f64() ? sizeof(double) : sizeof(float); }

@@ -37,6 +37,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -217,6 +218,12 @@ class CopyPool {
   std::atomic<unsigned> left_{0};
 };
 
+// the process's copy threads, started on first use
+CopyPool& copy_pool() {
+  static CopyPool pool(std::min(kMaxCopyThreads, std::max(1u, std::thread::hardware_concurrency())));
+  return pool;
+}
+
 // process-wide staging area (allocated on first use, kept until exit)
 struct Stage {
   std::mutex mu;
@@ -261,9 +268,7 @@ cudaError_t stage_setup(Stage& S) {
         return e;
       }
     }
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    static CopyPool pool(std::min(kMaxCopyThreads, hw));
-    S.pool = &pool;
+    S.pool = &copy_pool();
   }
   stage_drop_events(S);
   S.device = -1;
@@ -320,6 +325,63 @@ cudaError_t copy_direct_while_fast(char* dst, const char* src, size_t bytes, cud
 
 }  // namespace
 
+// Downloads of 1 to 64 MB into pageable memory: fields of a level, a box or a
+// request, which programs mostly read into arrays made for them.  Such pages are
+// new, and what a copy into them costs is making them, one after another in the
+// copying thread.  They arrive in two page-locked buffers and the copy threads
+// bring them over: 24 boxes of 13 MB in 9 ms of an ensemble's pass, against 7 to
+// 25 by direct copies (fast or slow for a whole process).
+constexpr size_t kSmallMin = (size_t)1 << 20;
+constexpr size_t kSmallChunk = (size_t)4 << 20;
+struct SmallStage {
+  std::mutex mu;
+  char* buf[2] = {};
+  bool failed = false;
+};
+static SmallStage& small_stage() {
+  static SmallStage s;
+  return s;
+}
+static cudaError_t download_small(char* dst, const char* src, size_t bytes, cudaStream_t st) {
+  SmallStage& S = small_stage();
+  std::unique_lock<std::mutex> lock(S.mu, std::try_to_lock);
+  if (lock && !S.buf[0] && !S.failed) {
+    char* p = nullptr;
+    bool threads = true;
+    try {
+      copy_pool();
+    } catch (const std::exception&) {  // no threads to be had
+      threads = false;
+    }
+    if (threads && cudaHostAlloc(&p, 2 * kSmallChunk, cudaHostAllocPortable) == cudaSuccess) {
+      S.buf[0] = p;
+      S.buf[1] = p + kSmallChunk;
+    } else {
+      cudaGetLastError();
+      S.failed = true;
+    }
+  }
+  if (!lock || !S.buf[0]) {  // in use by another thread, or not to be had: directly
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+  }
+  // each chunk is waited for before the next one is asked for, so that the
+  // stream holds one copy more at most while a chunk is brought over
+  const size_t chunks = (bytes + kSmallChunk - 1) / kSmallChunk;
+  auto len = [&](size_t c) { return std::min(kSmallChunk, bytes - c * kSmallChunk); };
+  cudaError_t e = cudaMemcpyAsync(S.buf[0], src, len(0), cudaMemcpyDeviceToHost, st);
+  for (size_t c = 0; c < chunks; ++c) {
+    const cudaError_t w = cudaStreamSynchronize(st);  // also when a copy could not be queued
+    if (e == cudaSuccess) e = w;
+    if (e != cudaSuccess) return e;
+    if (c + 1 < chunks)
+      e = cudaMemcpyAsync(S.buf[(c + 1) & 1], src + (c + 1) * kSmallChunk, len(c + 1),
+                          cudaMemcpyDeviceToHost, st);
+    copy_pool().copy(dst + c * kSmallChunk, S.buf[c & 1], len(c));
+  }
+  return e;
+}
+
 // whether p is page-locked host memory known to CUDA (cudaHostAlloc,
 // cudaHostRegister, or pinned by another user of the same context): the copy
 // engine moves it at the link rate (211 GB/s measured for 4.3 GB), while a
@@ -363,6 +425,8 @@ cudaError_t upload_host(void* dst, const void* src, size_t bytes, cudaStream_t s
 }
 
 cudaError_t download_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  if (bytes >= kSmallMin && bytes < kStageMin && !pinned_host(dst))
+    return download_small(static_cast<char*>(dst), static_cast<const char*>(src), bytes, st);
   if (bytes < kStageMin || pinned_host(dst)) {
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
     return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
