@@ -242,6 +242,23 @@ __host__ __device__ __forceinline__ void cell_fill_from_coarse(const T* __restri
     st_pop(fine, q * c.fb.sq + fc, c.fb, ld_pop_ro(coarse, q * c.cb.sq + cc, c.cb));
 }
 
+// Faces of the storage that cell (sx,sy,sz) lies on, one bit a face (x low, x
+// high, y low, ...), and the faces through which population q leaves the storage
+// from such a cell, or would have come.  A row of a 64^3 patch is two warps, each
+// with a cell on a face: with a path of its own for such cells nearly every warp
+// took both.
+__host__ __device__ __forceinline__ unsigned face_bits(const Box3& b, int sx, int sy, int sz) {
+  const int g = 2 * b.g - 1;
+  return (sx == 0) | (sx == b.n[0] + g) << 1 | (sy == 0) << 2 | (sy == b.n[1] + g) << 3 |
+         (sz == 0) << 4 | (sz == b.n[2] + g) << 5;
+}
+__host__ __device__ constexpr unsigned faces_out(int cx, int cy, int cz) {
+  return (cx < 0 ? 1u : cx > 0 ? 2u : 0u) | (cy < 0 ? 4u : cy > 0 ? 8u : 0u) |
+         (cz < 0 ? 16u : cz > 0 ? 32u : 0u);
+}
+__host__ __device__ constexpr unsigned faces_out(int q) { return faces_out(CX(q), CY(q), CZ(q)); }
+__host__ __device__ constexpr unsigned faces_in(int q) { return faces_out(-CX(q), -CY(q), -CZ(q)); }
+
 // AMR patch, storage cell (sx,sy,sz) of the grown box: valid cells collide
 // (covered ones emit zeros), ghost cells stream raw, pushes leaving the
 // storage are dropped and entries nothing streams into are set empty.
@@ -264,23 +281,15 @@ __host__ __device__ __forceinline__ void cell_step_patch(const T* __restrict__ f
     for (int q = 0; q < NV; ++q) f[q] = ld_pop(fin, (I)q * sq + c, b);
     if (valid) collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);
   }
-  const int SX = b.n[0] + 2 * g, SY = b.n[1] + 2 * g, SZ = b.n[2] + 2 * g;
-  if (sx > 0 && sx < SX - 1 && sy > 0 && sy < SY - 1 && sz > 0 && sz < SZ - 1) {
-    // every target lies in the storage and every source too: constant offsets
+  const unsigned m = face_bits(b, sx, sy, sz);
 #pragma unroll
-    for (int q = 0; q < NV; ++q)
-      st_pop(fout, (I)q * sq + c + (I)CZ(q) * rxy + (I)CY(q) * rx + (I)CX(q), b, f[q]);
-    return;
-  }
+  for (int q = 0; q < NV; ++q)
+    if (!(m & faces_out(q)))
+      st_pop(fout, (I)q * sq + c + ((I)CZ(q) * rxy + (I)CY(q) * rx + (I)CX(q)), b, f[q]);
+  if (m == 0) return;
 #pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    const int tx = sx + CX(q), ty = sy + CY(q), tz = sz + CZ(q);
-    if (tx >= 0 && tx < SX && ty >= 0 && ty < SY && tz >= 0 && tz < SZ)
-      st_pop(fout, (I)q * sq + sidx_i<I>(b, tx, ty, tz), b, f[q]);
-    const int ux = sx - CX(q), uy = sy - CY(q), uz = sz - CZ(q);
-    if (!(ux >= 0 && ux < SX && uy >= 0 && uy < SY && uz >= 0 && uz < SZ))
-      st_pop(fout, (I)q * sq + c, b, zero_pop<T>(q, rho0));
-  }
+  for (int q = 0; q < NV; ++q)
+    if (m & faces_in(q)) st_pop(fout, (I)q * sq + c, b, zero_pop<T>(q, rho0));
 }
 
 // ---- pull form of the conservative coupling (batch engine) ------------------
@@ -327,20 +336,12 @@ __host__ __device__ __forceinline__ void cell_step_patch_pull(const T* __restric
     return;
   }
   T f[NV];
-  const int SX = b.n[0] + 2 * g, SY = b.n[1] + 2 * g, SZ = b.n[2] + 2 * g;
-  if (sx > 0 && sx < SX - 1 && sy > 0 && sy < SY - 1 && sz > 0 && sz < SZ - 1) {
+  const unsigned m = face_bits(b, sx, sy, sz);
 #pragma unroll
-    for (int q = 0; q < NV; ++q)
-      f[q] = ld_pop(fin, (I)q * sq + c - ((I)CZ(q) * rxy + (I)CY(q) * rx + (I)CX(q)), b);
-  } else {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      const int ux = sx - CX(q), uy = sy - CY(q), uz = sz - CZ(q);
-      f[q] = (ux >= 0 && ux < SX && uy >= 0 && uy < SY && uz >= 0 && uz < SZ)
-                 ? ld_pop(fin, (I)q * sq + sidx_i<I>(b, ux, uy, uz), b)
-                 : zero_pop<T>(q, rho0);
-    }
-  }
+  for (int q = 0; q < NV; ++q)
+    f[q] = m & faces_in(q)
+               ? zero_pop<T>(q, rho0)
+               : ld_pop(fin, (I)q * sq + c - ((I)CZ(q) * rxy + (I)CY(q) * rx + (I)CX(q)), b);
   if (valid) collide_cell<T, false, true>(f, om_s, om_b, rho0, r);
 #pragma unroll
   for (int q = 0; q < NV; ++q) st_pop(fout, (I)q * sq + c, b, f[q]);

@@ -245,6 +245,7 @@ __host__ __device__ __forceinline__ uint32_t divide(uint32_t x, const Divisor& d
 struct Box3 {
   int n[3];        // valid extents
   Divisor row, plane;  // of valid cells in order, by n[0] and by n[0] n[1]
+  Divisor srow;        // of storage cells, by sx
   int g;           // ghost layers in storage
   long long sx;    // row length  = n[0] + 2g
   long long sxy;   // plane size  = (n[1] + 2g) * sx
@@ -263,6 +264,7 @@ inline Box3 make_box(int nx, int ny, int nz, int g) {
   b.plane = make_divisor((uint32_t)((long long)nx * ny));
   b.g = g;
   b.sx = nx + 2 * g;
+  b.srow = make_divisor((uint32_t)b.sx);
   b.sxy = (long long)(ny + 2 * g) * b.sx;
   b.sq = (long long)(nz + 2 * g) * b.sxy;
   return b;

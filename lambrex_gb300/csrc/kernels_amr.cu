@@ -23,7 +23,7 @@ namespace {
 // storage coordinates of a grown box: (sx, sy, sz) in [0, n + 2g).  Storage
 // rows (n + 4 cells) are never a multiple of a warp, so each x-y plane is
 // flattened over blocks of `threads` (grid.x) and z is grid.y (grown_launch);
-// one 32-bit division per thread recovers (sx, sy).
+// one multiplicative division per thread recovers (sx, sy).
 struct GIdx {
   int x, y, z;
 };
@@ -31,7 +31,7 @@ __device__ __forceinline__ bool grown_index(const Box3& b, GIdx& s) {
   const int SX = b.n[0] + 2 * b.g;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= SX * (b.n[1] + 2 * b.g)) return false;
-  s.y = t / SX;
+  s.y = (int)divide((uint32_t)t, b.srow);
   s.x = t - s.y * SX;
   s.z = blockIdx.y;
   return true;
