@@ -140,6 +140,18 @@ __host__ __device__ __forceinline__ double fx_to_f64(int64_t v, int ex) {  // v 
   t >>= 10;
   return d_from_words((uint32_t)(t >> 32) + ((uint32_t)(ex + (int)p) << 20), (uint32_t)t);
 }
+// the same with the conversion instruction, which the FP64 pipe executes: two of
+// a cell's fifteen keep that pipe, idle otherwise, and the integer pipe both busy
+// (192^3: 276.4 -> 273.6 us a step, rescaled 104x88x72 138.6 -> 136.3; four: 270.2
+// and 134.9, but 10x10x50 2.37 -> 2.44; all fifteen: 302 and 137.7)
+__host__ __device__ __forceinline__ double fx_to_f64_fp64(int64_t v, int ex) {
+#ifdef __CUDA_ARCH__
+  const double d = __ll2double_rn(v);
+  return __hiloint2double(__double2hiint(d) + ((ex - 1054) << 20), __double2loint(d));
+#else
+  return fx_to_f64(v, ex);
+#endif
+}
 // the same for every v (zero, negative, small)
 __host__ __device__ __forceinline__ double fx_to_f64_any(int64_t v, int ex) {
   const uint64_t m = v < 0 ? 0ull - (uint64_t)v : (uint64_t)v;
@@ -305,7 +317,8 @@ __host__ __device__ __forceinline__ bool collide_fx(double* f, const FxRates& r)
   const int xa = E - 26, xd = E - 29;
   if (low > 0) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) f[q] = fx_to_f64(g[q], q < 7 ? xa : xd);
+    for (int q = 0; q < NV; ++q)
+      f[q] = q < 2 ? fx_to_f64_fp64(g[q], xa) : fx_to_f64(g[q], q < 7 ? xa : xd);
   } else {
 #pragma unroll
     for (int q = 0; q < NV; ++q) f[q] = fx_to_f64_any(g[q], q < 7 ? xa : xd);

@@ -108,7 +108,7 @@ cudaError_t launch_copy_out(const T* f, const Box3& b, double rho0, double* out,
 // one step Q -> C(S(Q)); paired selects the paired-FP32 collision (FP64 store)
 template <typename T>
 cudaError_t launch_step_pull(const T* fin, T* fout, const Box3& b, double om_s, double om_b,
-                             double rho0, bool paired, cudaStream_t st, int block = 256);
+                             double rho0, bool paired, cudaStream_t st);
 // the same step with CalcHydroVars fused in: rho, u of the state the step
 // gathers (what launch_hydro with gather gives) are written on the way
 template <typename T>

@@ -584,10 +584,19 @@ cudaError_t launch_copy_out(const T* f, const Box3& b, double rho0, double* out,
   return cudaGetLastError();
 }
 
+// FP32: blocks of 128 threads while both stores fit in the 129 MB of L2, where
+// the step is bound by latency (80^3: 6.70 us against 6.97 in blocks of 256), of
+// 256 where it is bound by HBM (512^3: 2,313 us against 2,349)
+template <typename T>
+static int pull_threads(const Box3& b) {
+  if (sizeof(T) == 8) return kF64Threads;
+  return 2ll * NV * (long long)sizeof(T) * b.sq <= 129000000ll ? 128 : 256;
+}
+
 template <typename T, typename I>
 cudaError_t launch_step_pull_i(const T* fin, T* fout, const Box3& b, double om_s, double om_b,
-                               double rho0, bool paired, cudaStream_t st, int block) {
-  const CellLaunch rl = cell_launch(b, sizeof(T) == 8 ? kF64Threads : block);
+                               double rho0, bool paired, cudaStream_t st) {
+  const CellLaunch rl = cell_launch(b, pull_threads<T>(b));
   if constexpr (sizeof(T) == 8) {
     if (collides_in_pairs(paired, df_rates(om_s, om_b))) {
       chained(k_step_pull<double, true, I>, rl.grid, rl.block, st, fin, fout, b, om_s, om_b, 0.0,
@@ -602,20 +611,20 @@ cudaError_t launch_step_pull_i(const T* fin, T* fout, const Box3& b, double om_s
 
 template <typename T>
 cudaError_t launch_step_pull(const T* fin, T* fout, const Box3& b, double om_s, double om_b,
-                             double rho0, bool paired, cudaStream_t st, int block) {
-  // the FP64 store is instruction-bound: narrower index arithmetic pays
-  // there (1,889 -> 1,786 instructions per cell, paired); the FP32 store is
-  // bound by HBM and keeps the 64-bit form it was tuned with
-  if (sizeof(T) == 8 && (long long)NV * b.sq < (1ll << 31))
-    return launch_step_pull_i<T, int>(fin, fout, b, om_s, om_b, rho0, paired, st, block);
-  return launch_step_pull_i<T, long long>(fin, fout, b, om_s, om_b, rho0, paired, st, block);
+                             double rho0, bool paired, cudaStream_t st) {
+  // 64-bit element indices only where a store needs them: they cost a fifth of
+  // the FP32 step's instructions (80^3: 8.33 us a step against 6.97, 512^3: 2,401
+  // against 2,313) and more of the FP64 one's registers
+  if (index32(b))
+    return launch_step_pull_i<T, int>(fin, fout, b, om_s, om_b, rho0, paired, st);
+  return launch_step_pull_i<T, long long>(fin, fout, b, om_s, om_b, rho0, paired, st);
 }
 
 template <typename T, typename I>
 cudaError_t launch_step_pull_hydro_i(const T* fin, T* fout, const Box3& b, double om_s,
                                      double om_b, double rho0, bool paired, double* rho,
                                      double* u, cudaStream_t st) {
-  const CellLaunch rl = cell_launch(b, sizeof(T) == 8 ? kF64Threads : 256);
+  const CellLaunch rl = cell_launch(b, pull_threads<T>(b));
   if constexpr (sizeof(T) == 8) {
     if (collides_in_pairs(paired, df_rates(om_s, om_b))) {
       chained(k_step_pull_hydro<double, true, I>, rl.grid, rl.block, st, fin, fout, b, om_s, om_b, 0.0, df_rates(om_s, om_b), rho0, rho, u);
@@ -631,7 +640,7 @@ template <typename T>
 cudaError_t launch_step_pull_hydro(const T* fin, T* fout, const Box3& b, double om_s, double om_b,
                                    double rho0, bool paired, double* rho, double* u,
                                    cudaStream_t st) {
-  if (sizeof(T) == 8 && (long long)NV * b.sq < (1ll << 31))
+  if (index32(b))
     return launch_step_pull_hydro_i<T, int>(fin, fout, b, om_s, om_b, rho0, paired, rho, u, st);
   return launch_step_pull_hydro_i<T, long long>(fin, fout, b, om_s, om_b, rho0, paired, rho, u, st);
 }
@@ -703,7 +712,7 @@ cudaError_t launch_reduce(const T* f, const Box3& b, IBox skip, double rho0, dou
   template cudaError_t launch_step_pull_hydro<T>(const T*, T*, const Box3&, double, double,    \
                                                  double, bool, double*, double*, cudaStream_t);  \
   template cudaError_t launch_step_pull<T>(const T*, T*, const Box3&, double, double, double,  \
-                                           bool, cudaStream_t, int);                            \
+                                           bool, cudaStream_t);                                 \
   template cudaError_t launch_unstream<T>(const T*, T*, const Box3&, cudaStream_t);             \
   template cudaError_t launch_init_pulse<T>(T*, const Box3&, int, int, double, double,          \
                                             cudaStream_t);                                      \
