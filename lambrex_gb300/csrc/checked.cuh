@@ -104,6 +104,16 @@ __host__ __device__ __forceinline__ void st_pop(T* __restrict__ p, I i, const Bo
   if (idx_ok((long long)i, NV * b.sq)) p[i] = v;
 }
 
+__host__ __device__ __forceinline__ unsigned ld_plain(const unsigned* p) {
+#ifdef __CUDA_ARCH__
+  unsigned v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+#else
+  return *p;
+#endif
+}
+
 // two neighbours of a row from an even element on, in one access
 __host__ __device__ __forceinline__ void ld_plain2(const double* p, double* v) {
 #ifdef __CUDA_ARCH__

@@ -504,6 +504,19 @@ __host__ __device__ __forceinline__ bool is_rest(const double* f) {
   return d == 0;
 }
 
+// whether a cell's populations are those of a fluid at rest (fx_at_rest)
+__host__ __device__ __forceinline__ bool at_rest(const double* f) {
+  uint32_t h[NV], l[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) d_words(f[q], &h[q], &l[q]);
+  const uint32_t top = fx_top(h);
+  if (!fx_top_ok(top)) return false;
+  int64_t g[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) g[q] = fx_unit(h[q], l[q], fx_base(top >> 20));
+  return fx_at_rest(fx_sums(g));
+}
+
 // The FP64 collision of one cell: in fixed point, or with FP64 instructions
 // where the cell or the rates are outside its range.  A host build forms the
 // digits of rates that were not given here; the kernels' launchers give them.

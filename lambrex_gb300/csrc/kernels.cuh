@@ -154,7 +154,8 @@ cudaError_t launch_explode(const T* coarse, T* fine, const Coupling& c, double o
 // ghost cells stream raw, populations leaving the storage are dropped.
 template <typename T>
 cudaError_t launch_step_patch(const T* fin, T* fout, const Box3& b, IBox covered, double om_s,
-                              double om_b, double rho0, cudaStream_t st, bool paired = false);
+                              double om_b, double rho0, cudaStream_t st, bool paired = false,
+                              const unsigned* moving = nullptr);
 // coarse ring cells += volume-weighted populations that left the patch
 template <typename T>
 cudaError_t launch_coalesce(const T* fine, T* coarse, const Coupling& c, double rho0,
@@ -168,7 +169,8 @@ cudaError_t launch_restrict(const T* fine, T* coarse, const Coupling& c, cudaStr
 template <typename T>
 cudaError_t launch_explode_resc(const T* cprev, const T* cnow, T* fine, const Coupling& c,
                                 double om_s, double om_b, double rho0, double wp, double wn,
-                                cudaStream_t st, bool paired = false);
+                                cudaStream_t st, bool paired = false,
+                                const unsigned* moving = nullptr);
 // Both at once: the step of a periodic level (launch_step_periodic, refined) and
 // the explosion onto the level above it of the state the step starts from
 // (launch_explode, or with rescaled launch_explode_resc at wp = 1, wn = 0 and
@@ -176,11 +178,17 @@ cudaError_t launch_explode_resc(const T* cprev, const T* cnow, T* fine, const Co
 template <typename T>
 cudaError_t launch_step_explode(const T* fin, T* fout, const Box3& b, IBox covered, double om_s,
                                 double om_b, double rho0, T* fine, const Coupling& c, bool rescaled,
-                                double es, double eb, cudaStream_t st, bool paired = false);
+                                double es, double eb, cudaStream_t st, bool paired = false,
+                                const unsigned* moving = nullptr);
 // covered coarse cells <- mean of their children collided at the restriction rates
 template <typename T>
 cudaError_t launch_restrict_resc(const T* fine, T* coarse, const Coupling& c, double om_s,
-                                 double om_b, double rho0, cudaStream_t st, bool paired = false);
+                                 double om_b, double rho0, cudaStream_t st, bool paired = false,
+                                 unsigned* moving = nullptr);
+// FP64: sets *moving where the valid cells of a finer level are not all at rest
+// (a look at every fourth along each axis); the other launches read it, the
+// restriction onto level 0 clears it for the next step
+cudaError_t launch_moving(const double* f, const Box3& b, unsigned* moving, cudaStream_t st);
 // level creation: fine grown box <- parent coarse cell (piecewise constant)
 template <typename T>
 cudaError_t launch_fill_from_coarse(const T* coarse, T* fine, const Coupling& c,

@@ -57,8 +57,9 @@ __global__ void k_explode(const T* __restrict__ coarse, T* __restrict__ fine, Co
 // 104x88x72 took 158 us, against 162, 164 and 169 with six, five and four
 template <typename T, bool COVER, bool PAIRED, typename I>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 1) k_step_patch(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov,
-                             T om_s, T om_b, T rho0, DfRates r) {
+                             T om_s, T om_b, T rho0, DfRates r, const unsigned* moving) {
   chain_begin();
+  if (sizeof(T) == 8 && moving && ld_plain(moving)) r.fx.quiet = 0;
   GIdx s;
   if (!grown_index(b, s)) return;
   cell_step_patch<T, COVER, PAIRED, I>(fin, fout, b, cov, s.x, s.y, s.z, om_s, om_b, rho0, r);
@@ -87,8 +88,9 @@ __global__ void k_restrict(const T* __restrict__ fine, T* __restrict__ coarse, C
 template <typename T, bool PAIRED, typename I>
 __global__ void k_explode_resc(const T* __restrict__ cprev, const T* __restrict__ cnow,
                                T* __restrict__ fine, Coupling c, T om_s, T om_b, T rho0, T wp, T wn,
-                               DfRates r) {
+                               DfRates r, const unsigned* moving) {
   chain_begin();
+  if (sizeof(T) == 8 && moving && ld_plain(moving)) r.fx.quiet = 0;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if constexpr (sizeof(T) == 8) {
     Ring g;
@@ -110,8 +112,9 @@ template <typename T, bool COVER, bool PAIRED, typename I, bool RESC>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 1)
     k_step_explode(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov, T om_s, T om_b,
                    T rho0, DfRates r, T* __restrict__ fine, Coupling c, T es, T eb, DfRates re,
-                   unsigned first) {
+                   unsigned first, const unsigned* moving) {
   chain_begin();
+  if (RESC && sizeof(T) == 8 && moving && ld_plain(moving)) r.fx.quiet = re.fx.quiet = 0;
   if (blockIdx.x < first) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     int s[3];
@@ -127,10 +130,34 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 1)
   cell_step_periodic<T, COVER, PAIRED, I>(fin, fout, b, cov, x, y, z, om_s, om_b, rho0, r);
 }
 
+// Whether anything moves on a level, of the cells at every fourth place: sets
+// *moving, which the last kernel of the step before cleared.  Only the speed of a
+// refined FP64 step depends on it.  While a patch is at rest, its cells and the
+// coarse ones take the FP64 instructions (collide_f64); once a wave is in it,
+// what is rounding alone no longer shows, and the fluid at rest elsewhere is
+// collided in fixed point like the rest (a pulse's first 20 steps in 104x88x72,
+// rescaled: 5.5 to 8.3 ms without the look, 3.4 to 4.4 with it, 3.2 and 3.3
+// later on).
+__global__ void __launch_bounds__(128) k_moving(const double* __restrict__ f, Box3 b, unsigned* moving) {
+  chain_begin();
+  const int nx = (b.n[0] + 3) / 4, ny = (b.n[1] + 3) / 4, nz = (b.n[2] + 3) / 4;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  bool moves = false;
+  if (t < nx * ny * nz) {
+    const long long c = b.at(4 * (t % nx), 4 * (t / nx % ny), 4 * (t / (nx * ny)));
+    double p[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) p[q] = ld_pop(f, q * b.sq + c, b);
+    moves = !at_rest(p);
+  }
+  if (__syncthreads_or(moves) && threadIdx.x == 0) *moving = 1;
+}
+
 template <typename T, bool PAIRED, typename I>
 __global__ void k_restrict_resc(const T* __restrict__ fine, T* __restrict__ coarse, Coupling c,
-                                T om_s, T om_b, T rho0, DfRates r) {
+                                T om_s, T om_b, T rho0, DfRates r, unsigned* moving) {
   chain_begin();
+  if (moving && blockIdx.x == 0 && threadIdx.x == 0) *moving = 0;  // until the next look
   const int ex = c.fb.n[0] / 2, ey = c.fb.n[1] / 2, ez = c.fb.n[2] / 2;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)ex * ey * ez) return;
@@ -241,7 +268,8 @@ cudaError_t launch_explode(const T* coarse, T* fine, const Coupling& c, double o
 
 template <typename T>
 cudaError_t launch_step_patch(const T* fin, T* fout, const Box3& b, IBox covered, double om_s,
-                              double om_b, double rho0, cudaStream_t st, bool paired) {
+                              double om_b, double rho0, cudaStream_t st, bool paired,
+                              const unsigned* moving) {
   const bool cov = covered.hi[0] >= covered.lo[0] && covered.hi[1] >= covered.lo[1] &&
                    covered.hi[2] >= covered.lo[2];
   const CellLaunch rl = grown_launch(b, 128);
@@ -251,13 +279,13 @@ cudaError_t launch_step_patch(const T* fin, T* fout, const Box3& b, IBox covered
     constexpr bool P = sizeof(T) == 8;
     const T ts = (T)om_s, tb = (T)om_b, t0 = (T)rho0;
     if (P && paired && cov)
-      chained(k_step_patch<T, true, P, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r);
+      chained(k_step_patch<T, true, P, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r, moving);
     else if (P && paired)
-      chained(k_step_patch<T, false, P, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r);
+      chained(k_step_patch<T, false, P, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r, moving);
     else if (cov)
-      chained(k_step_patch<T, true, false, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r);
+      chained(k_step_patch<T, true, false, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r, moving);
     else
-      chained(k_step_patch<T, false, false, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r);
+      chained(k_step_patch<T, false, false, I>, rl.grid, rl.block, st, fin, fout, b, covered, ts, tb, t0, r, moving);
   });
   return cudaGetLastError();
 }
@@ -282,7 +310,7 @@ cudaError_t launch_restrict(const T* fine, T* coarse, const Coupling& c, cudaStr
 template <typename T>
 cudaError_t launch_explode_resc(const T* cprev, const T* cnow, T* fine, const Coupling& c,
                                 double om_s, double om_b, double rho0, double wp, double wn,
-                                cudaStream_t st, bool paired) {
+                                cudaStream_t st, bool paired, const unsigned* moving) {
   const int threads = sizeof(T) == 8 ? kRingThreads : 128;
   const unsigned grid =
       blocks_for(sizeof(T) == 8 ? ring_cells_of(c) : ghost_cells_of(c.fb), threads);
@@ -290,10 +318,10 @@ cudaError_t launch_explode_resc(const T* cprev, const T* cnow, T* fine, const Co
   with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
     using I = decltype(i);
     if (sizeof(T) == 8 && paired)
-      chained(k_explode_resc<T, sizeof(T) == 8, I>, grid, threads, st, cprev, cnow, fine, c, (T)om_s, (T)om_b, (T)rho0, (T)wp, (T)wn, r);
+      chained(k_explode_resc<T, sizeof(T) == 8, I>, grid, threads, st, cprev, cnow, fine, c, (T)om_s, (T)om_b, (T)rho0, (T)wp, (T)wn, r, moving);
     else
       chained(k_explode_resc<T, false, I>, grid, threads, st, cprev, cnow, fine, c, (T)om_s, (T)om_b,
-                                                        (T)rho0, (T)wp, (T)wn, r);
+                                                        (T)rho0, (T)wp, (T)wn, r, moving);
   });
   return cudaGetLastError();
 }
@@ -301,44 +329,52 @@ cudaError_t launch_explode_resc(const T* cprev, const T* cnow, T* fine, const Co
 template <typename T, bool COVER, bool PAIRED, bool RESC>
 static void step_explode(const T* fin, T* fout, const Box3& b, const IBox& cov, double om_s,
                          double om_b, double rho0, T* fine, const Coupling& c, double es, double eb,
-                         cudaStream_t st) {
+                         cudaStream_t st, const unsigned* moving) {
   const unsigned first = blocks_for(ghost_cells_of(c.fb), 128);
   const unsigned cells = blocks_for((long long)b.n[0] * b.n[1] * b.n[2], 128);
   with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
     chained(k_step_explode<T, COVER, PAIRED, decltype(i), RESC>, first + cells, 128, st, fin, fout, b,
             cov, (T)om_s, (T)om_b, (T)rho0, quiet(rates_of<T>(om_s, om_b)), fine, c, (T)es, (T)eb,
-            quiet(rates_of<T>(es, eb)), first);
+            quiet(rates_of<T>(es, eb)), first, moving);
   });
 }
 template <typename T>
 cudaError_t launch_step_explode(const T* fin, T* fout, const Box3& b, IBox covered, double om_s,
                                 double om_b, double rho0, T* fine, const Coupling& c, bool rescaled,
-                                double es, double eb, cudaStream_t st, bool paired) {
+                                double es, double eb, cudaStream_t st, bool paired,
+                                const unsigned* moving) {
   constexpr bool P = sizeof(T) == 8;
   if (rescaled && P && paired)
-    step_explode<T, false, P, true>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st);
+    step_explode<T, false, P, true>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st, moving);
   else if (rescaled)
-    step_explode<T, false, false, true>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st);
+    step_explode<T, false, false, true>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st, moving);
   else if (P && paired)
-    step_explode<T, true, P, false>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st);
+    step_explode<T, true, P, false>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st, moving);
   else
-    step_explode<T, true, false, false>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st);
+    step_explode<T, true, false, false>(fin, fout, b, covered, om_s, om_b, rho0, fine, c, es, eb, st, moving);
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_restrict_resc(const T* fine, T* coarse, const Coupling& c, double om_s,
-                                 double om_b, double rho0, cudaStream_t st, bool paired) {
+                                 double om_b, double rho0, cudaStream_t st, bool paired,
+                                 unsigned* moving) {
   const long long n = (long long)(c.fb.n[0] / 2) * (c.fb.n[1] / 2) * (c.fb.n[2] / 2);
   const DfRates r = quiet(rates_of<T>(om_s, om_b));
   with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
     using I = decltype(i);
     if (sizeof(T) == 8 && paired)
-      chained(k_restrict_resc<T, sizeof(T) == 8, I>, blocks_for(n, 128), 128, st, fine, coarse, c, (T)om_s, (T)om_b, (T)rho0, r);
+      chained(k_restrict_resc<T, sizeof(T) == 8, I>, blocks_for(n, 128), 128, st, fine, coarse, c, (T)om_s, (T)om_b, (T)rho0, r, moving);
     else
       chained(k_restrict_resc<T, false, I>, blocks_for(n, 128), 128, st, fine, coarse, c, (T)om_s,
-                                                                       (T)om_b, (T)rho0, r);
+                                                                       (T)om_b, (T)rho0, r, moving);
   });
+  return cudaGetLastError();
+}
+
+cudaError_t launch_moving(const double* f, const Box3& b, unsigned* moving, cudaStream_t st) {
+  const long long n = (long long)((b.n[0] + 3) / 4) * ((b.n[1] + 3) / 4) * ((b.n[2] + 3) / 4);
+  chained(k_moving, blocks_for(n, 128), 128, st, f, b, moving);
   return cudaGetLastError();
 }
 
@@ -353,18 +389,18 @@ cudaError_t launch_fill_from_coarse(const T* coarse, T* fine, const Coupling& c,
   template cudaError_t launch_explode<T>(const T*, T*, const Coupling&, double, double, double, \
                                          cudaStream_t, bool);                                  \
   template cudaError_t launch_step_patch<T>(const T*, T*, const Box3&, IBox, double, double,   \
-                                            double, cudaStream_t, bool);                       \
+                                            double, cudaStream_t, bool, const unsigned*);      \
   template cudaError_t launch_step_explode<T>(const T*, T*, const Box3&, IBox, double, double, \
                                               double, T*, const Coupling&, bool, double,       \
-                                              double, cudaStream_t, bool);                     \
+                                              double, cudaStream_t, bool, const unsigned*);    \
   template cudaError_t launch_coalesce<T>(const T*, T*, const Coupling&, double, cudaStream_t); \
   template cudaError_t launch_restrict<T>(const T*, T*, const Coupling&, cudaStream_t);        \
   template cudaError_t launch_fill_from_coarse<T>(const T*, T*, const Coupling&, cudaStream_t); \
   template cudaError_t launch_explode_resc<T>(const T*, const T*, T*, const Coupling&, double,   \
                                               double, double, double, double, cudaStream_t,     \
-                                              bool);                                            \
+                                              bool, const unsigned*);                           \
   template cudaError_t launch_restrict_resc<T>(const T*, T*, const Coupling&, double, double,   \
-                                               double, cudaStream_t, bool);
+                                               double, cudaStream_t, bool, unsigned*);
 LBX_INST(double)
 LBX_INST(float)
 #undef LBX_INST

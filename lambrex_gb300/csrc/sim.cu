@@ -145,6 +145,7 @@ struct lbx_sim {
   double* d_partials = nullptr;
   double* d_out4 = nullptr;
   double* h_out4 = nullptr;
+  unsigned* d_moving = nullptr;  // FP64, rescaled: whether a finer level moves (launch_moving)
   long long launches = 0;  // kernels issued by lbx_iterate (counted per launch)
   // replayable macro steps (lbx_iterate): a short and a long graph for each of
   // the two store roles, since a step taken ahead by CalcHydroVars swaps them
@@ -526,6 +527,13 @@ int r_advance(lbx_sim* s, int L) {
   Level& l = s->lev[L];
   const bool paired = s->precision == LBX_F64_PAIRED;
   const bool both = L == 0 && s->finest > 0;  // the step and the first explosion at once
+  unsigned* moving = sizeof(T) == 8 && !paired && s->finest > 0 ? s->d_moving : nullptr;
+  if (L == 0 && moving)
+    for (int k = 1; k <= s->finest; ++k) {
+      const Level& f = s->lev[k];
+      CK(lbx::launch_moving(P<double>(f.buf[f.now]), f.box, moving, s->stream));
+      ++s->launches;
+    }
   ++s->launches;
   if (both) {
     Level& f = s->lev[1];
@@ -533,7 +541,7 @@ int r_advance(lbx_sim* s, int L) {
     CK(lbx::launch_step_explode<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box,
                                    lbx::empty_ibox(), omega(l.tau_s), omega(l.tau_b), s->rho0,
                                    P<T>(f.buf[f.now]), coupling(s, 1), true, R.es, R.eb, s->stream,
-                                   paired));
+                                   paired, moving));
   } else if (L == 0) {
     CK(lbx::launch_step_periodic<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box,
                                     lbx::empty_ibox(), omega(l.tau_s), omega(l.tau_b), s->rho0,
@@ -541,7 +549,7 @@ int r_advance(lbx_sim* s, int L) {
   } else {
     CK(lbx::launch_step_patch<T>(P<T>(l.buf[l.now]), P<T>(l.buf[l.next]), l.box,
                                  lbx::empty_ibox(), omega(l.tau_s), omega(l.tau_b), s->rho0,
-                                 s->stream, paired));
+                                 s->stream, paired, moving));
   }
   std::swap(l.now, l.next);
   if (L < s->finest) {
@@ -552,13 +560,13 @@ int r_advance(lbx_sim* s, int L) {
       if (k > 0 || !both) {
         CK(lbx::launch_explode_resc<T>(P<T>(l.buf[l.next]), P<T>(l.buf[l.now]), P<T>(f.buf[f.now]),
                                        cp, R.es, R.eb, s->rho0, 1.0 - 0.5 * k, 0.5 * k, s->stream,
-                                       paired));
+                                       paired, moving));
         ++s->launches;
       }
       RET(r_advance<T>(s, L + 1));
     }
     CK(lbx::launch_restrict_resc<T>(P<T>(f.buf[f.now]), P<T>(l.buf[l.now]), cp, R.rs, R.rb,
-                                    s->rho0, s->stream, paired));
+                                    s->rho0, s->stream, paired, L == 0 ? moving : nullptr));
     ++s->launches;
   }
   l.time += l.dt;
@@ -972,6 +980,10 @@ int lbx_create(int nx, int ny, int nz, int max_level, const int* periodicity, do
   if (e == cudaSuccess) e = cudaMalloc(&s->d_partials, lbx::reduce_partials_doubles() * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&s->d_out4, 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMallocHost(&s->h_out4, 4 * sizeof(double));
+  if (e == cudaSuccess && amr_mode == LBX_AMR_RESCALED && max_level > 0 && precision == LBX_F64) {
+    e = cudaMalloc(&s->d_moving, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->d_moving, 0, sizeof(unsigned), s->stream);
+  }
   if (e != cudaSuccess) {
     lbx::note_error("lbx_create", e);
     lbx_destroy(s);
@@ -991,6 +1003,7 @@ int lbx_destroy(lbx_sim* s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->d_partials) cudaFree(s->d_partials);
   if (s->d_out4) cudaFree(s->d_out4);
+  if (s->d_moving) cudaFree(s->d_moving);
   if (s->h_out4) cudaFreeHost(s->h_out4);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
