@@ -25,10 +25,13 @@ __device__ __forceinline__ void stage(D& to, const D& from) {
 // One kernel per box kind (every launch covers boxes of one kind), so each
 // instantiation carries only its own cell body.  The tile's box descriptor
 // is staged in shared memory: the cell code reads its geometry from there
-// instead of holding it in registers, which keeps occupancy high.  (FP64 held
-// to 64 registers spills and is no faster: 109.2 us a step against 107.9.)
-template <typename T, int KIND, int CPT>
-__global__ void __launch_bounds__(512) k_b_step(const BBox* __restrict__ boxes,
+// instead of holding it in registers, which keeps occupancy high.  In blocks of
+// 128 (MAXT) the FP64 kernels are held to 72 registers, seven blocks to an SM: 24
+// boxes of 9.9 M cells 463 us a step, against 483 at 98 to 116 registers, 469 with
+// five or six blocks and 480 with eight (spills); six served FP64 requests 13.5 ms
+// of steps against 14.0.
+template <typename T, int KIND, int CPT, int MAXT>
+__global__ void __launch_bounds__(MAXT, sizeof(T) == 8 && MAXT == 128 ? 7 : 0) k_b_step(const BBox* __restrict__ boxes,
                                                 const BTile* __restrict__ tiles, int ntiles,
                                                 int flip) {
   __shared__ BBox sbox;
@@ -71,22 +74,24 @@ __global__ void __launch_bounds__(512) k_b_step(const BBox* __restrict__ boxes,
 }
 
 template <typename T, int KIND>
+using StepKernel = void (*)(const BBox*, const BTile*, int, int);
+template <typename T, int KIND>
+StepKernel<T, KIND> step_kernel(int block, int cpt) {
+  if (block <= 128) return cpt >= 2 ? k_b_step<T, KIND, 2, 128> : k_b_step<T, KIND, 1, 128>;
+  return cpt >= 2 ? k_b_step<T, KIND, 2, 512> : k_b_step<T, KIND, 1, 512>;
+}
+
+template <typename T, int KIND>
 int occupancy(int block, int cpt) {
   int n = 0;
-  if (cpt >= 2)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_b_step<T, KIND, 2>, block, 0);
-  else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_b_step<T, KIND, 1>, block, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, step_kernel<T, KIND>(block, cpt), block, 0);
   return n;
 }
 
 template <typename T, int KIND>
 void launch_kind(const BBox* boxes, const BTile* tiles, int ntiles, int flip, int grid, int block,
                  int cpt, cudaStream_t st) {
-  if (cpt >= 2)
-    k_b_step<T, KIND, 2><<<grid, block, 0, st>>>(boxes, tiles, ntiles, flip);
-  else
-    k_b_step<T, KIND, 1><<<grid, block, 0, st>>>(boxes, tiles, ntiles, flip);
+  step_kernel<T, KIND>(block, cpt)<<<grid, block, 0, st>>>(boxes, tiles, ntiles, flip);
 }
 
 template <typename T>

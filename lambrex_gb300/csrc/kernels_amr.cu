@@ -54,10 +54,13 @@ __global__ void k_explode(const T* __restrict__ coarse, T* __restrict__ fine, Co
 }
 
 // FP64: eight blocks an SM (64 registers): a rescaled two-level coarse step of
-// 104x88x72 took 158 us, against 162, 164 and 169 with six, five and four
+// 104x88x72 took 158 us, against 162, 164 and 169 with six, five and four.  FP32:
+// the compiler's own choice, 40 registers (conservative 64^3 21.4 us against 22.2
+// at the 48 that it takes when told of one block; 128^3 154.8 against 154.0)
 template <typename T, bool COVER, bool PAIRED, typename I>
-__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 1) k_step_patch(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov,
-                             T om_s, T om_b, T rho0, DfRates r, const unsigned* moving) {
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 0)
+    k_step_patch(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov, T om_s, T om_b,
+                 T rho0, DfRates r, const unsigned* moving) {
   chain_begin();
   if (sizeof(T) == 8 && moving && ld_plain(moving)) r.fx.quiet = 0;
   GIdx s;
@@ -109,7 +112,7 @@ __global__ void k_explode_resc(const T* __restrict__ cprev, const T* __restrict_
 // the warp slots); as the first blocks of the step's launch it is done before
 // the step is.  64^3 conservative FP32: 25.4 -> 22.9 us a coarse step.
 template <typename T, bool COVER, bool PAIRED, typename I, bool RESC>
-__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 1)
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : RESC ? 1 : 0)
     k_step_explode(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov, T om_s, T om_b,
                    T rho0, DfRates r, T* __restrict__ fine, Coupling c, T es, T eb, DfRates re,
                    unsigned first, const unsigned* moving) {
