@@ -139,23 +139,27 @@ __host__ __device__ __forceinline__ void f_cell_sum_from_fine(const double* __re
                                                              int rz) {
   const int cgx = c.flo[0] / 2 + rx - 1, cgy = c.flo[1] / 2 + ry - 1, cgz = c.flo[2] / 2 + rz - 1;
   const int fx0 = 2 * cgx - c.flo[0], fy0 = 2 * cgy - c.flo[1], fz0 = 2 * cgz - c.flo[2];
+  // the means first, with all loads in flight, then the images of the cell
+  // (41.6 us a launch with the 27 images looked for once per population, 64^3)
+  double avg[NV];
+#pragma unroll
   for (int q = 0; q < NV; ++q) {
     double s = 0.0;
-    for (int kr = 0; kr < 2; ++kr)
-      for (int jr = 0; jr < 2; ++jr)
-        for (int ir = 0; ir < 2; ++ir)
-          s += ld_pop_ro(fnow, q * c.fb.sq + c.fb.at(fx0 + ir, fy0 + jr, fz0 + kr), c.fb);
-    const double avg = 0.125 * s;
-    for (int sz = -1; sz <= 1; ++sz)
-      for (int sy = -1; sy <= 1; ++sy)
-        for (int sx = -1; sx <= 1; ++sx) {
-          const int a = cgx + sx * c.cdom[0] - c.clo[0];
-          const int bb = cgy + sy * c.cdom[1] - c.clo[1];
-          const int e = cgz + sz * c.cdom[2] - c.clo[2];
-          if (!in_valid(c.cb, a, bb, e)) continue;
-          f_add_pop(cnext, q * c.cb.sq + c.cb.at(a, bb, e), c.cb, avg);
-        }
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+      s += ld_pop_ro(fnow, q * c.fb.sq + c.fb.at(fx0 + (m & 1), fy0 + ((m >> 1) & 1), fz0 + (m >> 2)), c.fb);
+    avg[q] = 0.125 * s;
   }
+  for (int sz = -1; sz <= 1; ++sz)
+    for (int sy = -1; sy <= 1; ++sy)
+      for (int sx = -1; sx <= 1; ++sx) {
+        const int a = cgx + sx * c.cdom[0] - c.clo[0];
+        const int bb = cgy + sy * c.cdom[1] - c.clo[1];
+        const int e = cgz + sz * c.cdom[2] - c.clo[2];
+        if (!in_valid(c.cb, a, bb, e)) continue;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) f_add_pop(cnext, q * c.cb.sq + c.cb.at(a, bb, e), c.cb, avg[q]);
+      }
 }
 
 }  // namespace lbx
