@@ -662,22 +662,22 @@ bool graph_matches(lbx_sim* s, int left) {
   }
   return best > 0;
 }
-// Launches of a long graph: between the kernels of one graph there is no gap
-// (chained, launch.cuh), between two replays there is, so a run of
-// kGraphLongRun launches or more is replayed in long graphs; what is left, and
-// shorter runs, in graphs of one period.
-constexpr int kGraphLong = 32, kGraphLongRun = 2 * kGraphLong;
+// Steps of the graph that `left` steps are to be taken in, 0: launch them
+// directly.  Between the kernels of one graph there is no gap (chained,
+// launch.cuh), between two replays there is: graphs of 32 launches, and of 8 for
+// what is left (10x10x50 FP64, 60 steps: 4.1 us a step in graphs of two).
 int graph_steps(const lbx_sim* s, int left) {
   const int per_step = std::max(1, s->finest == 0 ? 1 : 4 << (s->finest - 1));  // launches, about
-  return (long long)left * per_step >= kGraphLongRun ? std::max(2, kGraphLong / per_step) : 1;
+  for (const int launches : {32, 8})
+    if ((long long)left * per_step >= launches) return std::max(1, launches / per_step);
+  return 0;
 }
-
 // Capture macro steps from the simulation's own launches until every level's
 // buffers are back in their roles, then run the captured steps once (the
 // host-side bookkeeping already advanced while capturing).  Keeps the graph
 // for replay when the roles did return.
 int capture_graph(lbx_sim* s, int* left) {
-  const int atleast = std::min(graph_steps(s, *left), *left);
+  const int atleast = std::min(std::max(1, graph_steps(s, *left)), *left);
   s->gcur = 0;  // replaces the one not used for longest
   for (int i = 1; i < 4; ++i)
     if (s->graphs[i].used < s->graphs[s->gcur].used) s->gcur = i;
@@ -1199,7 +1199,9 @@ int lbx_iterate(lbx_sim* s, int nsteps) {
   }
   if (left >= kGraphMinSteps) {
     while (left >= kGraphMinSteps) {
-      if (!graph_matches(s, left) || s->graphs[s->gcur].period < graph_steps(s, left)) {
+      const int steps = graph_steps(s, left);
+      if (steps == 0) break;
+      if (!graph_matches(s, left) || s->graphs[s->gcur].period < steps) {
         RET(capture_graph(s, &left));  // runs what it captures
         if (!s->graphs[s->gcur].exec) break;
         continue;
