@@ -1201,7 +1201,18 @@ int lbx_iterate(lbx_sim* s, int nsteps) {
     while (left >= kGraphMinSteps) {
       const int steps = graph_steps(s, left);
       if (steps == 0) break;
-      if (!graph_matches(s, left) || s->graphs[s->gcur].period < steps) {
+      const bool have = graph_matches(s, left);
+      if (!have || s->graphs[s->gcur].period < steps) {
+        // inside a capture of the caller's no new graph can be made: the shorter
+        // one at hand, or the steps themselves, become nodes of the caller's
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(s->stream, &cs));
+        if (cs != cudaStreamCaptureStatusNone) {
+          if (!have) break;
+          for (const int period = s->graphs[s->gcur].period; left >= period; left -= period)
+            RET(replay_graph(s));
+          continue;
+        }
         RET(capture_graph(s, &left));  // runs what it captures
         if (!s->graphs[s->gcur].exec) break;
         continue;
