@@ -9,8 +9,8 @@ equilibrium.  Synthetic data (the reference publishes no dataset).
 One bench "step" is one lattice time step over the whole domain.
   value : FP32 shifted-population store, state resident in HBM, CUDA events
           on the simulation's stream around K steps -> MLUPS.
-  fp64, fp64_paired : the FP64 drop-in on the same input (native FP64
-          arithmetic; FP64 store with the paired-FP32 collision).
+  fp64, fp64_paired : the FP64 drop-in on the same input (both stores
+          collide in 64-bit fixed point).
   fp32_vs_fp64 : rho / u error of the FP32 run against the FP64 run after
           500 steps (the roofline configuration's stated step count).
   e2e   : the same K steps through the public AmrSim API from host vectors:
@@ -874,11 +874,11 @@ def main():
                  "ms_per_step": res["f64"]["ms"] / K,
                  "roofline": hbm_roofline(BYTES_F64, cells * K, t64,
                                           traffic=traffic_from_profiles("step_pull_f64"),
-                                          note="bound by the FP64 pipe (85 % busy), not HBM"),
+                                          note="collision in 64-bit fixed point on the integer pipe"),
                  "clocks": r["clocks"]["f64"]},
         "fp64_paired": {"value": aggregate_mlups(world, cells, K, t64p), "unit": UNIT,
                         "ms_per_step": res["f64p"]["ms"] / K,
-                        "what": "FP64 store, collision in paired-FP32 arithmetic",
+                        "what": "FP64 store, LBX_F64_PAIRED",
                         "roofline": hbm_roofline(BYTES_F64, cells * K, t64p,
                                                  traffic=traffic_from_profiles("step_pull_f64_paired")),
                         "vs_fp64": r["err_p"], "clocks": r["clocks"]["f64p"]},

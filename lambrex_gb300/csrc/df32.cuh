@@ -1,8 +1,10 @@
 // df32.cuh -- FP64-store collision carried in pairs of FP32 values.
 //
 // GB300 issues about 1.9 FP64 instructions per clock per SM against 128 FP32
-// ones, so the native FP64 step is bound by the FP64 pipe at about a sixth of
-// the HBM roofline.  This variant keeps the FP64 store and the reference's
+// ones, so a step of FP64 instructions runs at about a sixth of the HBM
+// roofline.  The FP64 stores are collided in 64-bit fixed point instead
+// (fx64.cuh); this variant serves the paired store at rates that the fixed point
+// cannot hold and in refined runs.  It keeps the FP64 store and the reference's
 // algorithm but does the arithmetic of the collision on the FP32 pipe: each
 // population is split (with integer operations, no FP64 instruction) into an
 // unevaluated sum hi + lo of two floats (48-bit significand), the collision of

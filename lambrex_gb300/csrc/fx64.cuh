@@ -21,8 +21,9 @@
 // 1.1e-16.
 //
 // Measured on one GB300: 192^3, 40 steps with the readout, 13.2 ms against
-// 63.1 ms with FP64 instructions; 10x10x50, 100 steps, 0.56 ms against 1.19 ms
-// (there a warp's FP64 instructions alone took 1.1 us of each step).
+// 63.1 ms with FP64 instructions (12.3 since the step is held to 64 registers);
+// 10x10x50, 100 steps, 0.56 ms against 1.19 ms (0.28 in chained launches; a
+// warp's FP64 instructions alone took 1.1 us of each step).
 //
 // Range.  Cells that the fixed point cannot hold (a negative, infinite or NaN
 // population, a largest one outside 2^-950..2^1000, |u_a| above 1/4, density

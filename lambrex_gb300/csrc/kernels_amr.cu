@@ -55,8 +55,8 @@ __global__ void k_explode(const T* __restrict__ coarse, T* __restrict__ fine, Co
 
 // FP64: eight blocks an SM (64 registers): a rescaled two-level coarse step of
 // 104x88x72 took 158 us, against 162, 164 and 169 with six, five and four.  FP32:
-// the compiler's own choice, 40 registers (conservative 64^3 21.4 us against 22.2
-// at the 48 that it takes when told of one block; 128^3 154.8 against 154.0)
+// the compiler's own choice, 48 registers (conservative 64^3 21.4 us against 22.2
+// at the 56 that it takes when told of one block; 128^3 154.8 against 154.0)
 template <typename T, bool COVER, bool PAIRED, typename I>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : 0)
     k_step_patch(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov, T om_s, T om_b,
