@@ -515,30 +515,44 @@ __host__ __device__ __forceinline__ void cell_explode_resc(const T* __restrict__
   for (int q = 0; q < NV; ++q) st_pop(fine, (I)q * fsq + fc, c.fb, a[q]);
 }
 
+// storage index of covered coarse cell (rx,ry,rz) of coarsen(patch)
+template <typename I>
+__host__ __device__ __forceinline__ I covered_index(const Coupling& c, int rx, int ry, int rz) {
+  int P[3] = {c.flo[0] / 2 + rx, c.flo[1] / 2 + ry, c.flo[2] / 2 + rz};
+  if (c.cper)
+    for (int d = 0; d < 3; ++d) P[d] = wrapi(P[d], c.cdom[d]);
+  return sidx_i<I>(c.cb, P[0] - c.clo[0] + c.cb.g, P[1] - c.clo[1] + c.cb.g,
+                   P[2] - c.clo[2] + c.cb.g);
+}
+// population q of its eight children
+template <typename T, typename I>
+__host__ __device__ __forceinline__ void ld_covered(const T* __restrict__ fine, const Coupling& c,
+                                                    int rx, int ry, int rz, int q, T* v) {
+  const int g = c.fb.g;
+#pragma unroll
+  for (int m = 0; m < 8; m += 2)
+    ld_pop2(fine,
+            (I)q * (I)c.fb.sq +
+                sidx_i<I>(c.fb, 2 * rx + g, 2 * ry + ((m >> 1) & 1) + g, 2 * rz + (m >> 2) + g),
+            c.fb, v + m);
+}
+
 // covered coarse cell (rx,ry,rz) of coarsen(patch) <- the mean of its
-// children collided at the restriction rates (the inverse rescaling)
+// children collided at the restriction rates (the inverse rescaling).  The
+// children of the next population are loaded before the mean of one is taken,
+// whose branches loads do not pass.
 template <typename T, bool PAIRED = false, typename I = long long>
 __host__ __device__ __forceinline__ void cell_restrict_resc(const T* __restrict__ fine,
                                                    T* __restrict__ coarse, const Coupling& c,
                                                    int rx, int ry, int rz, T om_s, T om_b,
                                                    T rho0, const DfRates& r = DfRates{}) {
-  int P[3] = {c.flo[0] / 2 + rx, c.flo[1] / 2 + ry, c.flo[2] / 2 + rz};
-  if (c.cper)
-    for (int d = 0; d < 3; ++d) P[d] = wrapi(P[d], c.cdom[d]);
-  const I cc = sidx_i<I>(c.cb, P[0] - c.clo[0] + c.cb.g, P[1] - c.clo[1] + c.cb.g,
-                         P[2] - c.clo[2] + c.cb.g);
-  const I csq = (I)c.cb.sq, fsq = (I)c.fb.sq;
-  const int g = c.fb.g;
-  T f[NV];
+  const I cc = covered_index<I>(c, rx, ry, rz), csq = (I)c.cb.sq;
+  T f[NV], v[2][8];
+  ld_covered<T, I>(fine, c, rx, ry, rz, 0, v[0]);
 #pragma unroll
   for (int q = 0; q < NV; ++q) {
-    T v[8];
-#pragma unroll
-    for (int m = 0; m < 8; m += 2)
-      ld_pop2(fine,
-              (I)q * fsq + sidx_i<I>(c.fb, 2 * rx + g, 2 * ry + ((m >> 1) & 1) + g, 2 * rz + (m >> 2) + g),
-              c.fb, v + m);
-    f[q] = mean8(v);
+    if (q + 1 < NV) ld_covered<T, I>(fine, c, rx, ry, rz, q + 1, v[(q + 1) & 1]);
+    f[q] = mean8(v[q & 1]);
   }
   collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);
 #pragma unroll
@@ -658,28 +672,20 @@ __host__ __device__ __forceinline__ void cell_coalesce_q(const T* __restrict__ f
          (ld_pop_rw(coarse, i, c.cb) + T(0.125) * T(k) * T(W(q)) * rho0) + T(0.125) * sum);
 }
 
-// covered coarse cell (rx,ry,rz) of coarsen(patch) <- mean of its children
+// population q of covered coarse cell (rx,ry,rz) of coarsen(patch) <- the mean
+// of its children
+template <typename T, typename I = long long>
+__host__ __device__ __forceinline__ void cell_restrict_q(const T* __restrict__ fine,
+                                                T* __restrict__ coarse, const Coupling& c, int rx,
+                                                int ry, int rz, int q) {
+  T v[8];
+  ld_covered<T, I>(fine, c, rx, ry, rz, q, v);
+  st_pop(coarse, (I)q * (I)c.cb.sq + covered_index<I>(c, rx, ry, rz), c.cb, mean8(v));
+}
 template <typename T, typename I = long long>
 __host__ __device__ __forceinline__ void cell_restrict(const T* __restrict__ fine, T* __restrict__ coarse,
                                               const Coupling& c, int rx, int ry, int rz) {
-  int P[3] = {c.flo[0] / 2 + rx, c.flo[1] / 2 + ry, c.flo[2] / 2 + rz};
-  if (c.cper)
-    for (int d = 0; d < 3; ++d) P[d] = wrapi(P[d], c.cdom[d]);
-  const I cc = sidx_i<I>(c.cb, P[0] - c.clo[0] + c.cb.g, P[1] - c.clo[1] + c.cb.g,
-                         P[2] - c.clo[2] + c.cb.g);
-  const I csq = (I)c.cb.sq, fsq = (I)c.fb.sq;
-  const int g = c.fb.g;
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    T v[8];
-#pragma unroll
-    for (int m = 0; m < 8; ++m)
-      v[m] = ld_pop_ro(fine,
-                    (I)q * fsq + sidx_i<I>(c.fb, 2 * rx + (m & 1) + g, 2 * ry + ((m >> 1) & 1) + g,
-                                           2 * rz + (m >> 2) + g),
-                    c.fb);
-    st_pop(coarse, (I)q * csq + cc, c.cb, mean8(v));
-  }
+  for (int q = 0; q < NV; ++q) cell_restrict_q<T, I>(fine, coarse, c, rx, ry, rz, q);
 }
 
 }  // namespace lbx

@@ -79,13 +79,16 @@ __global__ void k_coalesce(const T* __restrict__ fine, T* __restrict__ coarse, C
   cell_coalesce_q<T, I>(fine, coarse, c, r[0], r[1], r[2], q, rho0);
 }
 
-template <typename T>
+// one thread a covered cell and population, neighbouring cells of one per warp
+// (a thread a cell took 13.5 to 14.2 us whatever the size, its loads in turn;
+// 9,216 / 32,768 / 49,152 covered cells, FP32, out of L2: 4.3 / 6.6 / 8.0)
+template <typename T, typename I>
 __global__ void k_restrict(const T* __restrict__ fine, T* __restrict__ coarse, Coupling c) {
   const int ex = c.fb.n[0] / 2, ey = c.fb.n[1] / 2, ez = c.fb.n[2] / 2;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)ex * ey * ez) return;
   const int rx = (int)(t % ex), ry = (int)((t / ex) % ey), rz = (int)(t / ((long long)ex * ey));
-  cell_restrict<T>(fine, coarse, c, rx, ry, rz);
+  cell_restrict_q<T, I>(fine, coarse, c, rx, ry, rz, blockIdx.y);
 }
 
 template <typename T, bool PAIRED, typename I>
@@ -166,6 +169,48 @@ __global__ void k_restrict_resc(const T* __restrict__ fine, T* __restrict__ coar
   if (t >= (long long)ex * ey * ez) return;
   const int rx = (int)(t % ex), ry = (int)((t / ex) % ey), rz = (int)(t / ((long long)ex * ey));
   cell_restrict_resc<T, PAIRED, I>(fine, coarse, c, rx, ry, rz, om_s, om_b, rho0, r);
+}
+
+// The same for few cells: one thread a cell takes its fifteen means one after
+// the other, each a round of loads.  Here four warps take a quarter of the
+// populations of 32 cells each, and the first of them collides the means.
+// Where the line lies: us a coarse step, one thread a cell against this, FP64
+// with 1,728 / 13,824 / 32,768 / 64,000 / 82,368 / 190,000 covered cells 33.9 / 48.2
+// / 76.7 / 115.0 / 136.9 / 277.7 against 29.1 / 45.6 / 74.0 / 113.5 / 141.5 / 280.8
+// (36.1 / 51.1 / 78.8 / 117.2 / 141.6 / 281.9 before the loads ran ahead); FP32 with
+// 32,768 / 82,368 / 128,128 / 262,144 28.9 / 66.2 / 95.2 / 187.3 against 26.9 / 63.7 /
+// 94.4 / 189.7.  From there on a thread a cell fills the chip, and this form's
+// blocks hold three idle warps while the first collides.
+constexpr int kMeanCells = 32, kMeanWarps = 4;
+constexpr long long kFewCells = 1 << 16;
+template <typename T, bool PAIRED, typename I>
+__global__ void __launch_bounds__(kMeanCells* kMeanWarps, sizeof(T) == 8 ? 0 : 8)
+    k_restrict_resc_few(const T* __restrict__ fine, T* __restrict__ coarse, Coupling c, T om_s,
+                        T om_b, T rho0, DfRates r, unsigned* moving) {
+  __shared__ T mean[NV][kMeanCells];
+  chain_begin();
+  if (moving && blockIdx.x == 0 && threadIdx.x == 0) *moving = 0;
+  const int ex = c.fb.n[0] / 2, ey = c.fb.n[1] / 2, ez = c.fb.n[2] / 2;
+  const int lane = threadIdx.x % kMeanCells, part = threadIdx.x / kMeanCells;
+  const int t = blockIdx.x * kMeanCells + lane;
+  const bool in = t < ex * ey * ez;
+  const int rx = t % ex, ry = (t / ex) % ey, rz = t / (ex * ey);
+#pragma unroll
+  for (int k = 0; k < NV; k += kMeanWarps)
+    if (in && k + part < NV) {
+      T v[8];
+      ld_covered<T, I>(fine, c, rx, ry, rz, k + part, v);
+      mean[k + part][lane] = mean8(v);
+    }
+  __syncthreads();
+  if (part != 0 || !in) return;
+  T f[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) f[q] = mean[q][lane];
+  const I cc = covered_index<I>(c, rx, ry, rz), csq = (I)c.cb.sq;
+  collide_cell<T, PAIRED, true>(f, om_s, om_b, rho0, r);
+#pragma unroll
+  for (int q = 0; q < NV; ++q) st_pop(coarse, (I)q * csq + cc, c.cb, f[q]);
 }
 
 template <typename T>
@@ -306,7 +351,9 @@ cudaError_t launch_coalesce(const T* fine, T* coarse, const Coupling& c, double 
 template <typename T>
 cudaError_t launch_restrict(const T* fine, T* coarse, const Coupling& c, cudaStream_t st) {
   const long long n = (long long)(c.fb.n[0] / 2) * (c.fb.n[1] / 2) * (c.fb.n[2] / 2);
-  k_restrict<T><<<blocks_for(n, 128), 128, 0, st>>>(fine, coarse, c);
+  with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
+    k_restrict<T, decltype(i)><<<dim3(blocks_for(n, 128), NV), 128, 0, st>>>(fine, coarse, c);
+  });
   return cudaGetLastError();
 }
 
@@ -364,13 +411,20 @@ cudaError_t launch_restrict_resc(const T* fine, T* coarse, const Coupling& c, do
                                  unsigned* moving) {
   const long long n = (long long)(c.fb.n[0] / 2) * (c.fb.n[1] / 2) * (c.fb.n[2] / 2);
   const DfRates r = quiet(rates_of<T>(om_s, om_b));
+  const bool few = n < (sizeof(T) == 8 ? kFewCells : 2 * kFewCells);
+  const unsigned grid = blocks_for(n, few ? kMeanCells : 128);
   with_index(index32(c.cb) && index32(c.fb), [&](auto i) {
     using I = decltype(i);
+    auto go = [&](auto pairs) {
+      constexpr bool P = decltype(pairs)::value;
+      chained(few ? k_restrict_resc_few<T, P, I> : k_restrict_resc<T, P, I>, grid,
+              few ? kMeanCells * kMeanWarps : 128, st, fine, coarse, c, (T)om_s, (T)om_b, (T)rho0, r,
+              moving);
+    };
     if (sizeof(T) == 8 && paired)
-      chained(k_restrict_resc<T, sizeof(T) == 8, I>, blocks_for(n, 128), 128, st, fine, coarse, c, (T)om_s, (T)om_b, (T)rho0, r, moving);
+      go(std::integral_constant<bool, sizeof(T) == 8>());
     else
-      chained(k_restrict_resc<T, false, I>, blocks_for(n, 128), 128, st, fine, coarse, c, (T)om_s,
-                                                                       (T)om_b, (T)rho0, r, moving);
+      go(std::false_type());
   });
   return cudaGetLastError();
 }
