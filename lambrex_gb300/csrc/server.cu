@@ -457,6 +457,9 @@ int run_macro_steps(lbx_server* s, int n) {
 
 template <typename T>
 int finish_request(lbx_server* s, Req& q) {
+  if (!s->d_work)  // with the first request that finishes
+    CK(cudaMalloc(&s->d_work, (lbx::reduce_partials_doubles() + 4 * kMaxLevels) * sizeof(double)));
+  if (!s->h_work) CK(cudaMallocHost(&s->h_work, (4 * kMaxLevels + 1) * sizeof(double)));
   // every level back to its streamed state, gathered from the store each
   // level's last step read (its coarse cells' entries hold the coalescence);
   // a request of zero steps never left it
@@ -540,12 +543,8 @@ int lbx_server_create(size_t hbm_budget_bytes, int max_active, int precision, lb
       e = cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
   }
-  if (e == cudaSuccess)
-    e = cudaMalloc(&s->d_work, (lbx::reduce_partials_doubles() + 4 * kMaxLevels) * sizeof(double));
-  if (e == cudaSuccess) e = cudaMallocHost(&s->h_work, (4 * kMaxLevels + 1) * sizeof(double));
   if (e != cudaSuccess) {
     lbx::note_error("lbx_server_create", e);
-    if (s->d_work) cudaFree(s->d_work);
     if (s->pool) cudaMemPoolDestroy(s->pool);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
