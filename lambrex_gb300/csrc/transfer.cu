@@ -32,7 +32,6 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
-#include <condition_variable>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -40,8 +39,8 @@
 #include <exception>
 #include <mutex>
 #include <thread>
-#include <vector>
 
+#include "copy_pool.h"
 #include "sim_internal.h"
 
 namespace lbx {
@@ -157,66 +156,6 @@ constexpr size_t kProbeChunk = (size_t)16 << 20;  // first direct chunk of a lar
 constexpr double kDirectMinRate = 100e9;          // B/s below which the rest is staged
 constexpr int kBufs = 4;                          // staging buffers
 constexpr unsigned kMaxCopyThreads = 12;          // memcpy saturates near 12
-
-// Persistent copy threads: copy() splits one memcpy over all of them (the
-// caller takes part 0) and returns when every part is done.  The threads
-// sleep on a condition variable between copies.
-class CopyPool {
- public:
-  explicit CopyPool(unsigned threads) : T_(threads) {
-    for (unsigned i = 1; i < T_; ++i) ts_.emplace_back([this, i] { worker(i); });
-  }
-  ~CopyPool() {
-    {
-      std::lock_guard<std::mutex> l(mu_);
-      stop_ = true;
-    }
-    cv_.notify_all();
-    for (auto& t : ts_) t.join();
-  }
-  void copy(char* dst, const char* src, size_t len) {
-    {
-      std::lock_guard<std::mutex> l(mu_);
-      dst_ = dst;
-      src_ = src;
-      len_ = len;
-      left_.store(T_ - 1);
-      ++gen_;
-    }
-    cv_.notify_all();
-    part(0);
-    while (left_.load() > 0) std::this_thread::yield();
-  }
-
- private:
-  void part(unsigned i) {
-    const size_t p = (len_ + T_ - 1) / T_, o = (size_t)i * p;
-    if (o < len_) std::memcpy(dst_ + o, src_ + o, std::min(p, len_ - o));
-  }
-  void worker(unsigned i) {
-    long seen = 0;
-    for (;;) {
-      {
-        std::unique_lock<std::mutex> l(mu_);
-        cv_.wait(l, [&] { return stop_ || gen_ != seen; });
-        if (stop_) return;
-        seen = gen_;
-      }
-      part(i);
-      left_.fetch_sub(1);
-    }
-  }
-  const unsigned T_;
-  std::vector<std::thread> ts_;
-  std::mutex mu_;
-  std::condition_variable cv_;
-  long gen_ = 0;
-  bool stop_ = false;
-  char* dst_ = nullptr;
-  const char* src_ = nullptr;
-  size_t len_ = 0;
-  std::atomic<unsigned> left_{0};
-};
 
 // the process's copy threads, started on first use
 CopyPool& copy_pool() {
@@ -377,7 +316,9 @@ static cudaError_t download_small(char* dst, const char* src, size_t bytes, cuda
     if (c + 1 < chunks)
       e = cudaMemcpyAsync(S.buf[(c + 1) & 1], src + (c + 1) * kSmallChunk, len(c + 1),
                           cudaMemcpyDeviceToHost, st);
-    copy_pool().copy(dst + c * kSmallChunk, S.buf[c & 1], len(c));
+    // in this thread alone while the pool brings over another caller's chunk
+    if (!copy_pool().try_copy(dst + c * kSmallChunk, S.buf[c & 1], len(c)))
+      std::memcpy(dst + c * kSmallChunk, S.buf[c & 1], len(c));
   }
   return e;
 }
