@@ -6,6 +6,7 @@
 #include <condition_variable>
 #include <cstddef>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -18,8 +19,16 @@ namespace lbx {
 // a second caller waits for the first one's (copy) or is told so (try_copy).
 class CopyPool {
  public:
-  explicit CopyPool(unsigned threads) : T_(threads) {
-    for (unsigned i = 1; i < T_; ++i) ts_.emplace_back([this, i] { worker(i); });
+  // with as many of the threads as the system gives: at worst the caller's alone
+  explicit CopyPool(unsigned threads) {
+    try {
+      ts_.reserve(threads);
+      for (unsigned i = 1; i < threads; ++i) {
+        ts_.emplace_back([this, i] { worker(i); });
+        T_ = i + 1;  // no worker reads it before the first job
+      }
+    } catch (const std::exception&) {
+    }
   }
   ~CopyPool() {
     {
@@ -72,7 +81,7 @@ class CopyPool {
       left_.fetch_sub(1);
     }
   }
-  const unsigned T_;
+  unsigned T_ = 1;  // the caller and the threads
   std::vector<std::thread> ts_;
   std::mutex job_;  // held for the whole of a copy
   std::mutex mu_;

@@ -36,7 +36,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <exception>
 #include <mutex>
 #include <thread>
 
@@ -286,13 +285,7 @@ static cudaError_t download_small(char* dst, const char* src, size_t bytes, cuda
   std::unique_lock<std::mutex> lock(S.mu, std::try_to_lock);
   if (lock && !S.buf[0] && !S.failed) {
     char* p = nullptr;
-    bool threads = true;
-    try {
-      copy_pool();
-    } catch (const std::exception&) {  // no threads to be had
-      threads = false;
-    }
-    if (threads && cudaHostAlloc(&p, 2 * kSmallChunk, cudaHostAllocPortable) == cudaSuccess) {
+    if (cudaHostAlloc(&p, 2 * kSmallChunk, cudaHostAllocPortable) == cudaSuccess) {
       S.buf[0] = p;
       S.buf[1] = p + kSmallChunk;
     } else {

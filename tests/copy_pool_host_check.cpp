@@ -1,9 +1,13 @@
 // Host build of the copy threads (csrc/copy_pool.h) for tests/test_copy_pool.py.
 //
-// usage: copy_pool_host_check threads rounds
+// usage: copy_pool_host_check threads rounds [of them the system gives]
 // Two callers at once, one with chunks of 16 MB and one with chunks of 1 MB and
 // less of ever other lengths; prints how many copies came out wrong, or wrote
 // beyond their end.
+#include <dlfcn.h>
+#include <pthread.h>
+
+#include <cerrno>
 #include <cstdio>
 #include <cstdlib>
 #include <string>
@@ -11,6 +15,15 @@
 #include <vector>
 
 #include "copy_pool.h"
+
+static int g_threads_given = -1;  // pthread_create fails from then on; -1: never
+extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* arg) {
+  using create = int (*)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*);
+  static const create real = (create)dlsym(RTLD_NEXT, "pthread_create");
+  if (g_threads_given == 0) return EAGAIN;
+  if (g_threads_given > 0) --g_threads_given;
+  return real(t, a, f, arg);
+}
 
 namespace {
 constexpr size_t kGuard = 4096;
@@ -32,8 +45,10 @@ int caller(lbx::CopyPool& pool, size_t len, int rounds, unsigned seed, bool wait
 }  // namespace
 
 int main(int argc, char** argv) {
-  if (argc != 3) return 2;
+  if (argc != 3 && argc != 4) return 2;
+  if (argc == 4) g_threads_given = std::atoi(argv[3]);
   lbx::CopyPool pool((unsigned)std::atoi(argv[1]));
+  g_threads_given = -1;
   const int rounds = std::atoi(argv[2]);
   int wrong[2];
   std::thread a([&] { wrong[0] = caller(pool, (size_t)16 << 20, rounds, 1, true); });

@@ -18,7 +18,7 @@ def harness(tmp_path_factory):
     if not gxx:
         pytest.skip("g++ is not available")
     exe = str(tmp_path_factory.mktemp("pool") / "copy_pool_host_check")
-    subprocess.run([gxx, "-std=c++17", "-O2", "-pthread", "-I" + os.path.join(ROOT, "lambrex_gb300", "csrc"),
+    subprocess.run([gxx, "-std=c++17", "-O2", "-pthread", "-ldl", "-I" + os.path.join(ROOT, "lambrex_gb300", "csrc"),
                     os.path.join(HERE, "copy_pool_host_check.cpp"), "-o", exe], check=True, capture_output=True)
     return exe
 
@@ -26,6 +26,13 @@ def harness(tmp_path_factory):
 @pytest.mark.parametrize("threads", [1, 2, 12])
 def test_two_callers_at_once(harness, threads):
     out = subprocess.run([harness, str(threads), "60"], check=True, capture_output=True, text=True, timeout=300)
+    assert out.stdout.split() == ["0", "0"]
+
+
+@pytest.mark.parametrize("given", [0, 1, 5])
+def test_fewer_threads_than_asked_for(harness, given):
+    """The pool goes on with the threads that the system gives."""
+    out = subprocess.run([harness, "12", "20", str(given)], check=True, capture_output=True, text=True, timeout=300)
     assert out.stdout.split() == ["0", "0"]
 
 
