@@ -223,12 +223,14 @@ __host__ __device__ __forceinline__ void equilibrium_shifted(double rho, double 
 
 // Division of numbers below 2^31 by a fixed d >= 1 (round-up method, Granlund
 // and Montgomery 1994): with 2^(l-1) < d <= 2^l and m = floor(2^32 (2^l - d) / d)
-// + 1, x / d = (floor(x m / 2^32) + x) >> l; the sum stays below 2^32.
+// + 1, x / d = (floor(x m / 2^32) + x) >> l; the sum stays below 2^32.  A d of
+// 2^31 and more has none (boxes of so many cells: cell_coords).
 struct Divisor {
   uint32_t m;
   int l;
 };
-inline Divisor make_divisor(uint32_t d) {
+inline Divisor make_divisor(uint64_t d) {
+  if (d >> 31) return Divisor{0, 0};
   int l = 0;
   while ((uint64_t(1) << l) < d) ++l;
   return Divisor{(uint32_t)(((uint64_t(1) << 32) * ((uint64_t(1) << l) - d)) / d + 1), l};
@@ -260,11 +262,11 @@ inline Box3 make_box(int nx, int ny, int nz, int g) {
   b.n[0] = nx;
   b.n[1] = ny;
   b.n[2] = nz;
-  b.row = make_divisor((uint32_t)nx);
-  b.plane = make_divisor((uint32_t)((long long)nx * ny));
+  b.row = make_divisor((uint64_t)nx);
+  b.plane = make_divisor((uint64_t)nx * ny);
   b.g = g;
   b.sx = nx + 2 * g;
-  b.srow = make_divisor((uint32_t)b.sx);
+  b.srow = make_divisor((uint64_t)b.sx);
   b.sxy = (long long)(ny + 2 * g) * b.sx;
   b.sq = (long long)(nz + 2 * g) * b.sxy;
   return b;

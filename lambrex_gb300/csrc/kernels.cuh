@@ -30,22 +30,42 @@ struct CellLaunch {
   dim3 grid, block;
 };
 inline CellLaunch cell_launch(const Box3& b, int threads) {
-  const long long n = (long long)b.n[0] * b.n[1] * b.n[2];
-  while (threads > 32 && n < 76ll * threads) threads /= 2;
-  return CellLaunch{dim3((unsigned)((n + threads - 1) / threads)), dim3((unsigned)threads)};
+  const double n = (double)b.n[0] * b.n[1] * b.n[2];
+  while (threads > 32 && n < 76.0 * threads) threads /= 2;
+  const double blocks = std::ceil(n / threads);  // past a grid's limit: refused by the launch
+  return CellLaunch{dim3(blocks < 4294967295.0 ? (unsigned)blocks : 4294967295u), dim3((unsigned)threads)};
+}
+// Whether the cells of a box are numbered in 32 bits.  The simulations and the
+// batch engine refuse larger boxes; the steps, the equilibrium and the fields on
+// device pointers take them.
+inline bool cells32(const Box3& b) { return (double)b.n[0] * b.n[1] * b.n[2] < 2147483648.0; }
+// (x, y, z) of valid cell c in storage order, false beyond the last one; 64-bit
+// numbers (C) take the place of Box3's multipliers, which hold below 2^31
+template <typename C>
+__host__ __device__ __forceinline__ bool cell_coords(const Box3& b, C c, int& x, int& y, int& z) {
+  if constexpr (sizeof(C) == 4) {
+    z = (int)divide(c, b.plane);
+    const uint32_t p = c - (uint32_t)z * (uint32_t)(b.n[0] * b.n[1]);
+    y = (int)divide(p, b.row);
+    x = (int)(p - (uint32_t)y * (uint32_t)b.n[0]);
+    return z < b.n[2];
+  } else {
+    const C row = (C)b.n[0], plane = row * (C)b.n[1], q = c / plane, p = c - q * plane;
+    if (q >= (C)b.n[2]) return false;
+    z = (int)q;
+    y = (int)(p / row);
+    x = (int)(p - (C)y * row);
+    return true;
+  }
 }
 // whether every element index of a store fits in 31 bits (512^3 does)
 inline bool index32(const Box3& b) { return (long long)NV * b.sq < (1ll << 31); }
 #ifdef __CUDACC__
 // (x, y, z) of this thread's cell under cell_launch (its first block being
 // block `first` of the grid); false beyond the last one
+template <typename C = uint32_t>
 __device__ __forceinline__ bool cell_xyz(const Box3& b, int& x, int& y, int& z, unsigned first = 0) {
-  const uint32_t c = (blockIdx.x - first) * blockDim.x + threadIdx.x;
-  z = (int)divide(c, b.plane);
-  const uint32_t p = c - (uint32_t)z * (uint32_t)(b.n[0] * b.n[1]);
-  y = (int)divide(p, b.row);
-  x = (int)(p - (uint32_t)y * (uint32_t)b.n[0]);
-  return z < b.n[2];
+  return cell_coords<C>(b, (C)(blockIdx.x - first) * blockDim.x + threadIdx.x, x, y, z);
 }
 #endif
 

@@ -24,13 +24,13 @@ constexpr int kPushThreads = 128;
 // (src/AmrSim.cpp:25-135; include/component.h:22-29 written as a push:
 // f_new(x + c_q, q) = C(f)(x, q) is the same map as the reference's pull
 // f_new(x, q) = C(f)(x - c_q, q)).
-template <typename T, bool COVER, bool PAIRED, typename I>
+template <typename T, bool COVER, bool PAIRED, typename I, typename C = uint32_t>
 __global__ void LBX_STEP_BOUNDS(T)
     k_step_periodic(const T* __restrict__ fin, T* __restrict__ fout, Box3 b, IBox cov, T om_s,
                     T om_b, T rho0, DfRates r) {
   chain_begin();
   int x, y, z;
-  if (!cell_xyz(b, x, y, z)) return;
+  if (!cell_xyz<C>(b, x, y, z)) return;
   cell_step_periodic<T, COVER, PAIRED, I>(fin, fout, b, cov, x, y, z, om_s, om_b, rho0, r);
 }
 
@@ -71,11 +71,11 @@ __global__ void k_shift(const T* __restrict__ fin, T* __restrict__ fout, Box3 b)
   for (int q = 0; q < NV; ++q) st_pop(fout, q * b.sq + c, b, v[q]);
 }
 
-template <typename T>
+template <typename T, typename C>
 __global__ void k_equilibrium(const double* __restrict__ rho, const double* __restrict__ u,
                               T* __restrict__ f, Box3 b, double rho0) {
   int x, y, z;
-  if (!cell_xyz(b, x, y, z)) return;
+  if (!cell_xyz<C>(b, x, y, z)) return;
   const long long n = (long long)b.n[0] * b.n[1] * b.n[2];
   const long long v = ((long long)z * b.n[1] + y) * b.n[0] + x;
   const double r = ld_cell(rho, v, n), ux = ld_cell(u, v, 3 * n), uy = ld_cell(u, n + v, 3 * n),
@@ -116,12 +116,12 @@ __global__ void k_init_pulse(T* __restrict__ f, Box3 b, int axis, int index, dou
   }
 }
 
-template <typename T, bool GATHER>
+template <typename T, bool GATHER, typename C = uint32_t>
 __global__ void k_hydro(const T* __restrict__ f, Box3 b, double rho0, double* __restrict__ rho,
                         double* __restrict__ u) {
   chain_begin();
   int x, y, z;
-  if (!cell_xyz(b, x, y, z)) return;
+  if (!cell_xyz<C>(b, x, y, z)) return;
   cell_hydro<T, GATHER>(f, b, rho0, rho, u, x, y, z);
 }
 
@@ -484,8 +484,10 @@ static void step_periodic(const T* fin, T* fout, const Box3& b, const IBox& cove
   const CellLaunch rl = cell_launch(b, kPushThreads);
   if (index32(b))
     chained(k_step_periodic<T, COVER, PAIRED, int>, rl.grid, rl.block, st, fin, fout, b, covered, (T)om_s, (T)om_b, (T)rho0, r);
-  else
+  else if (COVER || cells32(b))  // a covered box is a simulation's
     chained(k_step_periodic<T, COVER, PAIRED, long long>, rl.grid, rl.block, st, fin, fout, b, covered, (T)om_s, (T)om_b, (T)rho0, r);
+  else
+    chained(k_step_periodic<T, false, PAIRED, long long, uint64_t>, rl.grid, rl.block, st, fin, fout, b, covered, (T)om_s, (T)om_b, (T)rho0, r);
 }
 
 template <typename T>
@@ -515,7 +517,10 @@ template <typename T>
 cudaError_t launch_equilibrium(const double* rho, const double* u, T* f, const Box3& b,
                                double rho0, cudaStream_t st) {
   const CellLaunch rl = cell_launch(b, 128);
-  k_equilibrium<T><<<rl.grid, rl.block, 0, st>>>(rho, u, f, b, rho0);
+  if (cells32(b))
+    k_equilibrium<T, uint32_t><<<rl.grid, rl.block, 0, st>>>(rho, u, f, b, rho0);
+  else
+    k_equilibrium<T, uint64_t><<<rl.grid, rl.block, 0, st>>>(rho, u, f, b, rho0);
   return cudaGetLastError();
 }
 
@@ -568,8 +573,10 @@ cudaError_t launch_hydro(const T* f, const Box3& b, double rho0, double* rho, do
   const CellLaunch rl = cell_launch(b, 128);
   if (gather)
     chained(k_hydro<T, true>, rl.grid, rl.block, st, f, b, rho0, rho, u);
-  else
+  else if (cells32(b))
     chained(k_hydro<T, false>, rl.grid, rl.block, st, f, b, rho0, rho, u);
+  else
+    chained(k_hydro<T, false, uint64_t>, rl.grid, rl.block, st, f, b, rho0, rho, u);
   return cudaGetLastError();
 }
 
