@@ -19,6 +19,7 @@
 #include "kernels.cuh"
 #include "lbx.h"
 #include "sim_internal.h"
+#include "step_graphs.h"
 
 using lbx::Box3;
 using lbx::Coupling;
@@ -623,8 +624,7 @@ int macro_step(lbx_sim* s) {
   return s->f64() ? c_advance<double>(s, 0) : c_advance<float>(s, 0);
 }
 
-constexpr int kGraphMinSteps = 4;   // shorter runs launch directly
-constexpr int kGraphMaxPeriod = 12; // buffer roles cycle with a period dividing 6 or 2
+constexpr int kGraphMinSteps = 4;  // shorter runs launch directly, as those that no graph fits
 
 std::vector<LevelSig> signature(const lbx_sim* s) {
   std::vector<LevelSig> v(s->lev.size());
@@ -662,32 +662,12 @@ bool graph_matches(lbx_sim* s, int left) {
   }
   return best > 0;
 }
-// Steps of the graph that `left` steps are to be taken in, 0: launch them
-// directly.  Between the kernels of one graph there is no gap (chained,
-// launch.cuh), between two replays there is: graphs of 32 launches, and of 8 for
-// what is left (10x10x50 FP64, 60 steps: 4.1 us a step in graphs of two).
-int graph_steps(const lbx_sim* s, int left) {
-  const int per_step = std::max(1, s->finest == 0 ? 1 : 4 << (s->finest - 1));  // launches, about
-  for (const int launches : {32, 8})
-    if ((long long)left * per_step >= launches) return std::max(1, launches / per_step);
-  return 0;
-}
-// Capture macro steps from the simulation's own launches until every level's
-// buffers are back in their roles, then run the captured steps once (the
-// host-side bookkeeping already advanced while capturing).  Keeps the graph
-// for replay when the roles did return.
-int capture_graph(lbx_sim* s, int* left) {
-  const int atleast = std::min(std::max(1, graph_steps(s, *left)), *left);
-  s->gcur = 0;  // replaces the one not used for longest
-  for (int i = 1; i < 4; ++i)
-    if (s->graphs[i].used < s->graphs[s->gcur].used) s->gcur = i;
-  StepGraph& G = s->graphs[s->gcur];
-  G.used = ++s->gclock;
-  if (G.exec) {
-    CK(cudaStreamSynchronize(s->stream));
-    cudaGraphExecDestroy(G.exec);
-    G.exec = nullptr;
-  }
+// Capture `steps` macro steps, after which every level's buffers are back in
+// their roles, from the simulation's own launches and run them once (the
+// host-side bookkeeping already advanced while capturing).  Keeps the graph for
+// replay; *kept: whether it did.
+int capture_graph(lbx_sim* s, int steps, bool* kept) {
+  *kept = false;
   const std::vector<LevelSig> sig0 = signature(s);
   std::vector<double> t0(s->lev.size());
   std::vector<int> n0(s->lev.size());
@@ -697,12 +677,8 @@ int capture_graph(lbx_sim* s, int* left) {
   }
   const long long launches0 = s->launches;
   CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-  int m = 0, rc = LBX_OK;
-  do {
-    rc = macro_step(s);
-    ++m;
-  } while (rc == LBX_OK && m < std::min(kGraphMaxPeriod + atleast - 1, *left) &&
-           (m < atleast || !(signature(s) == sig0)));
+  int rc = LBX_OK;
+  for (int m = 0; rc == LBX_OK && m < steps; ++m) rc = macro_step(s);
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(s->stream, &g);
   if (rc != LBX_OK || e != cudaSuccess) {
@@ -714,15 +690,24 @@ int capture_graph(lbx_sim* s, int* left) {
   const cudaError_t ei = cudaGraphInstantiate(&exec, g, 0);
   cudaGraphDestroy(g);
   CK(ei);
-  CK(cudaGraphLaunch(exec, s->stream));  // the m steps just captured
-  *left -= m;
   if (!(signature(s) == sig0)) {  // not replayable: run once, drop
+    CK(cudaGraphLaunch(exec, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     cudaGraphExecDestroy(exec);
     return LBX_OK;
   }
+  s->gcur = 0;  // in place of the one not used for longest
+  for (int i = 1; i < 4; ++i)
+    if (s->graphs[i].used < s->graphs[s->gcur].used) s->gcur = i;
+  StepGraph& G = s->graphs[s->gcur];
+  G.used = ++s->gclock;
+  if (G.exec) {
+    CK(cudaStreamSynchronize(s->stream));
+    cudaGraphExecDestroy(G.exec);
+  }
+  *kept = true;
   G.exec = exec;
-  G.period = m;
+  G.period = steps;
   G.launches = s->launches - launches0;
   G.sig = sig0;
   G.finest = s->finest;
@@ -733,6 +718,7 @@ int capture_graph(lbx_sim* s, int* left) {
     G.dtime[L] = s->lev[L].time - t0[L];  // exact: dt is a power of two
     G.dstep[L] = s->lev[L].step - n0[L];
   }
+  CK(cudaGraphLaunch(exec, s->stream));  // the steps just captured
   return LBX_OK;
 }
 
@@ -1197,29 +1183,26 @@ int lbx_iterate(lbx_sim* s, int nsteps) {
     RET(macro_step(s));
     --left;
   }
-  if (left >= kGraphMinSteps) {
-    while (left >= kGraphMinSteps) {
-      const int steps = graph_steps(s, left);
-      if (steps == 0) break;
-      const bool have = graph_matches(s, left);
-      if (!have || s->graphs[s->gcur].period < steps) {
-        // inside a capture of the caller's no new graph can be made: the shorter
-        // one at hand, or the steps themselves, become nodes of the caller's
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        CK(cudaStreamIsCapturing(s->stream, &cs));
-        if (cs != cudaStreamCaptureStatusNone) {
-          if (!have) break;
-          for (const int period = s->graphs[s->gcur].period; left >= period; left -= period)
-            RET(replay_graph(s));
-          continue;
-        }
-        RET(capture_graph(s, &left));  // runs what it captures
-        if (!s->graphs[s->gcur].exec) break;
+  while (left >= kGraphMinSteps) {
+    const int steps = lbx::graph_steps(s->finest, s->amr_mode == LBX_AMR_FAITHFUL, left);
+    if (steps == 0) break;
+    const bool have = graph_matches(s, left);
+    if (!have || s->graphs[s->gcur].period < steps) {
+      // inside a capture of the caller's no new graph can be made: the shorter
+      // one at hand, or the steps themselves, become nodes of the caller's
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      CK(cudaStreamIsCapturing(s->stream, &cs));
+      if (cs == cudaStreamCaptureStatusNone) {
+        bool kept;
+        RET(capture_graph(s, steps, &kept));  // runs what it captures
+        left -= steps;
+        if (!kept) break;
         continue;
       }
-      for (const int period = s->graphs[s->gcur].period; left >= period; left -= period)
-        RET(replay_graph(s));
+      if (!have) break;
     }
+    for (const int period = s->graphs[s->gcur].period; left >= period; left -= period)
+      RET(replay_graph(s));
   }
   for (; left > 0; --left) RET(macro_step(s));
   return LBX_OK;

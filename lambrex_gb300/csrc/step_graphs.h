@@ -1,0 +1,35 @@
+// step_graphs.h -- how many steps of a run are captured into one CUDA graph
+// (plain C++, so that the tests run it without the library).
+#pragma once
+#include <algorithm>
+
+namespace lbx {
+
+// Steps of level 0 after which every level's buffers are back in their roles.
+// A level's two buffers are swapped by each of its steps, and a finer level takes
+// an even number of them.  The faithful cycle rotates three buffers on each level
+// but the finest, which swaps two of its three once a cycle of the level below.
+inline int role_period(int finest, bool faithful) {
+  if (finest > 0 && faithful) return finest == 1 ? 6 : 3;
+  return 2;
+}
+
+// Steps of the graph that `left` steps are to be taken in, a multiple of the role
+// period and at most `left`; 0: launch them directly.  Between the kernels of one
+// graph there is no gap (chained, launch.cuh), between two replays there is:
+// graphs of 32 launches, and of 8 for what is left (10x10x50 FP64, 60 steps: 4.1 us
+// a step in graphs of two).  The faithful cycle's kernels are not chained: graphs
+// of one period, so that runs of any length find theirs again (of at least eight
+// steps, a run of nine was captured at each call).
+inline int graph_steps(int finest, bool faithful, int left) {
+  const int period = role_period(finest, faithful);
+  if (finest > 0 && faithful) return left >= period ? period : 0;
+  const int per_step = finest == 0 ? 1 : 4 << std::min(finest - 1, 8);  // launches, about
+  for (const int launches : {32, 8}) {
+    const int steps = (std::max(1, launches / per_step) + period - 1) / period * period;
+    if (left >= steps) return steps;
+  }
+  return 0;
+}
+
+}  // namespace lbx
