@@ -1183,23 +1183,19 @@ int lbx_iterate(lbx_sim* s, int nsteps) {
     RET(macro_step(s));
     --left;
   }
-  while (left >= kGraphMinSteps) {
+  // inside a capture of the caller's no graph can be made or launched: the steps
+  // themselves become nodes of the caller's
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (left >= kGraphMinSteps) CK(cudaStreamIsCapturing(s->stream, &cs));
+  while (left >= kGraphMinSteps && cs == cudaStreamCaptureStatusNone) {
     const int steps = lbx::graph_steps(s->finest, s->amr_mode == LBX_AMR_FAITHFUL, left);
     if (steps == 0) break;
-    const bool have = graph_matches(s, left);
-    if (!have || s->graphs[s->gcur].period < steps) {
-      // inside a capture of the caller's no new graph can be made: the shorter
-      // one at hand, or the steps themselves, become nodes of the caller's
-      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      CK(cudaStreamIsCapturing(s->stream, &cs));
-      if (cs == cudaStreamCaptureStatusNone) {
-        bool kept;
-        RET(capture_graph(s, steps, &kept));  // runs what it captures
-        left -= steps;
-        if (!kept) break;
-        continue;
-      }
-      if (!have) break;
+    if (!graph_matches(s, left) || s->graphs[s->gcur].period < steps) {
+      bool kept;
+      RET(capture_graph(s, steps, &kept));  // runs what it captures
+      left -= steps;
+      if (!kept) break;
+      continue;
     }
     for (const int period = s->graphs[s->gcur].period; left >= period; left -= period)
       RET(replay_graph(s));

@@ -123,3 +123,47 @@ def test_faithful_runs_equal_single_steps(gpu_lib, finest, n, calls):
             assert np.array_equal(a.copy_f(lev), b.copy_f(lev), equal_nan=True)
             assert a.GetTime(lev) == b.GetTime(lev) and a.GetTimeStep(lev) == b.GetTimeStep(lev)
         assert a.launch_count() == b.launch_count()
+
+
+def make(gpu_lib, precision, mode, levels, dims=(12, 16, 12)):
+    rho_c, u_c = smooth_random(*dims, seed=7)
+    s = gpu_lib.AmrSim(*dims, levels, [1, 1, 1], 0.9, 0.8, precision=precision, amr_mode=mode)
+    s.SetInitialDensity(rho_c)
+    s.SetInitialVelocity(u_c)
+    s.InitFromScratch(0.0)
+    if levels >= 1:
+        s.SetStaticRefinement(0, (3, 4, 3), (8, 11, 8))
+    if levels >= 2:
+        s.SetStaticRefinement(1, (8, 10, 8), (13, 19, 13))
+    s.synchronize()
+    return s
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,mode,levels", [("f32s", "conservative", 0), ("f64", "rescaled", 1)])
+@pytest.mark.parametrize("steps", [3, 9, 64])
+def test_steps_captured_with_graphs_at_hand(gpu_lib, precision, mode, levels, steps):
+    """Steps captured by the caller where the handle has graphs for them (a
+    capture takes no launch of a graph, so they are not used there)."""
+    import ctypes
+
+    import torch
+
+    a, b = make(gpu_lib, precision, mode, levels), make(gpu_lib, precision, mode, levels)
+    for s in (a, b):
+        for n in (1, 300, 40):  # an even number from the first: the roles are those of the graphs
+            s.Iterate(n)
+        s.synchronize()
+    a.Iterate(steps)
+    p = ctypes.c_void_p()
+    assert b._L.lbx_get_stream(b._h, ctypes.byref(p)) == 0
+    stream = torch.cuda.ExternalStream(p.value)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream, capture_error_mode="thread_local"):
+        b.Iterate(steps)
+    with torch.cuda.stream(stream):
+        g.replay()  # once: a second run would want the stores back in their roles
+    stream.synchronize()
+    for lev in range(levels + 1):
+        assert np.array_equal(a.copy_f(lev), b.copy_f(lev))
+    del g
