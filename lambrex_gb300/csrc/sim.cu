@@ -154,6 +154,7 @@ struct lbx_sim {
   StepGraph graphs[4];
   int gcur = 0;            // the slot that matched or was captured last
   unsigned long long gclock = 0;
+  long long direct = 0;    // launches made without one (run_directly)
   // CalcHydroVars on a single pull-form level runs the next step with the
   // fields as its epilogue once the program has shown that it steps on after
   // reading fields (an Iterate after a CalcHydroVars); until then it runs the
@@ -1187,10 +1188,14 @@ int lbx_iterate(lbx_sim* s, int nsteps) {
   // themselves become nodes of the caller's
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (left >= kGraphMinSteps) CK(cudaStreamIsCapturing(s->stream, &cs));
+  const bool faithful = s->amr_mode == LBX_AMR_FAITHFUL;
+  const bool direct = lbx::run_directly(s->finest, faithful, left, s->direct);
   while (left >= kGraphMinSteps && cs == cudaStreamCaptureStatusNone) {
-    const int steps = lbx::graph_steps(s->finest, s->amr_mode == LBX_AMR_FAITHFUL, left);
+    const int steps = lbx::graph_steps(s->finest, faithful, left);
     if (steps == 0) break;
-    if (!graph_matches(s, left) || s->graphs[s->gcur].period < steps) {
+    const bool have = graph_matches(s, left);
+    if (!have && direct) break;
+    if (!have || s->graphs[s->gcur].period < steps) {
       bool kept;
       RET(capture_graph(s, steps, &kept));  // runs what it captures
       left -= steps;
@@ -1200,7 +1205,9 @@ int lbx_iterate(lbx_sim* s, int nsteps) {
     for (const int period = s->graphs[s->gcur].period; left >= period; left -= period)
       RET(replay_graph(s));
   }
+  const long long launches0 = s->launches;
   for (; left > 0; --left) RET(macro_step(s));
+  if (direct) s->direct += s->launches - launches0;
   return LBX_OK;
 }
 

@@ -25,7 +25,7 @@ def choose(tmp_path_factory):
                     os.path.join(HERE, "step_graphs_host_check.cpp"), "-o", exe], check=True, capture_output=True)
 
     def run(finest, faithful):
-        """for left = 0 .. 1000: (role period, steps)"""
+        """for left = 0 .. 1000: (role period, steps, whether a first run is direct)"""
         out = subprocess.run([exe], input="".join("%d %d %d\n" % (finest, faithful, n) for n in range(1001)),
                              check=True, capture_output=True, text=True).stdout.split("\n")[:1001]
         return [tuple(int(v) for v in line.split()) for line in out]
@@ -65,7 +65,7 @@ def test_graphs_return_the_roles(choose, finest, faithful):
     while period == 0 or roles != first:
         step(roles, finest, faithful)
         period += 1
-    for left, (p, steps) in enumerate(choose(finest, faithful)):
+    for left, (p, steps, _) in enumerate(choose(finest, faithful)):
         assert p % period == 0 and p <= 6
         assert steps % p == 0 and 0 <= steps <= left
 
@@ -83,7 +83,7 @@ def test_repeated_calls_capture_nothing(choose, finest, faithful, n):
         left, captured = n, 0
         while left >= MIN_STEPS and table[left][1]:
             have = max((k[1] for k in kept if k[0] == at % period and k[1] <= left), default=0)
-            if have < table[left][1]:
+            if have < table[left][1]:  # (a handle's first direct runs are over)
                 captured += 1
                 have = table[left][1]
                 kept.append((at % period, have))
@@ -167,3 +167,45 @@ def test_steps_captured_with_graphs_at_hand(gpu_lib, precision, mode, levels, st
     for lev in range(levels + 1):
         assert np.array_equal(a.copy_f(lev), b.copy_f(lev))
     del g
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,mode,levels", [("f64", "conservative", 0), ("f32s", "conservative", 0),
+                                                   ("f64", "rescaled", 1), ("f32s", "conservative", 2)])
+@pytest.mark.parametrize("lengths", [(300, 40, 9), (130, 70, 33, 64), (100, 29, 8, 45)])
+def test_direct_runs_and_graphs_equal_single_steps(gpu_lib, precision, mode, levels, lengths):
+    """A long first run in graphs; first runs launched directly, later ones in graphs."""
+    a, b = make(gpu_lib, precision, mode, levels), make(gpu_lib, precision, mode, levels)
+    for n in lengths:
+        for _ in range(n):
+            a.Iterate(1)
+        b.Iterate(n)
+        for s in (a, b):  # a readout between the calls: the store roles swap
+            s.CalcHydroVars(0)
+        for lev in range(levels + 1):
+            assert np.array_equal(a.copy_f(lev), b.copy_f(lev)), (n, lev)
+            assert a.GetTime(lev) == b.GetTime(lev) and a.GetTimeStep(lev) == b.GetTimeStep(lev)
+        assert a.launch_count() == b.launch_count()
+
+
+@pytest.mark.gpu
+def test_a_first_run_costs_no_more_than_its_steps(gpu_lib):
+    """Nine steps of a new handle, against the same in runs too short for a
+    graph: making a graph of eight launches took as long as twenty of them."""
+    import statistics
+    import time
+
+    def first(lengths):
+        t = []
+        for _ in range(25):
+            s = make(gpu_lib, "f32s", "conservative", 0)
+            t0 = time.perf_counter()
+            for n in lengths:
+                s.Iterate(n)
+            s.synchronize()
+            t.append(time.perf_counter() - t0)
+            s.close()
+        return statistics.median(t)
+
+    first([9])
+    assert first([9]) < 1.5 * first([3, 3, 3])
