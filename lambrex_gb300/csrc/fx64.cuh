@@ -493,16 +493,18 @@ __host__ __device__ __forceinline__ void collide_rest(double* f, double om_s, do
 #pragma unroll
   for (int q = 1; q < NV; ++q) f[q] = q < 7 ? ex : bd;
 }
+// such a cell, of ordinary size and not negative (without a density the general
+// form is NaN: 0 / 0)
 __host__ __device__ __forceinline__ bool is_rest(const double* f) {
   uint32_t h[NV], l[NV], d = 0;
 #pragma unroll
-  for (int q = 1; q < NV; ++q) d_words(f[q], &h[q], &l[q]);
+  for (int q = 0; q < NV; ++q) d_words(f[q], &h[q], &l[q]);
 #pragma unroll
   for (int q = 2; q < NV; ++q) {
     const int t = q < 7 ? 1 : 7;
     d |= (h[q] ^ h[t]) | (l[q] ^ l[t]);
   }
-  return d == 0;
+  return (d == 0) & fx_top_ok(fx_umax(fx_umax(h[0], h[1]), h[7]));
 }
 
 // whether a cell's populations are those of a fluid at rest (fx_at_rest)
