@@ -384,7 +384,8 @@ __host__ __device__ __forceinline__ float mean8(const float* v) {
 }
 
 // wp a + wn b: halves as one addition and the sum's exponent lowered (the
-// bits of the general form), one FP64 instruction instead of two
+// bits of the general form), one FP64 instruction instead of two; the general
+// form where the sum leaves the ordinary range
 template <typename T>
 __host__ __device__ __forceinline__ T weighted(T wp, T a, T wn, T b) {
   if constexpr (sizeof(T) == 8) {
@@ -393,7 +394,7 @@ __host__ __device__ __forceinline__ T weighted(T wp, T a, T wn, T b) {
       uint32_t h, l;
       d_words(s, &h, &l);
       const uint32_t e = (h >> 20) & 2047u;
-      return e - 2u < 2044u ? d_from_words(h - 0x100000u, l) : 0.5 * s;
+      if (e - 2u < 2044u) return d_from_words(h - 0x100000u, l);
     }
   }
   return wp * a + wn * b;
