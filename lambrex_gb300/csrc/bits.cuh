@@ -56,6 +56,16 @@ __host__ __device__ __forceinline__ float u2f(uint32_t r) {
 #endif
 }
 
+// to an integer toward zero, a value beyond the largest to that one (as the
+// device's conversion does; C++ leaves it undefined)
+__host__ __device__ __forceinline__ int f2i(float x) {
+#ifdef __CUDA_ARCH__
+  return __float2int_rz(x);
+#else
+  return x >= 0x1p31f ? 0x7fffffff : (int)x;
+#endif
+}
+
 // approximate FP32 reciprocal (the hardware's; any error below 2^-16 will do)
 __host__ __device__ __forceinline__ float rcp_approx(float x) {
 #ifdef __CUDA_ARCH__

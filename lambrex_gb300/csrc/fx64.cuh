@@ -121,7 +121,7 @@ __host__ __device__ __forceinline__ int64_t fx_mul(int64_t a, FxDigits b) {
 // second-order term), all in integers; relative error below 2^-56
 __host__ __device__ __forceinline__ int64_t fx_inverse(int64_t rho) {
   const uint32_t rh = (uint32_t)((uint64_t)rho >> 32), rl = (uint32_t)rho;
-  const uint32_t x0 = (uint32_t)(int)(rcp_approx(u2f(rh)) * 0x1p57f);  // 2^89 / rho, below 2^31
+  const uint32_t x0 = (uint32_t)f2i(rcp_approx(u2f(rh)) * 0x1p57f);  // 2^89 / rho, to 2^31 - 1
   const int64_t y = (int64_t)(((uint64_t)x0 * rl >> 32) + (uint64_t)x0 * rh);  // rho x0 / 2^32
   const int64_t e = (int64_t(1) << 57) - y;                                    // |e| < 2^36
   const int eh = (int)(e >> 6);
