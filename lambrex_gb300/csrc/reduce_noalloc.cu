@@ -29,27 +29,9 @@
 #include "lbx.h"
 #include "sim_internal.h"
 
-namespace {
-
-constexpr size_t kNoAllocScratch = (size_t)lbx::kReduceBlocks * 8;  // doubles
-constexpr size_t kNoAllocMaxCells = 0x7fffffff;  // cell index range of the kernel
-constexpr int kMaxDevices = 64;
-
-// Host code must not pass this symbol to a kernel: on the host it names a
-// stand-in object, not device memory.  Its device address comes from
-// cudaGetSymbolAddress below.
-static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScratch];
-
-std::mutex g_setup_mu;
-struct ScratchSlot {
-  unsigned long long ctx_id = 0;  // context the address belongs to (0: unknown)
-  double* addr = nullptr;
-};
-ScratchSlot g_scratch_addr[kMaxDevices];
-
-// Unique id of the calling thread's current context (cuCtxGetId), through
-// the driver entry points the runtime exposes; 0 if the driver lacks them.
-unsigned long long current_context_id() {
+// cuCtxGetId, through the driver entry points the runtime exposes; 0 if the
+// driver lacks them
+unsigned long long lbx::current_context_id() {
   typedef CUresult (*GetCurrentFn)(CUcontext*);
   typedef CUresult (*GetIdFn)(CUcontext, unsigned long long*);
   static GetCurrentFn get_current = nullptr;
@@ -71,6 +53,24 @@ unsigned long long current_context_id() {
   return get_id(ctx, &id) == CUDA_SUCCESS ? id : 0;
 }
 
+namespace {
+
+constexpr size_t kNoAllocScratch = (size_t)lbx::kReduceBlocks * 8;  // doubles
+constexpr size_t kNoAllocMaxCells = 0x7fffffff;  // cell index range of the kernel
+constexpr int kMaxDevices = 64;
+
+// Host code must not pass this symbol to a kernel: on the host it names a
+// stand-in object, not device memory.  Its device address comes from
+// cudaGetSymbolAddress below.
+static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScratch];
+
+std::mutex g_setup_mu;
+struct ScratchSlot {
+  unsigned long long ctx_id = 0;  // context the address belongs to (0: unknown)
+  double* addr = nullptr;
+};
+ScratchSlot g_scratch_addr[kMaxDevices];
+
 // device address of the scratch array in the current context (set up once
 // per device, again whenever the device's context has been re-created)
 int scratch_address(double** out) {
@@ -83,7 +83,7 @@ int scratch_address(double** out) {
   if (dev < 0 || dev >= kMaxDevices) return LBX_ERR_UNSUPPORTED;
   std::lock_guard<std::mutex> g(g_setup_mu);
   ScratchSlot& slot = g_scratch_addr[dev];
-  const unsigned long long ctx = current_context_id();
+  const unsigned long long ctx = lbx::current_context_id();
   if (!slot.addr || ctx == 0 || ctx != slot.ctx_id) {  // no context yet: the lookup makes it
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
@@ -92,7 +92,7 @@ int scratch_address(double** out) {
       return lbx::status_from_cuda(e);
     }
     slot.addr = static_cast<double*>(p);
-    slot.ctx_id = current_context_id();  // the lookup creates the context if needed
+    slot.ctx_id = lbx::current_context_id();  // the lookup creates the context if needed
   }
   *out = slot.addr;
   return LBX_OK;

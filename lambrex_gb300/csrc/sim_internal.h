@@ -18,6 +18,11 @@ cudaError_t upload_host(void* dst, const void* src, size_t bytes, cudaStream_t s
 // through the same staging buffers.
 cudaError_t download_host(void* dst, const void* src, size_t bytes, cudaStream_t st);
 
+// Unique id of the calling thread's current context (0: none, or not to be had).
+// What was allocated in a context is gone with it (cudaDeviceReset); the device's
+// next context has another id.
+unsigned long long current_context_id();
+
 // Named host range for profilers (NVTX; a no-op unless a tool is attached).
 // Every C-ABI call that launches work opens one, so a timeline shows which
 // API call issued which kernels.

@@ -271,23 +271,34 @@ cudaError_t copy_direct_while_fast(char* dst, const char* src, size_t bytes, cud
 // 25 by direct copies (fast or slow for a whole process).
 constexpr size_t kSmallMin = (size_t)1 << 20;
 constexpr size_t kSmallChunk = (size_t)4 << 20;
-struct SmallStage {
+struct SmallStage {  // of one device
   std::mutex mu;
   char* buf[2] = {};
   bool failed = false;
+  unsigned long long ctx = 0;  // the context that holds the buffers
+  int made = 0;                // how often they were: a program may go on between contexts
 };
-static SmallStage& small_stage() {
-  static SmallStage s;
-  return s;
+static SmallStage& small_stage(int dev) {
+  static SmallStage s[kMaxDev];
+  return s[dev];
 }
 static cudaError_t download_small(char* dst, const char* src, size_t bytes, cudaStream_t st) {
-  SmallStage& S = small_stage();
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) dev = 0;
+  SmallStage& S = small_stage(dev);
   std::unique_lock<std::mutex> lock(S.mu, std::try_to_lock);
+  const unsigned long long ctx = current_context_id();
+  if (lock && S.ctx != ctx) {  // the first time, or the buffers went with their context
+    S.buf[0] = S.buf[1] = nullptr;
+    S.failed = ctx == 0 || S.made >= 4;
+    S.ctx = ctx;
+  }
   if (lock && !S.buf[0] && !S.failed) {
     char* p = nullptr;
     if (cudaHostAlloc(&p, 2 * kSmallChunk, cudaHostAllocPortable) == cudaSuccess) {
       S.buf[0] = p;
       S.buf[1] = p + kSmallChunk;
+      ++S.made;
     } else {
       cudaGetLastError();
       S.failed = true;
