@@ -1,0 +1,24 @@
+// host_pages.h -- what the host knows of a caller's memory (plain C++, so that
+// the tests run it without the library).
+#pragma once
+#include <sys/mman.h>
+#include <unistd.h>
+
+#include <cstddef>
+#include <cstdint>
+#include <initializer_list>
+
+namespace lbx {
+
+// Whether the pages of [p, p + bytes) have been made, which a new array's are at
+// its first writing: a look at the first and the last (0.8 us each).
+inline bool pages_made(const void* p, size_t bytes) {
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), first = (uintptr_t)p, last = first + bytes - 1;
+  for (uintptr_t at : {first & ~(page - 1), last & ~(page - 1)}) {
+    unsigned char in = 0;
+    if (mincore(reinterpret_cast<void*>(at), page, &in) != 0 || !(in & 1)) return false;
+  }
+  return true;
+}
+
+}  // namespace lbx
