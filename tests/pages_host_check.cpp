@@ -1,8 +1,8 @@
 // Host build of the look at a caller's pages (csrc/host_pages.h) for
 // tests/test_host_pages.py: prints, in order, whether the pages are made of new
-// memory, of the same with its first, its middle and its last page left out, of
-// all of it written, of a part from the middle of a page on, and of memory that
-// is not mapped.
+// memory, of the same with its first and last page written, as an allocator
+// does, with its first and with its second half written, of all of it written,
+// of a part from the middle of a page on, and of memory that is not mapped.
 #include <cstdio>
 
 #include "host_pages.h"
@@ -14,18 +14,20 @@ int main() {
     madvise(p, n * page, MADV_NOHUGEPAGE);
     return p;
   };
-  char* p = fresh();
-  std::printf("%d", lbx::pages_made(p, n * page));
-  for (size_t skip : {(size_t)0, n - 1, n}) {
-    char* q = fresh();
-    for (size_t i = 0; i < n; ++i)
-      if (i != skip) q[i * page] = 1;
-    std::printf(" %d", lbx::pages_made(q, n * page));
-    if (skip == n) {
-      std::printf(" %d", lbx::pages_made(q + page / 2, 3 * page));
-      munmap(q, n * page);
-      std::printf(" %d\n", lbx::pages_made(q, n * page));
+  const struct {
+    size_t from, to;
+  } written[] = {{n, 0}, {0, n / 2}, {n / 2, n}, {0, n}};
+  for (const auto& w : written) {
+    char* p = fresh();
+    if (w.from > w.to) {
+      std::printf("%d ", lbx::pages_made(p, n * page));
+      p[0] = p[n * page - 1] = 1;
     }
+    for (size_t i = w.from; i < w.to; ++i) p[i * page] = 1;
+    std::printf("%d ", lbx::pages_made(p, n * page));
+    if (w.to - w.from == n) std::printf("%d ", lbx::pages_made(p + page / 2, 3 * page));
+    munmap(p, n * page);
+    if (w.to - w.from == n) std::printf("%d\n", lbx::pages_made(p, n * page));
   }
   return 0;
 }

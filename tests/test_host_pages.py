@@ -23,7 +23,7 @@ def test_pages_made(tmp_path):
     subprocess.run([gxx, "-std=c++17", "-O2", "-I" + os.path.join(ROOT, "lambrex_gb300", "csrc"),
                     os.path.join(HERE, "pages_host_check.cpp"), "-o", exe], check=True, capture_output=True)
     out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split()
-    assert out == ["0", "0", "0", "1", "1", "0"]
+    assert out == ["0", "0", "0", "0", "1", "1", "0"]
 
 
 @pytest.fixture(scope="module")
