@@ -6,6 +6,7 @@ import os
 import shutil
 import statistics
 import subprocess
+import sys
 import time
 
 import numpy as np
@@ -76,3 +77,34 @@ def test_used_pages_take_the_direct_copy(sim):
 
     times(copy)
     assert times(lambda: sim.density_field(0, out=out)) < 1.6 * times(copy)
+
+
+FIRST = """
+import mmap, time
+import numpy as np
+from lambrex_gb300 import lbx
+lbx.lambrexInit()
+s = lbx.AmrSim(80, 80, 80, 0, [1, 1, 1], 0.8, 0.8)
+s.SetInitialDensity(1.0)
+s.SetInitialVelocity(0.0)
+s.InitFromScratch(0.0)
+s.CalcHydroVars(0)
+s.mass_momentum(0)
+t = []
+for _ in range(3):
+    out = np.frombuffer(mmap.mmap(-1, 80 ** 3 * 8), dtype=np.float64).reshape(80, 80, 80)
+    t0 = time.perf_counter()
+    s.density_field(0, out=out)
+    t.append(time.perf_counter() - t0)
+print(t[0] / min(t[1:]))
+"""
+
+
+@pytest.mark.gpu
+def test_a_single_read_does_not_make_the_staging(gpu_lib):
+    """The first 4 MB of a process, against the next: making the buffers and the
+    copy threads took three times as long as the copy."""
+    ratio = [float(subprocess.run([sys.executable, "-c", FIRST], env=dict(os.environ, PYTHONPATH=ROOT), cwd=ROOT,
+                                  check=True, capture_output=True, text=True, timeout=300).stdout.split()[-1])
+             for _ in range(3)]
+    assert min(ratio) < 2.0, ratio
