@@ -12,6 +12,8 @@
 // refills the fine ghost shell before every sub-step from the parents
 // interpolated in time, with the non-equilibrium part rescaled between the
 // levels, and restricts the covered cells after the two sub-steps.
+#include <algorithm>
+
 #include "cells.cuh"
 #include "launch.cuh"
 #include "faithful.cuh"
@@ -242,11 +244,25 @@ __global__ void k_f_zero_ring0(double* __restrict__ f, Box3 b) {
   f_cell_zero_ring0(f, b, s.x, s.y, s.z);
 }
 
+// In pairs, a thread's place in the block is its place in a row: cells that the
+// pairs cannot hold (empty populations behind the covered cells' edge) lie at the
+// same places of many rows, and a warp with any of them takes the FP64
+// instructions too.  48x40x32 with a patch: 12.9 us, 16.9 with the cells in
+// storage order, as the fixed point takes them.
 template <bool PAIRED>
 __global__ void k_f_collide(double* __restrict__ f, Box3 b, IBox cov, double om_s, double om_b,
                             DfRates r) {
   int x, y, z;
-  if (!cell_xyz(b, x, y, z)) return;
+  if constexpr (PAIRED) {
+    const unsigned across = (b.n[0] + blockDim.x - 1) / blockDim.x;  // blocks to a row
+    const unsigned row = blockIdx.x / across * blockDim.y + threadIdx.y;
+    x = (int)(blockIdx.x % across * blockDim.x + threadIdx.x);
+    y = (int)(row % (unsigned)b.n[1]);
+    z = (int)(row / (unsigned)b.n[1]);
+    if (x >= b.n[0] || z >= b.n[2]) return;
+  } else if (!cell_xyz(b, x, y, z)) {
+    return;
+  }
   f_cell_collide<PAIRED>(f, b, cov, x, y, z, om_s, om_b, r);
 }
 
@@ -481,13 +497,16 @@ cudaError_t launch_f_zero_ring0(double* f, const Box3& b, cudaStream_t st) {
 }
 cudaError_t launch_f_collide(double* f, const Box3& b, IBox covered, double om_s, double om_b,
                              cudaStream_t st, bool paired) {
-  const CellLaunch rl = cell_launch(b, 128);
-  if (paired)
-    k_f_collide<true><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b,
-                                                    quiet(df_rates(om_s, om_b)));
-  else
-    k_f_collide<false><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b,
-                                                     quiet(df_rates(om_s, om_b)));
+  const DfRates r = quiet(df_rates(om_s, om_b));
+  if (paired) {  // rows rounded up to a warp, as many to a block of 128 as fit
+    const int bx = std::min((b.n[0] + 31) / 32 * 32, 128), by = 128 / bx;
+    const long long rows = (long long)b.n[1] * b.n[2];
+    const dim3 grid((unsigned)((b.n[0] + bx - 1) / bx * ((rows + by - 1) / by)));
+    k_f_collide<true><<<grid, dim3(bx, by, 1), 0, st>>>(f, b, covered, om_s, om_b, r);
+  } else {
+    const CellLaunch rl = cell_launch(b, 128);
+    k_f_collide<false><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b, r);
+  }
   return cudaGetLastError();
 }
 cudaError_t launch_f_stream(const double* src, double* dst, const Box3& b, cudaStream_t st) {
