@@ -244,22 +244,22 @@ __global__ void k_f_zero_ring0(double* __restrict__ f, Box3 b) {
   f_cell_zero_ring0(f, b, s.x, s.y, s.z);
 }
 
-// In pairs, a thread's place in the block is its place in a row: cells that the
-// pairs cannot hold (empty populations behind the covered cells' edge) lie at the
-// same places of many rows, and a warp with any of them takes the FP64
-// instructions too.  48x40x32 with a patch: 12.9 us, 16.9 with the cells in
-// storage order, as the fixed point takes them.
-template <bool PAIRED>
+// ROWS: a block's threads stand along rows of x, padded to warps, not along the
+// cells in storage order.  For the paired collision of small boxes with rows
+// longer than a warp: cells that the pairs cannot hold (empty populations behind
+// the covered cells' edge) lie at the same places of many rows, a warp with any of
+// them takes the FP64 instructions too, and there are too few warps to hide it.
+// us, rows | storage order: 48x40x32 12.2 | 15.9, 40^3 13.9 | 14.9, 48^3 18.1 | 18.1,
+// 20x60x60 21.9 | 17.4, 100x90x70 48.8 | 43.9, 130^3 144 | 126.
+template <bool PAIRED, bool ROWS = false>
 __global__ void k_f_collide(double* __restrict__ f, Box3 b, IBox cov, double om_s, double om_b,
                             DfRates r) {
   int x, y, z;
-  if constexpr (PAIRED) {
-    const unsigned across = (b.n[0] + blockDim.x - 1) / blockDim.x;  // blocks to a row
-    const unsigned row = blockIdx.x / across * blockDim.y + threadIdx.y;
-    x = (int)(blockIdx.x % across * blockDim.x + threadIdx.x);
-    y = (int)(row % (unsigned)b.n[1]);
-    z = (int)(row / (unsigned)b.n[1]);
-    if (x >= b.n[0] || z >= b.n[2]) return;
+  if (ROWS) {
+    x = blockIdx.x * blockDim.x + threadIdx.x;
+    y = blockIdx.y * blockDim.y + threadIdx.y;
+    z = blockIdx.z;
+    if (x >= b.n[0] || y >= b.n[1]) return;
   } else if (!cell_xyz(b, x, y, z)) {
     return;
   }
@@ -498,13 +498,15 @@ cudaError_t launch_f_zero_ring0(double* f, const Box3& b, cudaStream_t st) {
 cudaError_t launch_f_collide(double* f, const Box3& b, IBox covered, double om_s, double om_b,
                              cudaStream_t st, bool paired) {
   const DfRates r = quiet(df_rates(om_s, om_b));
-  if (paired) {  // rows rounded up to a warp, as many to a block of 128 as fit
+  const long long cells = (long long)b.n[0] * b.n[1] * b.n[2];
+  const CellLaunch rl = cell_launch(b, 128);
+  if (paired && b.n[0] > 32 && cells < (1 << 16)) {  // so y and z are within a grid's limits
     const int bx = std::min((b.n[0] + 31) / 32 * 32, 128), by = 128 / bx;
-    const long long rows = (long long)b.n[1] * b.n[2];
-    const dim3 grid((unsigned)((b.n[0] + bx - 1) / bx * ((rows + by - 1) / by)));
-    k_f_collide<true><<<grid, dim3(bx, by, 1), 0, st>>>(f, b, covered, om_s, om_b, r);
+    const dim3 grid((b.n[0] + bx - 1) / bx, (b.n[1] + by - 1) / by, b.n[2]);
+    k_f_collide<true, true><<<grid, dim3(bx, by, 1), 0, st>>>(f, b, covered, om_s, om_b, r);
+  } else if (paired) {
+    k_f_collide<true><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b, r);
   } else {
-    const CellLaunch rl = cell_launch(b, 128);
     k_f_collide<false><<<rl.grid, rl.block, 0, st>>>(f, b, covered, om_s, om_b, r);
   }
   return cudaGetLastError();

@@ -1,6 +1,7 @@
-"""The faithful cycle's paired collision gives a block whole rows
-(csrc/kernels_amr.cu): boxes whose rows are shorter and longer than a warp and a
-block, with row counts that leave a block part empty, against the oracle."""
+"""The faithful cycle's paired collision gives a block whole rows in small boxes
+with rows longer than a warp (csrc/kernels_amr.cu): rows shorter and longer than a
+warp and a block, row counts that leave a block part empty, a level on either side
+of the line, against the oracle."""
 import numpy as np
 import pytest
 
@@ -10,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dims,lo,hi", [((4, 5, 4), (1, 1, 1), (2, 3, 2)), ((33, 7, 6), (8, 2, 2), (20, 4, 3)),
-                                        ((64, 5, 9), (10, 1, 2), (40, 3, 6)), ((130, 6, 5), (20, 1, 1), (100, 4, 3))])
+                                        ((64, 5, 9), (10, 1, 2), (40, 3, 6)), ((130, 6, 5), (20, 1, 1), (100, 4, 3)),
+                                        ((44, 42, 40), (10, 10, 10), (30, 28, 26))])
 def test_rows_of_the_paired_collision(gpu_lib, oracle, dims, lo, hi):
     rho_c, u_c = smooth_random(*dims, seed=5)
     s = gpu_lib.AmrSim(*dims, 1, [1, 1, 1], 0.9, 0.8, precision="f64p", amr_mode="faithful")
