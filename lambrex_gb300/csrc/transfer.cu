@@ -378,7 +378,7 @@ cudaError_t upload_host(void* dst, const void* src, size_t bytes, cudaStream_t s
 }
 
 cudaError_t download_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-  if (bytes >= kSmallMin && bytes < kStageMin && !pages_made(dst, bytes) && !pinned_host(dst))
+  if (bytes >= kSmallMin && bytes < kStageMin && !pinned_host(dst) && !pages_made(dst, bytes))
     return download_small(static_cast<char*>(dst), static_cast<const char*>(src), bytes, st);
   if (bytes < kStageMin || pinned_host(dst)) {
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);

@@ -1,7 +1,7 @@
 // Host build of the look at a caller's pages (csrc/host_pages.h) for
 // tests/test_host_pages.py: prints, in order, whether the pages are made of new
 // memory, of the same with its first and last page written, as an allocator
-// does, with its first and with its second half written, of all of it written,
+// does, with its first and with its last third written, of all of it written,
 // of a part from the middle of a page on, and of memory that is not mapped.
 #include <cstdio>
 
@@ -16,7 +16,7 @@ int main() {
   };
   const struct {
     size_t from, to;
-  } written[] = {{n, 0}, {0, n / 2}, {n / 2, n}, {0, n}};
+  } written[] = {{n, 0}, {0, n / 3}, {n - n / 3, n}, {0, n}};
   for (const auto& w : written) {
     char* p = fresh();
     if (w.from > w.to) {
