@@ -475,18 +475,14 @@ __host__ __device__ __forceinline__ double times_pow2(double x, int k) {
 // eight diagonal ones are: what is left of it, with the roundings that its
 // operations have as the device's compiler contracts them, so that the bits are
 // its own: 14 FP64 instructions instead of 128 (powers of two change only the
-// exponents; 1/9, 2/9 and 1/72, and 1/3, 1/6 and 1/24 are such multiples).
-// False, f untouched, without an ordinary density: the general form divides by it.
-__host__ __device__ __forceinline__ bool collide_rest(double* f, double om_s, double om_b) {
+// exponents; 1/9, 2/9 and 1/72, and 1/3, 1/6 and 1/24 are such multiples)
+__host__ __device__ __forceinline__ void collide_rest(double* f, double om_s, double om_b) {
 #ifdef __CUDA_ARCH__
   const double A = __dmul_rn(6.0, f[1]);  // rounded, not part of an FMA
 #else
   const double A = 6.0 * f[1];
 #endif
   const double drho = fma(8.0, f[7], f[0] + A);
-  uint32_t h, l;
-  d_words(drho, &h, &l);
-  if (!fx_top_ok(h)) return false;
   const double d = fma(-1.0 / 3.0, A, times_pow2(f[1], 1));
   const double TrS = fma(24.0, f[7], A) - drho;
   const double m = fma(fma(om_b, -TrS, TrS), 1.0 / 3.0, fma(om_s, -d, d));
@@ -497,18 +493,19 @@ __host__ __device__ __forceinline__ bool collide_rest(double* f, double om_s, do
   f[0] = times_pow2(ba, 1);
 #pragma unroll
   for (int q = 1; q < NV; ++q) f[q] = q < 7 ? ex : bd;
-  return true;
 }
+// such a cell, none of its populations negative and one of them at least 2^-1022:
+// the general form divides by the density, an empty cell is NaN there
 __host__ __device__ __forceinline__ bool is_rest(const double* f) {
   uint32_t h[NV], l[NV], d = 0;
 #pragma unroll
-  for (int q = 1; q < NV; ++q) d_words(f[q], &h[q], &l[q]);
+  for (int q = 0; q < NV; ++q) d_words(f[q], &h[q], &l[q]);
 #pragma unroll
   for (int q = 2; q < NV; ++q) {
     const int t = q < 7 ? 1 : 7;
     d |= (h[q] ^ h[t]) | (l[q] ^ l[t]);
   }
-  return d == 0;
+  return (d == 0) & ((h[0] | h[1] | h[7]) - 0x00100000u < 0x7fe00000u);
 }
 
 // whether a cell's populations are those of a fluid at rest (fx_at_rest)
@@ -542,8 +539,10 @@ __host__ __device__ __forceinline__ void collide_f64(double* f, double om_s, dou
 #else
   if (collide_fx<QUIET>(f, r.ok ? r : fx_rates(om_s, om_b))) return;
 #endif
-  if (QUIET && is_rest(f) && collide_rest(f, om_s, om_b)) return;
-  collide<double>(f, om_s, om_b, 0.0);
+  if (QUIET && is_rest(f))
+    collide_rest(f, om_s, om_b);
+  else
+    collide<double>(f, om_s, om_b, 0.0);
 }
 
 }  // namespace lbx

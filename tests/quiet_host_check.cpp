@@ -21,7 +21,7 @@ int main(int argc, char** argv) {
   double f[2 * lbx::NV + 1], g[lbx::NV];
   while (std::fread(f, sizeof(double), lbx::NV, in) == (size_t)lbx::NV) {
     for (int q = 0; q < lbx::NV; ++q) f[lbx::NV + q] = g[q] = f[q];
-    f[2 * lbx::NV] = !lbx::collide_fx<true>(g, r) && lbx::is_rest(g) && lbx::collide_rest(g, om_s, om_b) ? 1.0 : 0.0;
+    f[2 * lbx::NV] = !lbx::collide_fx<true>(g, r) && lbx::is_rest(f) ? 1.0 : 0.0;
     lbx::collide_f64<true>(f, om_s, om_b, r);
     lbx::collide<double>(f + lbx::NV, om_s, om_b, 0.0);
     std::fwrite(f, sizeof(double), 2 * lbx::NV + 1, out);
