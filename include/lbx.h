@@ -170,7 +170,8 @@ int lbx_get_device_f(lbx_sim* sim, int level, void** ptr, int* storage_dims3, in
  * One fused collide+stream step of a fully periodic box, f_in -> f_out, FAB
  * order without ghosts, on `stream` (a cudaStream_t, NULL = default).
  * Replaces Collide + FillBoundary + Stream + UpdateNow of one level
- * (src/AmrSim.cpp:25-135, include/component.h:22-29). */
+ * (src/AmrSim.cpp:25-135, include/component.h:22-29).  Boxes of any number of
+ * cells: the limit of 2^31 - 1 is that of the handles and of the sums. */
 int lbx_step_periodic_f64(const double* f_in, double* f_out, int nx, int ny, int nz,
                           double tau_s, double tau_b, void* stream);
 /* the same with the collision of LBX_F64_PAIRED */

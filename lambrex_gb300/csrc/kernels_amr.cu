@@ -139,13 +139,14 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 8 : RESC ? 1 : 0)
 }
 
 // Whether anything moves on a level, of the cells at every fourth place: sets
-// *moving, which the last kernel of the step before cleared.  Only the speed of a
-// refined FP64 step depends on it.  While a patch is at rest, its cells and the
-// coarse ones take the FP64 instructions (collide_f64); once a wave is in it,
-// what is rounding alone no longer shows, and the fluid at rest elsewhere is
-// collided in fixed point like the rest (a pulse's first 20 steps in 104x88x72,
-// rescaled: 5.5 to 8.3 ms without the look, 3.4 to 4.4 with it, 3.2 and 3.3
-// later on).
+// *moving, which the last kernel of the step before cleared.  While a patch is at
+// rest, its cells and the coarse ones take the FP64 instructions (collide_f64);
+// once a wave is in it, what is rounding alone no longer shows, and the fluid at
+// rest elsewhere is collided in fixed point like the rest (a pulse's first 20 steps
+// in 104x88x72, rescaled: 5.5 to 8.3 ms without the look, 3.4 to 4.4 with it, 3.2
+// and 3.3 later on).  So the look chooses between two roundings of cells at rest:
+// last bits depend on it, and a wave that it misses leaves them at the error of the
+// FP64 instructions.
 __global__ void __launch_bounds__(128) k_moving(const double* __restrict__ f, Box3 b, unsigned* moving) {
   chain_begin();
   const int nx = (b.n[0] + 3) / 4, ny = (b.n[1] + 3) / 4, nz = (b.n[2] + 3) / 4;
